@@ -231,8 +231,7 @@ struct SchedArgs {
 };
 
 // Two fp32 values in one 64-bit register for Blackwell's packed arithmetic
-// (sub.rn.f32x2, mul.rn.f32x2): each half is rounded exactly like the scalar
-// instruction, so the box test below gives the same bits as scalar code.
+// (fma.rn.f32x2): each half is rounded exactly like the scalar instruction.
 __device__ __forceinline__ unsigned long long f2pack(float lo, float hi) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -243,12 +242,11 @@ __device__ __forceinline__ float2 f2unpack(unsigned long long v) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
   return r;
 }
-// (a - b) * c per half
-__device__ __forceinline__ float2 f2subMul(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d, e;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(e) : "l"(d), "l"(c));
-  return f2unpack(e);
+// a * b + c per half, rounded once
+__device__ __forceinline__ float2 f2fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return f2unpack(d);
 }
 
 // Rays per chunk of the scheduler: a multiple of 32 covering n rays in at

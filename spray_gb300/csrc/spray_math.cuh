@@ -215,12 +215,21 @@ SPRAY_HD bool slabTest(const float bmin[3], const float bmax[3], V3 org, V3 inv,
 // recomputed in double when one is exactly zero, no backface culling.
 // Barycentrics follow the (u, v) convention of the reference's hit record:
 // hit = (1-u-v)*v0 + u*v1 + v*v2.
+//
+// The axes are rotated so that kz is the direction's largest component.  The
+// published test also swaps kx and ky when that component is negative, to keep
+// the winding; without the swap U, V, W, det and T are exactly the negatives
+// (each is a difference of the same rounded products), and t, u and v, their
+// quotients, have the same bits, so the swap is left out.
 struct RayShear {
-  int kx, ky, kz;
+  int kz;
   float Sx, Sy, Sz;
 };
 
-SPRAY_HD float comp(V3 a, int k) { return k == 0 ? a.x : (k == 1 ? a.y : a.z); }
+// component kz + 1, kz + 2 (modulo 3) and kz of a vector
+SPRAY_HD float compX(V3 a, int kz) { return kz == 0 ? a.y : (kz == 1 ? a.z : a.x); }
+SPRAY_HD float compY(V3 a, int kz) { return kz == 0 ? a.z : (kz == 1 ? a.x : a.y); }
+SPRAY_HD float compZ(V3 a, int kz) { return kz == 0 ? a.x : (kz == 1 ? a.y : a.z); }
 
 SPRAY_HD RayShear makeShear(V3 d) {
   RayShear s;
@@ -229,19 +238,10 @@ SPRAY_HD RayShear makeShear(V3 d) {
   float m = ax;
   if (ay > m) { kz = 1; m = ay; }
   if (az > m) { kz = 2; }
-  int kx = kz + 1 == 3 ? 0 : kz + 1;
-  int ky = kx + 1 == 3 ? 0 : kx + 1;
-  if (comp(d, kz) < 0.0f) {
-    int t = kx;
-    kx = ky;
-    ky = t;
-  }
-  s.kx = kx;
-  s.ky = ky;
   s.kz = kz;
-  float dz = comp(d, kz);
-  s.Sx = comp(d, kx) / dz;
-  s.Sy = comp(d, ky) / dz;
+  float dz = compZ(d, kz);
+  s.Sx = compX(d, kz) / dz;
+  s.Sy = compY(d, kz) / dz;
   s.Sz = 1.0f / dz;
   return s;
 }
@@ -250,13 +250,13 @@ SPRAY_HD RayShear makeShear(V3 d) {
 SPRAY_HD bool intersectTriangle(const RayShear& sh, V3 org, V3 p0, V3 p1, V3 p2, float tnear,
                                 float tfar, float* t_o, float* u_o, float* v_o) {
   V3 A = p0 - org, B = p1 - org, C = p2 - org;
-  float Akz = comp(A, sh.kz), Bkz = comp(B, sh.kz), Ckz = comp(C, sh.kz);
-  float Ax = comp(A, sh.kx) - sh.Sx * Akz;
-  float Ay = comp(A, sh.ky) - sh.Sy * Akz;
-  float Bx = comp(B, sh.kx) - sh.Sx * Bkz;
-  float By = comp(B, sh.ky) - sh.Sy * Bkz;
-  float Cx = comp(C, sh.kx) - sh.Sx * Ckz;
-  float Cy = comp(C, sh.ky) - sh.Sy * Ckz;
+  float Akz = compZ(A, sh.kz), Bkz = compZ(B, sh.kz), Ckz = compZ(C, sh.kz);
+  float Ax = compX(A, sh.kz) - sh.Sx * Akz;
+  float Ay = compY(A, sh.kz) - sh.Sy * Akz;
+  float Bx = compX(B, sh.kz) - sh.Sx * Bkz;
+  float By = compY(B, sh.kz) - sh.Sy * Bkz;
+  float Cx = compX(C, sh.kz) - sh.Sx * Ckz;
+  float Cy = compY(C, sh.kz) - sh.Sy * Ckz;
   float U = Cx * By - Cy * Bx;
   float V = Ax * Cy - Ay * Cx;
   float W = Bx * Ay - By * Ax;

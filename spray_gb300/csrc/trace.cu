@@ -38,26 +38,22 @@ __device__ __forceinline__ bool anyRound(Walk& w, int* stack, const TravRay& r, 
       return true;
     }
     float tn[4];
+    bool ch_hit[4];
     ++nnodes;
-    // scalar: the packed test's registers make the refilling walk spill
-    const int mask = testChildrenScalar(w.nodes, w.cur, r, kRayEpsilon, tfar, tn);
+    testChildren(w.nodes, w.cur, r, kRayEpsilon, tfar, tn, ch_hit);
     const int4 ch = loadChildren(w.nodes, w.cur);
+    if (w.sp > kStack - 3) {
+      raise(ctr, kErrTraversalBound);
+      return true;
+    }
     // the last child hit continues the walk; the earlier ones are pushed
     // (the order a push of all of them and a pop would give)
     int next = kDone;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      if (!(mask & (1 << c))) continue;
-      const int ref = childAt(ch, c);
-      if (ref == kEmptyChild) continue;
-      if (next != kDone) {
-        if (w.sp == kStack) {
-          raise(ctr, kErrTraversalBound);
-          return true;
-        }
-        stack[w.sp++] = next;
-      }
-      next = ref;
+      if (!ch_hit[c]) continue;
+      if (next != kDone) stack[w.sp++] = next;
+      next = childAt(ch, c);
     }
     w.cur = next != kDone ? next : (w.sp > 0 ? stack[--w.sp] : kDone);
   }

@@ -16,88 +16,112 @@ namespace {
 constexpr float kBoxSlack = 1.0000004f;
 constexpr int kStack = 64;
 
-struct TravRay {
-  V3 org, dir, inv;
+// A ray as the box tests use it.  The distance of a plane p along an axis is
+// fma(p, inv, c): with inv = 1 / dir and c = -org * inv that is (p - org) / dir
+// but for relative roundings (the slack's part) and the rounding of org * inv,
+// at most 2^-24 of |org * inv| for the product and as much for c.  c is
+// therefore kept twice, moved by 2^-22 of |org * inv|: down for near planes, up
+// for far ones, so that the interval only ever grows.  |inv| is held within
+// [1e-30, 1e18], so that an empty slot (lo = +inf, hi = -inf) is never entered
+// and an axis the ray is parallel to gives finite distances of the right sign
+// (fma(p, inf, -inf) would be a NaN); its planes count as touched within 1e-6
+// of the origin (1e12 / 1e18), as (p - org) * inf = NaN for p = org would.
+struct BoxRay {
+  V3 inv, cnear, cfar;
   int sx, sy, sz;  // 1 when the direction component is negative
+};
+
+__device__ __forceinline__ float boxPad(float oi, float inv) {
+  return fabsf(oi) * 2.384185791015625e-7f + (fabsf(inv) > 1e18f ? 1e12f : 0.0f);
+}
+
+__device__ __forceinline__ void boxAxis(float org, float inv, float& binv, float& cnear, float& cfar) {
+  binv = copysignf(fminf(fmaxf(fabsf(inv), 1e-30f), 1e18f), inv);
+  const float oi = org * binv;
+  const float pad = boxPad(oi, inv);
+  cnear = -oi - pad;
+  cfar = pad - oi;
+}
+
+// inv = 1 / dir, as IEEE division gives it
+__device__ __forceinline__ BoxRay makeBoxRay(V3 org, V3 inv) {
+  BoxRay r;
+  boxAxis(org.x, inv.x, r.inv.x, r.cnear.x, r.cfar.x);
+  boxAxis(org.y, inv.y, r.inv.y, r.cnear.y, r.cfar.y);
+  boxAxis(org.z, inv.z, r.inv.z, r.cnear.z, r.cfar.z);
+  r.sx = inv.x < 0.0f;
+  r.sy = inv.y < 0.0f;
+  r.sz = inv.z < 0.0f;
+  return r;
+}
+
+// A ray as the walks use it.
+struct TravRay {
+  V3 org;
+  BoxRay box;
   RayShear sh;
 };
 
 __device__ __forceinline__ TravRay makeTravRay(V3 org, V3 dir) {
   TravRay r;
   r.org = org;
-  r.dir = dir;
-  r.inv = v3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
-  r.sx = r.inv.x < 0.0f;
-  r.sy = r.inv.y < 0.0f;
-  r.sz = r.inv.z < 0.0f;
+  r.box = makeBoxRay(org, v3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z));
   r.sh = makeShear(dir);
   return r;
 }
 
-// Intersects the four children of a node; returns a mask of hit children and
-// their entry distances.  Near and far planes are picked by the direction's
-// sign, so an empty slot (lo = +inf, hi = -inf) can never be entered.  Per
-// child: t0 = max(max(tx0, ty0), max(tz0, tnear)), t1 = min(min(tx1, ty1),
-// min(tz1, tfar)) * kBoxSlack with tx = (plane - org.x) * inv.x; children
-// (0, 1) and (2, 3) share the packed subtractions and products.
-__device__ __forceinline__ int testChildren(const BvhNode4* __restrict__ nodes, int node,
-                                            const TravRay& r, float tnear, float tfar,
-                                            float tn[4]) {
-  // the node stores lo/hi per axis as float4 pairs; the ray's signs pick the
-  // near and far plane of each pair by address
-  const float4* p = reinterpret_cast<const float4*>(nodes + node);
-  const float4 nx = __ldg(p + r.sx), fx = __ldg(p + (r.sx ^ 1));
-  const float4 ny = __ldg(p + 2 + r.sy), fy = __ldg(p + (3 - r.sy));
-  const float4 nz = __ldg(p + 4 + r.sz), fz = __ldg(p + (5 - r.sz));
-  const unsigned long long ox = f2pack(r.org.x, r.org.x), oy = f2pack(r.org.y, r.org.y),
-                           oz = f2pack(r.org.z, r.org.z);
-  const unsigned long long ix = f2pack(r.inv.x, r.inv.x), iy = f2pack(r.inv.y, r.inv.y),
-                           iz = f2pack(r.inv.z, r.inv.z);
-  int mask = 0;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float2 ax = f2subMul(h ? f2pack(nx.z, nx.w) : f2pack(nx.x, nx.y), ox, ix);
-    const float2 ay = f2subMul(h ? f2pack(ny.z, ny.w) : f2pack(ny.x, ny.y), oy, iy);
-    const float2 az = f2subMul(h ? f2pack(nz.z, nz.w) : f2pack(nz.x, nz.y), oz, iz);
-    const float2 bx = f2subMul(h ? f2pack(fx.z, fx.w) : f2pack(fx.x, fx.y), ox, ix);
-    const float2 by = f2subMul(h ? f2pack(fy.z, fy.w) : f2pack(fy.x, fy.y), oy, iy);
-    const float2 bz = f2subMul(h ? f2pack(fz.z, fz.w) : f2pack(fz.x, fz.y), oz, iz);
-    const float t00 = fmaxf(fmaxf(ax.x, ay.x), fmaxf(az.x, tnear));
-    const float t01 = fmaxf(fmaxf(ax.y, ay.y), fmaxf(az.y, tnear));
-    const float t10 = fminf(fminf(bx.x, by.x), fminf(bz.x, tfar)) * kBoxSlack;
-    const float t11 = fminf(fminf(bx.y, by.y), fminf(bz.y, tfar)) * kBoxSlack;
-    tn[2 * h] = t00;
-    tn[2 * h + 1] = t01;
-    if (t00 <= t10) mask |= 1 << (2 * h);
-    if (t01 <= t11) mask |= 1 << (2 * h + 1);
-  }
-  return mask;
+// max and min of three (one instruction on sm_100 and later; a NaN operand is
+// dropped, as by fmaxf and fminf)
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
-// The same test in scalar arithmetic (fewer live registers), for the
-// occlusion walk.
-__device__ __forceinline__ int testChildrenScalar(const BvhNode4* __restrict__ nodes, int node,
-                                                  const TravRay& r, float tnear, float tfar,
-                                                  float tn[4]) {
-  const float4* p = reinterpret_cast<const float4*>(nodes + node);
-  const float4 nx = __ldg(p + r.sx), fx = __ldg(p + (r.sx ^ 1));
-  const float4 ny = __ldg(p + 2 + r.sy), fy = __ldg(p + (3 - r.sy));
-  const float4 nz = __ldg(p + 4 + r.sz), fz = __ldg(p + (5 - r.sz));
-  const float nxa[4] = {nx.x, nx.y, nx.z, nx.w}, fxa[4] = {fx.x, fx.y, fx.z, fx.w};
-  const float nya[4] = {ny.x, ny.y, ny.z, ny.w}, fya[4] = {fy.x, fy.y, fy.z, fy.w};
-  const float nza[4] = {nz.x, nz.y, nz.z, nz.w}, fza[4] = {fz.x, fz.y, fz.z, fz.w};
-  int mask = 0;
+// Intersects the four boxes of a node: their entry distances tn, and hit.
+// Near and far planes are picked by the direction's sign, by address: the
+// node stores lo/hi per axis as float4 pairs.  Per box: t0 = max(near x, y, z,
+// tnear), t1 = min(far x, y, z, tfar) * slack; boxes (0, 1) and (2, 3) share
+// packed multiply-adds, and the maxima take three operands: the walks are
+// bound by instruction issue, the min/max/compare pipe first.
+__device__ __forceinline__ void testBoxes(float4 nx, float4 fx, float4 ny, float4 fy, float4 nz, float4 fz,
+                                          const BoxRay& r, float tnear, float tfar, float slack, float tn[4],
+                                          bool hit[4]) {
+  const unsigned long long ix = f2pack(r.inv.x, r.inv.x), iy = f2pack(r.inv.y, r.inv.y),
+                           iz = f2pack(r.inv.z, r.inv.z);
+  const unsigned long long nx2 = f2pack(r.cnear.x, r.cnear.x), ny2 = f2pack(r.cnear.y, r.cnear.y),
+                           nz2 = f2pack(r.cnear.z, r.cnear.z);
+  const unsigned long long fx2 = f2pack(r.cfar.x, r.cfar.x), fy2 = f2pack(r.cfar.y, r.cfar.y),
+                           fz2 = f2pack(r.cfar.z, r.cfar.z);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    float t0 = fmaxf(fmaxf((nxa[c] - r.org.x) * r.inv.x, (nya[c] - r.org.y) * r.inv.y),
-                     fmaxf((nza[c] - r.org.z) * r.inv.z, tnear));
-    float t1 = fminf(fminf((fxa[c] - r.org.x) * r.inv.x, (fya[c] - r.org.y) * r.inv.y),
-                     fminf((fza[c] - r.org.z) * r.inv.z, tfar)) *
-               kBoxSlack;
-    tn[c] = t0;
-    if (t0 <= t1) mask |= 1 << c;
+  for (int h = 0; h < 2; ++h) {
+    const float2 ax = f2fma(h ? f2pack(nx.z, nx.w) : f2pack(nx.x, nx.y), ix, nx2);
+    const float2 ay = f2fma(h ? f2pack(ny.z, ny.w) : f2pack(ny.x, ny.y), iy, ny2);
+    const float2 az = f2fma(h ? f2pack(nz.z, nz.w) : f2pack(nz.x, nz.y), iz, nz2);
+    const float2 bx = f2fma(h ? f2pack(fx.z, fx.w) : f2pack(fx.x, fx.y), ix, fx2);
+    const float2 by = f2fma(h ? f2pack(fy.z, fy.w) : f2pack(fy.x, fy.y), iy, fy2);
+    const float2 bz = f2fma(h ? f2pack(fz.z, fz.w) : f2pack(fz.x, fz.y), iz, fz2);
+    const float t00 = fmaxf(max3(ax.x, ay.x, az.x), tnear);
+    const float t01 = fmaxf(max3(ax.y, ay.y, az.y), tnear);
+    const float t10 = fminf(min3(bx.x, by.x, bz.x), tfar) * slack;
+    const float t11 = fminf(min3(bx.y, by.y, bz.y), tfar) * slack;
+    tn[2 * h] = t00;
+    tn[2 * h + 1] = t01;
+    hit[2 * h] = t00 <= t10;
+    hit[2 * h + 1] = t01 <= t11;
   }
-  return mask;
+}
+
+__device__ __forceinline__ void testChildren(const BvhNode4* __restrict__ nodes, int node, const TravRay& r,
+                                             float tnear, float tfar, float tn[4], bool hit[4]) {
+  const float4* p = reinterpret_cast<const float4*>(nodes + node);
+  testBoxes(__ldg(p + r.box.sx), __ldg(p + (r.box.sx ^ 1)), __ldg(p + 2 + r.box.sy), __ldg(p + (3 - r.box.sy)),
+            __ldg(p + 4 + r.box.sz), __ldg(p + (5 - r.box.sz)), r.box, tnear, tfar, kBoxSlack, tn, hit);
 }
 
 __device__ __forceinline__ int4 loadChildren(const BvhNode4* __restrict__ nodes, int node) {
@@ -222,43 +246,29 @@ __device__ bool traverseClosest(const SceneDev& sc, const DomainDev& dom, const 
         return finish();
       }
       float tn[4];
-      const int mask = testChildren(nodes, cur, r, kRayEpsilon, best_t, tn);
+      bool hit[4];
+      testChildren(nodes, cur, r, kRayEpsilon, best_t, tn, hit);
       const int4 ch = loadChildren(nodes, cur);
-      // Children sorted near to far by a key of the entry t with its two low
-      // bits replaced by the slot: t >= tnear > 0, so the bits order like the
-      // value, and the key's t (rounded down by at most 3 ulp) stays a lower
-      // bound of the entry.  A five-comparator network keeps it in registers.
+      // The nearest child continues the walk, the others go on the stack in
+      // slot order: a node rarely has more than two children hit (sorting
+      // them by a network costs more than the order of a third and fourth
+      // saves), and a pushed entry beyond the best hit is dropped on pop.
+      // The key is the entry t with its two low bits replaced by the slot:
+      // t >= tnear > 0, so the bits order like the value, and the key's t
+      // (rounded down by at most 3 ulp) stays a lower bound of the entry.
       uint32_t k[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        k[c] = ((mask & (1 << c)) && childAt(ch, c) != kEmptyChild)
-                   ? (__float_as_uint(tn[c]) & ~3u) | (uint32_t)c
-                   : 0xffffffffu;
-      auto cswap = [](uint32_t& x, uint32_t& y) {
-        const uint32_t lo = min(x, y), hi = max(x, y);
-        x = lo;
-        y = hi;
-      };
-      cswap(k[0], k[1]);
-      cswap(k[2], k[3]);
-      cswap(k[0], k[2]);
-      cswap(k[1], k[3]);
-      cswap(k[1], k[2]);
-      // The nearest child continues the walk when it starts within the best
-      // hit; the others go on the stack far to near.  Every other child starts
-      // at least as far as the nearest, so when the nearest is beyond the best
-      // hit all of them are (pop would drop them) and the walk pops instead.
-      if (k[0] != 0xffffffffu && __uint_as_float(k[0] & ~3u) <= best_t) {
-#pragma unroll
-        for (int j = 3; j >= 1; --j) {
-          if (k[j] == 0xffffffffu) continue;
-          if (sp == kStack) {
-            raise(ctr, kErrTraversalBound);
-            return finish();
-          }
-          stack[sp++] = make_uint2((uint32_t)childAt(ch, (int)(k[j] & 3u)), k[j] & ~3u);
+      for (int c = 0; c < 4; ++c) k[c] = hit[c] ? (__float_as_uint(tn[c]) & ~3u) | (uint32_t)c : 0xffffffffu;
+      const uint32_t kmin = min(__vimin3_u32(k[0], k[1], k[2]), k[3]);
+      if (kmin != 0xffffffffu) {
+        if (sp > kStack - 3) {
+          raise(ctr, kErrTraversalBound);
+          return finish();
         }
-        cur = childAt(ch, (int)(k[0] & 3u));
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (hit[c] && k[c] != kmin) stack[sp++] = make_uint2((uint32_t)childAt(ch, c), k[c] & ~3u);
+        cur = childAt(ch, (int)(kmin & 3u));
       } else {
         cur = pop();
       }
@@ -286,23 +296,20 @@ __device__ bool traverseAny(const SceneDev& sc, const DomainDev& dom, const Trav
         return false;
       }
       float tn[4];
-      const int mask = testChildren(g.nodes, cur, r, kRayEpsilon, tfar, tn);
+      bool hit[4];
+      testChildren(g.nodes, cur, r, kRayEpsilon, tfar, tn, hit);
       const int4 ch = loadChildren(g.nodes, cur);
+      if (sp > kStack - 3) {
+        raise(ctr, kErrTraversalBound);
+        nnodes += steps;
+        return false;
+      }
       int next = kDone;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        if (!(mask & (1 << c))) continue;
-        const int ref = childAt(ch, c);
-        if (ref == kEmptyChild) continue;
-        if (next != kDone) {
-          if (sp == kStack) {
-            raise(ctr, kErrTraversalBound);
-            nnodes += steps;
-            return false;
-          }
-          stack[sp++] = next;
-        }
-        next = ref;
+        if (!hit[c]) continue;
+        if (next != kDone) stack[sp++] = next;
+        next = childAt(ch, c);
       }
       cur = next != kDone ? next : (sp > 0 ? stack[--sp] : kDone);
     }
