@@ -20,7 +20,7 @@ CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-CU_SOURCES = ["sched.cu", "trace.cu", "shade.cu", "tracer.cu", "insitu.cu", "bvh_build.cu", "noalloc.cu",
+CU_SOURCES = ["sched.cu", "trace.cu", "walk_rays.cu", "shade.cu", "tracer.cu", "insitu.cu", "bvh_build.cu", "noalloc.cu",
               "rounds.cu", "mlp.cu", "mlp_api.cu"]
 CPP_SOURCES = ["bvh.cpp", "host_scene.cpp", "host_api.cpp"]
 

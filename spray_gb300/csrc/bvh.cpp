@@ -392,4 +392,52 @@ void buildDomainBvh4(const float* boxes, int n, std::vector<BvhNode4>* out) {
   c.emit(0);
 }
 
+void buildDomainGroups(const float* boxes, int n, std::vector<BvhNode4>* out, int* l1_count) {
+  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  auto centre = [&](int d, int k) { return 0.5f * boxes[6 * d + k] + 0.5f * boxes[6 * d + 3 + k]; };
+  for (int d = 0; d < n; ++d)
+    for (int k = 0; k < 3; ++k) {
+      lo[k] = std::min(lo[k], centre(d, k));
+      hi[k] = std::max(hi[k], centre(d, k));
+    }
+  std::vector<std::pair<uint32_t, int>> order(n);
+  for (int d = 0; d < n; ++d) {
+    uint32_t code = 0;
+    for (int k = 0; k < 3; ++k) {
+      const float e = hi[k] - lo[k];
+      const float f = e > 0.0f ? (centre(d, k) - lo[k]) / e : 0.0f;  // NaN and infinite boxes: any place will do
+      const uint32_t q = f > 0.0f ? (uint32_t)std::min(f * 1023.0f, 1023.0f) : 0u;
+      for (int b = 0; b < 10; ++b) code |= ((q >> b) & 1u) << (3 * b + k);
+    }
+    order[d] = {code, d};
+  }
+  std::sort(order.begin(), order.end());
+  const int n2 = (n + 3) / 4, n1 = (n + 63) / 64;
+  BvhNode4 empty;
+  std::memset(&empty, 0, sizeof(empty));
+  const float none_lo[3] = {INFINITY, INFINITY, INFINITY}, none_hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  for (int c = 0; c < 4; ++c) DomCollapse::setSlot(empty, c, none_lo, none_hi, kEmptyChild);
+  out->assign((size_t)n1 + n2, empty);
+  *l1_count = n1;
+  // a NaN bound spans everything, so that the group test never rejects a domain
+  // the exact slab test accepts; an inverted box (lo > hi) is never entered, as
+  // in the hierarchy over the boxes
+  for (int g = 0; g < (n + 15) / 16; ++g) {
+    float glo[3] = {INFINITY, INFINITY, INFINITY}, ghi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int i = 16 * g; i < std::min(n, 16 * g + 16); ++i) {
+      const float* b = boxes + 6 * (size_t)order[i].second;
+      float l[3], h[3];
+      for (int k = 0; k < 3; ++k) {
+        const bool bad = std::isnan(b[k]) || std::isnan(b[3 + k]);
+        l[k] = bad ? -INFINITY : b[k];
+        h[k] = bad ? INFINITY : b[3 + k];
+        glo[k] = std::min(glo[k], l[k]);
+        ghi[k] = std::max(ghi[k], h[k]);
+      }
+      DomCollapse::setSlot((*out)[n1 + i / 4], i & 3, l, h, order[i].second);
+    }
+    DomCollapse::setSlot((*out)[g / 4], g & 3, glo, ghi, g);
+  }
+}
+
 }  // namespace spray

@@ -49,6 +49,13 @@ void buildDomainBvh(const float* boxes, int n, std::vector<DomNode>* out);
 // leaf ~domain, unused slots empty (lo = +inf, hi = -inf, kEmptyChild).
 void buildDomainBvh4(const float* boxes, int n, std::vector<BvhNode4>* out);
 
+// The domains in groups of 4, 16 and 64 for the list pass: L1 nodes hold four
+// group-of-16 boxes each, then L2 nodes (index *l1_count + k) four domain boxes
+// each with child = the domain; the group of 16 behind slot c of L1 node q is
+// L2 nodes 4 * (4 * q + c) .. + 3.  Domains are in Morton order of their
+// centres, unused slots are empty boxes.
+void buildDomainGroups(const float* boxes, int n, std::vector<BvhNode4>* out, int* l1_count);
+
 struct BvhBuildResult {
   std::vector<BvhNode4> nodes;     // nodes[0] is the root
   std::vector<uint32_t> tri_order;  // leaf order -> original face index

@@ -186,6 +186,17 @@ struct ViewDev {
   int32_t bins_x;       // screen bins per image row
 };
 
+// Domain boxes for the list pass: buildDomainGroups' nodes, or with l1 = 0 none
+// (few domains: every box is tested; many: the hierarchy is descended).
+struct DomainGroups {
+  const BvhNode4* nodes;      // l1 nodes of four groups of 16, then l2 nodes of four domains
+  int l1, l2;
+  const BvhNode4* tree;       // 4-wide hierarchy over the boxes (tree_count 0: none)
+  int tree_count;
+};
+constexpr int kGroupMin = 16;    // fewer domains: the exact test of every box
+constexpr int kGroupMax = 1024;  // more: testing a sixteenth of them per ray costs more than the descent
+
 // Scheduling of one ray set into per-domain queues.
 struct SchedArgs {
   int shadow;                 // 0 radiance, 1 shadow rays
@@ -296,6 +307,50 @@ struct TraceArgs {
   Counters* ctr;
 };
 
+// A node as the whole-ray walks read it (made from BvhNode4 by
+// launchWalkNodes): the child boxes as centre c and half extent e per axis, so
+// that a 256-bit load brings both and the ray's direction signs select
+// nothing; children numbered scene-wide (inner nodes by node, leaves by
+// leaf-ordered triangle), so that a walk carries no per-domain base.
+struct alignas(128) WalkNode {
+  float cx[4], ex[4], cy[4], ey[4], cz[4], ez[4];
+  int32_t child[4];
+  int32_t pad[4];
+};
+static_assert(sizeof(WalkNode) == 128, "walk node must be one 128-byte line");
+// Triangles a walk can number: leaf references keep 28 bits of the first one.
+constexpr uint64_t kMaxWalkTris = (uint64_t)1 << 28;
+
+// Whole-ray walks in core (walk_rays.cu): a list pass writes every ray's
+// sorted domains, then each ray walks its list.
+struct RayWalkArgs {
+  SceneDev scene;
+  const uint32_t* count;      // rays (device)
+  const uint32_t* list;       // ray ids (sample for radiance, shadow id for shadow)
+  RayBuf rays;
+  ShadowBuf sh;
+  int shadow;
+  int slots;
+  DomainGroups groups;
+  const float* dboxes;        // domain boxes, 6 floats each
+  // primary rays: candidate domains per screen bin (null: not primary rays)
+  const uint32_t* bin_start;
+  const uint16_t* bin_ids;
+  const ViewDev* views;
+  int bin_shift;
+  // per ray of `list`: its entries in the arena, (domain, entry t bits) in walk order
+  uint2* arena;
+  unsigned long long* arena_top;
+  unsigned long long arena_cap;
+  uint2* list_ref;            // (first entry, entries)
+  const WalkNode* nodes;
+  uint32_t num_nodes, num_tris;
+  unsigned int* work;         // work counter of the walk (zeroed before launch)
+  uint64_t* ray_key;          // per sample: closest hit
+  float4* hit_ns;             // per sample: its Ns xyz, colour bits in w
+  Counters* ctr;
+};
+
 struct ShadeArgs {
   SceneDev scene;
   const uint32_t* count;      // alive rays
@@ -362,6 +417,11 @@ void launchTraceClosest(cudaStream_t s, const TraceArgs& a, int nblocks);
 // the records after out-of-core and domain-parallel launches.
 void launchResolve(cudaStream_t s, const TraceArgs& a, float4* hit_ns, int nblocks, bool interpolate);
 void launchTraceOccluded(cudaStream_t s, const TraceArgs& a, int nblocks);
+void launchWalkNodes(cudaStream_t s, const BvhNode4* nodes, uint32_t num_nodes, const DomainDev* domains, int D,
+                     WalkNode* out);
+void launchListDomains(cudaStream_t s, const RayWalkArgs& a, int num_sms);
+void launchWalkClosest(cudaStream_t s, const RayWalkArgs& a, int nblocks);
+void launchWalkOccluded(cudaStream_t s, const RayWalkArgs& a, int nblocks);
 void launchShade(cudaStream_t s, const ShadeArgs& a, int nblocks);
 // Stable compaction of flag[i] != 0 for i < n (n from *n_dev or n_host when
 // n_dev is null) into list, count and, optionally, index_of[i] (-1 if unset).

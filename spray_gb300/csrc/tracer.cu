@@ -357,6 +357,8 @@ void Tracer::freeScene() {
   devFree(d_segs);
   devFree(d_dnodes);
   devFree(d_dboxes);
+  devFree(d_groups);
+  group_l1 = group_l2 = 0;
   freeRounds();  // sized by the domain count
   bvh_dump.clear();
   dnode_count = 0;
@@ -366,6 +368,7 @@ void Tracer::freeScene() {
   bins_key.clear();  // new domain boxes
   devFree(d_domains);
   devFree(d_nodes);
+  devFree(d_wnodes);
   devFree(d_tris);
   devFree(d_faces);
   devFree(d_colors);
@@ -425,6 +428,10 @@ void Tracer::freeBuffers() {
   devFree(d_rec_key);
   devFree(d_rec_attr);
   devFree(d_work);
+  devFree(d_walk_work);
+  devFree(d_walk_top);
+  devFree(d_list_ref);
+  walk_work_cap = 0;
   devFree(d_scan_tmp);
   devFree(d_block_tmp);
   devFree(d_block_tmp2);
@@ -589,6 +596,7 @@ void Tracer::installScene(std::vector<DomainPack>& packs, const spray_gpu_light*
   }
   if (max_bvh_depth * 3 + 4 > 64) throw std::runtime_error("BVH deeper than the traversal stack");
   total_tris = nt;
+  total_nodes = nn;
   scene_bytes = nn * sizeof(BvhNode4) + 3 * nt * sizeof(float4) + 3 * nt * 4 + nvv * 4 + 3 * nvv * 4;
   // out-of-core when the cache holds fewer domains than the scene has
   size_t max_nodes = 0, max_tris = 0, max_verts = 0;
@@ -646,6 +654,13 @@ void Tracer::installScene(std::vector<DomainPack>& packs, const spray_gpu_light*
     devAlloc(&d_dnodes, dn.size());
     CK(cudaMemcpy(d_dnodes, dn.data(), dn.size() * sizeof(BvhNode4), cudaMemcpyHostToDevice));
   }
+  if (nd >= kGroupMin && nd <= kGroupMax) {
+    std::vector<BvhNode4> g;
+    buildDomainGroups(boxes.data(), nd, &g, &group_l1);
+    group_l2 = (int)g.size() - group_l1;
+    devAlloc(&d_groups, g.size());
+    CK(cudaMemcpy(d_groups, g.data(), g.size() * sizeof(BvhNode4), cudaMemcpyHostToDevice));
+  }
   std::vector<float> lf(13 * std::max(nl, 1), 0.f);
   for (int l = 0; l < nl; ++l) {
     float* q = &lf[13 * l];
@@ -656,6 +671,11 @@ void Tracer::installScene(std::vector<DomainPack>& packs, const spray_gpu_light*
       q[7 + c] = ls[l].edge1[c];
       q[10 + c] = ls[l].edge2[c];
     }
+  }
+  if (walksRays()) {
+    devAlloc(&d_wnodes, nn);
+    launchWalkNodes(stream, d_nodes, (uint32_t)nn, d_domains, nd, d_wnodes);
+    CK(cudaGetLastError());
   }
   devAlloc(&d_lights, lf.size());
   CK(cudaMemcpy(d_lights, lf.data(), lf.size() * 4, cudaMemcpyHostToDevice));
@@ -979,7 +999,7 @@ void Tracer::ensureBuffers(int64_t nsamples) {
   if (chunkSize((uint64_t)std::max<int64_t>(nsamples, 1024) * S, sched_chunks) >= 65536)
     throw std::runtime_error("too few scheduling chunks for 16-bit histogram counters");
   if (nsamples <= cap_samples && cap_entries >= needed_entries && frame_pixels <= image_cap &&
-      (int64_t)tiles.size() <= tiles_cap && fviews.size() <= views_cap)
+      (int64_t)tiles.size() <= tiles_cap && fviews.size() <= views_cap && walkLaunches() <= walk_work_cap)
     return;
   freeBuffers();
   ++buf_gen;
@@ -987,6 +1007,7 @@ void Tracer::ensureBuffers(int64_t nsamples) {
   int64_t NS = N * S;
   if (needed_entries == 0) needed_entries = (uint64_t)std::max<int64_t>(4 * N, 2 * NS);
   uint64_t E = needed_entries;
+  const bool queues = !walksRays();
   for (int k = 0; k < 2; ++k) {
     devAlloc(&rays[k].org, N);
     devAlloc(&rays[k].dir, N);
@@ -1014,16 +1035,29 @@ void Tracer::ensureBuffers(int64_t nsamples) {
   devAlloc(&d_shadow_flag, NS);
   devAlloc(&d_shadow_list, NS);
   devAlloc(&d_shadow_count, 1);
-  devAlloc(&d_arena, E);
-  devAlloc(&d_arena_top, 1);
-  devAlloc(&d_list_off, NS);
-  devAlloc(&d_list_cnt, NS);
-  devAlloc(&d_hist, (size_t)nkeys * sched_chunks);
-  devAlloc(&d_dstats, (size_t)D * cfg.list_size);
-  devAlloc(&d_entries, E);
-  if (cfg.debug_capture) devAlloc(&d_dbg_depth, E);  // list positions of the captured queues
-  devAlloc(&d_key_start, nkeys + 1);
-  devAlloc(&d_num_entries, 1);
+  if (queues) {
+    devAlloc(&d_arena, E);
+    devAlloc(&d_arena_top, 1);
+    devAlloc(&d_list_off, NS);
+    devAlloc(&d_list_cnt, NS);
+    devAlloc(&d_hist, (size_t)nkeys * sched_chunks);
+    devAlloc(&d_dstats, (size_t)D * cfg.list_size);
+    devAlloc(&d_entries, E);
+    if (cfg.debug_capture) devAlloc(&d_dbg_depth, E);  // list positions of the captured queues
+    devAlloc(&d_key_start, nkeys + 1);
+    devAlloc(&d_num_entries, 1);
+    devAlloc(&d_rec_key, E);
+    devAlloc(&d_rec_attr, E);
+    devAlloc(&d_work, kDepthBuckets);
+    scan_words = scanTmpWords(nkeys, sched_chunks);
+    devAlloc(&d_scan_tmp, scan_words);
+  } else {
+    devAlloc(&d_arena, E);
+    devAlloc(&d_list_ref, NS);
+    walk_work_cap = walkLaunches();
+    devAlloc(&d_walk_work, walk_work_cap);
+    devAlloc(&d_walk_top, walk_work_cap);
+  }
   if (learned()) {
     devAlloc(&d_pred, N);
     devAlloc(&d_lab, N);
@@ -1036,11 +1070,6 @@ void Tracer::ensureBuffers(int64_t nsamples) {
     devAlloc(&d_skey_start, nkeys + 1);
     devAlloc(&d_snum_entries, 1);
   }
-  devAlloc(&d_rec_key, E);
-  devAlloc(&d_rec_attr, E);
-  devAlloc(&d_work, kDepthBuckets);
-  scan_words = scanTmpWords(nkeys, sched_chunks);
-  devAlloc(&d_scan_tmp, scan_words);
   compact_blocks = num_sms * kCompactBlocksPerSm;
   devAlloc(&d_block_tmp, compact_blocks);
   devAlloc(&d_block_tmp2, compact_blocks);  // the shader's bounce counts per block
@@ -1138,6 +1167,48 @@ TraceArgs Tracer::traceArgs(int order_by_depth, int S) {
   return t;
 }
 
+RayWalkArgs Tracer::walkArgs(bool shadow, bool primary, int S) {
+  RayWalkArgs a{};
+  a.scene = sceneDev();
+  a.count = shadow ? d_shadow_count : d_alive_count;
+  a.list = shadow ? d_shadow_list : d_alive_list;
+  a.rays = rays[cur];
+  a.sh = sh;
+  a.slots = S;
+  a.shadow = shadow;
+  a.groups = domainGroups();
+  a.dboxes = d_dboxes;
+  if (primary && use_bins) {
+    a.bin_start = d_bin_start;
+    a.bin_ids = d_bin_ids;
+    a.views = d_views;
+    a.bin_shift = kBinShift;
+  }
+  a.arena = d_arena;
+  a.arena_top = d_walk_top + walk_launch;
+  a.arena_cap = cap_entries;
+  a.list_ref = d_list_ref;
+  a.nodes = d_wnodes;
+  a.num_nodes = (uint32_t)total_nodes;
+  a.num_tris = (uint32_t)total_tris;
+  a.work = d_walk_work + walk_launch++;
+  a.ray_key = d_ray_key;
+  a.hit_ns = d_hit_ns;
+  a.ctr = d_ctr;
+  return a;
+}
+
+// The frame's counters and image, and the walks' work counters.
+void Tracer::clearFrame() {
+  CK(cudaMemsetAsync(d_ctr, 0, sizeof(Counters), stream));
+  CK(cudaMemsetAsync(d_image, 0, (size_t)frame_pixels * sizeof(float4), stream));
+  walk_launch = 0;
+  if (walksRays()) {
+    CK(cudaMemsetAsync(d_walk_work, 0, walk_work_cap * sizeof(unsigned int), stream));
+    CK(cudaMemsetAsync(d_walk_top, 0, walk_work_cap * sizeof(unsigned long long), stream));
+  }
+}
+
 SceneDev Tracer::sceneDev() const {
   SceneDev s;
   s.domains = d_domains;
@@ -1213,6 +1284,49 @@ ShadeArgs Tracer::shadeArgs(int b, int S) {
   sa.num_lights = (int)lights.size();
   sa.ctr = d_ctr;
   return sa;
+}
+
+// A wave whose rays walk their domains themselves: per depth closest hits
+// (with the hits' colours and normals), shading, the shadow rays' compaction,
+// occlusion, retire and the next depth's alive list.
+void Tracer::traceWaveWalks(const Wave& w) {
+  const int S = std::max(slots(), 1);
+  const int nb_total = maxBounces();
+  const int nblk = num_sms * kStreamBlocksPerSm;
+  beginWave(w);
+  for (int b = 0; b < nb_total; ++b) {
+    cudaEvent_t s0 = poolEvent(), t0 = poolEvent(), t1 = poolEvent(), o0 = poolEvent(), o1 = poolEvent();
+    const RayWalkArgs wr = walkArgs(false, b == 0, S);
+    record(s0);
+    launchListDomains(stream, wr, num_sms);
+    record(t0);
+    launchWalkClosest(stream, wr, traceBlocks());
+    record(t1);
+    sched_events.push_back({s0, t0});
+    trace_events.push_back({t0, t1});
+    ShadeArgs sa = shadeArgs(b, S);
+    sa.blk_shadow = d_block_tmp;
+    sa.blk_next = d_block_tmp2;
+    launchShade(stream, sa, compact_blocks);
+    launchCompactCounted(stream, d_shadow_flag, d_alive_count, (uint32_t)S, d_shadow_list, d_shadow_count,
+                         nullptr, nullptr, d_block_tmp, compact_blocks);
+    const RayWalkArgs ws = walkArgs(true, false, S);
+    launchListDomains(stream, ws, num_sms);
+    record(o0);
+    launchWalkOccluded(stream, ws, traceBlocks());
+    record(o1);
+    occl_events.push_back({o0, o1});
+    launchRetire(stream, d_image, d_views, d_alive_list, d_alive_count, rays[cur], sh, d_shadow_flag, S, nblk);
+    launches += 7;
+    if (b + 1 < nb_total) {
+      launchCompactCounted(stream, d_next_flag, d_alive_count, 1, d_alive_list2, d_alive_count2, nullptr,
+                           d_alive_list, d_block_tmp2, compact_blocks);
+      std::swap(d_alive_list, d_alive_list2);
+      std::swap(d_alive_count, d_alive_count2);
+      launches += 1;
+      cur ^= 1;
+    }
+  }
 }
 
 void Tracer::traceWave(const Wave& w, bool capture) {
@@ -1858,9 +1972,11 @@ void Tracer::captureFrame() {
   CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed));
   capturing = true;
   try {
-    CK(cudaMemsetAsync(d_ctr, 0, sizeof(Counters), stream));
-    CK(cudaMemsetAsync(d_image, 0, (size_t)frame_pixels * sizeof(float4), stream));
-    for (const Wave& w : waves) traceWave(w, false);
+    clearFrame();
+    for (const Wave& w : waves) {
+      if (walksRays()) traceWaveWalks(w);
+      else traceWave(w, false);
+    }
   } catch (...) {
     capturing = false;
     cudaStreamEndCapture(stream, &g);
@@ -2090,8 +2206,7 @@ void Tracer::traceFrame(float* out, bool out_is_device, spray_gpu_stats* st) {
       trace_events = graph_trace;
       occl_events = graph_occl;
     } else {
-      CK(cudaMemsetAsync(d_ctr, 0, sizeof(Counters), stream));
-      CK(cudaMemsetAsync(d_image, 0, (size_t)frame_pixels * sizeof(float4), stream));
+      clearFrame();
       if (rounded()) {
         traceRounds();
       } else {
@@ -2099,6 +2214,7 @@ void Tracer::traceFrame(float* out, bool out_is_device, spray_gpu_stats* st) {
           const bool capture = cfg.debug_capture && k == 0;
           if (ooc && (cfg.schedule_policy == 2 || cfg.schedule_policy == 3) && !capture)
             traceWaveBatched(waves[k]);
+          else if (walksRays()) traceWaveWalks(waves[k]);
           else traceWave(waves[k], capture);
         }
       }

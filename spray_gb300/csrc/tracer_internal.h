@@ -167,6 +167,7 @@ class Tracer {
   void freeBuffers();
   void traceWave(const Wave& w, bool capture);
   void traceWaveBatched(const Wave& w);
+  void traceWaveWalks(const Wave& w);
   void beginWave(const Wave& w);
   ShadeArgs shadeArgs(int b, int S);
   void schedule(bool shadow, int order_by_depth, uint32_t* count, uint32_t* list, int S,
@@ -175,6 +176,15 @@ class Tracer {
   bool learned() const { return cfg.schedule_policy == 3; }
   // the non-speculative round loop (schedule_policy 5)
   bool rounded() const { return cfg.schedule_policy == 5; }
+  // In core, frames that need no per-domain queues walk whole rays
+  // (walk_rays.cu): the queues stay for the captured stage buffers, the pairs
+  // the proposal learns from, domain-parallel ranks, uncut visits (cull 0) and
+  // the per-bucket launches with their own visit counts.
+  bool walksRays() const {
+    return !ooc && !situ() && !learned() && !rounded() && cfg.cull && !cfg.debug_capture &&
+           cfg.bucket_launches != kDepthBuckets && total_tris < kMaxWalkTris;
+  }
+  RayWalkArgs walkArgs(bool shadow, bool primary, int S);
   void setupProposal();
   void freeProposal();
   mlp::ArenaSource arenaSource() const;
@@ -249,6 +259,8 @@ class Tracer {
   std::vector<spray_gpu_light> lights;
   DomainDev* d_domains = nullptr;
   BvhNode4* d_nodes = nullptr;
+  size_t total_nodes = 0;
+  WalkNode* d_wnodes = nullptr;  // d_nodes as the whole-ray walks read them
   float4* d_tris = nullptr;
   uint32_t* d_faces = nullptr;
   uint32_t* d_colors = nullptr;
@@ -284,6 +296,9 @@ class Tracer {
   BvhNode4* d_dnodes = nullptr;  // 4-wide hierarchy over the domain boxes
   float* d_dboxes = nullptr;     // domain boxes for the scheduler, 6 floats each
   int dnode_count = 0;
+  BvhNode4* d_groups = nullptr;  // the boxes in groups of 4, 16 and 64 (buildDomainGroups)
+  int group_l1 = 0, group_l2 = 0;
+  DomainGroups domainGroups() const { return DomainGroups{d_groups, group_l1, group_l2, d_dnodes, dnode_count}; }
   // screen bins of candidate domains for the primary rays
   static constexpr int kBinShift = 4;
   static constexpr int kBinSize = 1 << kBinShift;
@@ -363,6 +378,13 @@ class Tracer {
   uint64_t* d_rec_key = nullptr;
   float4* d_rec_attr = nullptr;
   unsigned int* d_work = nullptr;
+  // whole-ray walks: a work counter per launch of a frame, zeroed together
+  unsigned int* d_walk_work = nullptr;
+  unsigned long long* d_walk_top = nullptr;  // and an arena cursor
+  uint2* d_list_ref = nullptr;
+  size_t walk_work_cap = 0, walk_launch = 0;
+  size_t walkLaunches() const { return walksRays() ? waves.size() * (size_t)maxBounces() * 2 : 0; }
+  void clearFrame();
   uint32_t* d_scan_tmp = nullptr;
   uint8_t* d_dbg_depth = nullptr;  // debug capture only
   uint32_t* d_block_tmp2 = nullptr;  // compaction counts from the shader

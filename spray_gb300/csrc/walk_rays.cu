@@ -1,0 +1,661 @@
+// Closest hits and occlusion of whole rays, in core.
+//
+// When every domain is resident no domain has to be waited for, so a ray's
+// domains need no queues.  kListDomains writes each ray's (t, id)-sorted domain
+// list (the list Isector::isect makes, src/ooc/ooc_isector.h:116-174, exact slab
+// tests and all); then a thread walks a ray's listed domains front to back.
+// Radiance rays stop at the first domain that starts beyond the hit found;
+// shadow rays run first in the domain that spawned them (TContext::procShads2)
+// and stop at the first occluder.  The closest hit is the smallest packed
+// (t | triangle) key over the domains visited, as in the queue kernels
+// (trace.cu), so the image does not change; visits plus culled entries still
+// add up to the listed (ray, domain) pairs.
+//
+// The queues' partition (histogram, scan, scatter), the per-entry records and
+// the resolve pass fall away, and a ray sets up its walk once instead of once
+// per domain.  Path tracing 64 domains at 1920x1080, 16 spp, 5 bounces: lists
+// 1.72 -> 0.87 ms a frame (with the partition), closest hits with their colours
+// and normals 4.48 + 0.39 -> 4.00 ms, occlusion 1.71 -> 1.47 ms.
+#include "domain_walk.cuh"
+#include "kernels.cuh"
+#include "spray_math.cuh"
+#include "traverse.cuh"
+
+#ifndef SPRAY_WALK_REFILL
+#define SPRAY_WALK_REFILL 20
+#endif
+
+#ifndef SPRAY_WALK_SWITCH
+#define SPRAY_WALK_SWITCH 8
+#endif
+
+namespace spray {
+
+namespace {
+
+constexpr int kWalkThreads = 256;
+// Idle lanes a warp gathers before it fetches new rays for them (closest hits
+// of that frame at 12, 16, 20 and 24: 4.13, 4.05, 4.00 and 4.17 ms).
+constexpr int kRefill = SPRAY_WALK_REFILL;
+// Lanes at the end of a domain that the warp gathers before it moves them on.
+constexpr int kSwitch = SPRAY_WALK_SWITCH;
+// A node of the group table in shared memory takes 9 float4 instead of 8: the
+// four boxes of a node are read by all lanes at once, but near and far planes
+// differ by lane, and the exact tests read different nodes.
+constexpr int kNodeStride = 9;
+// Slack of the group test: the exact slab test rounds (plane - org) * inv and
+// this one fma(plane, inv, -org * inv); 2e-6 covers both by far.
+constexpr float kGroupSlack = 1.000002f;
+
+// Floats as integers that order like them (negative t: the ray starts inside
+// the box; -0 was made +0 by the caller).
+__device__ __forceinline__ uint32_t orderedBits(float t) {
+  const uint32_t u = __float_as_uint(t);
+  return u ^ ((u & 0x80000000u) ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ float orderedFloat(uint32_t k) {
+  return __uint_as_float(k ^ ((k & 0x80000000u) ? 0x80000000u : 0xffffffffu));
+}
+
+// Per-lane sorted list of (entry t, domain), 64-bit keys in local memory.
+struct DomainList {
+  uint64_t key[kMaxList];
+  int n = 0;
+  __device__ __forceinline__ void insert(float t, int d, Counters* ctr) {
+    const uint64_t k = ((uint64_t)orderedBits(t + 0.0f) << 32) | (uint32_t)d;
+    if (n == kMaxList) {
+      atomicAdd(&ctr->list_overflows, 1ull);
+      return;  // the frame is refused
+    }
+    int j = n++;
+    while (j > 0 && key[j - 1] > k) {
+      key[j] = key[j - 1];
+      --j;
+    }
+    key[j] = k;
+  }
+};
+
+// The four boxes of a table node against the ray: bit k set when box k may be hit.
+__device__ __forceinline__ uint32_t boxMask(const float4* p, const BoxRay& r, float t1) {
+  float tn[4];
+  bool h[4];
+  testBoxes(p[r.sx], p[r.sx ^ 1], p[2 + r.sy], p[3 - r.sy], p[4 + r.sz], p[5 - r.sz], r, kRayEpsilon, t1, kGroupSlack,
+            tn, h);
+  return (h[0] ? 1u : 0u) | (h[1] ? 2u : 0u) | (h[2] ? 4u : 0u) | (h[3] ? 8u : 0u);
+}
+
+// Calls consider(d) for a superset of the domains whose boxes the ray enters
+// within (1e-3, t1], 64 at a time: every group of 16 is tested, the four nodes
+// of a group some lane may enter are tested by all of the warp's lanes that
+// may, at the same addresses, and then each lane goes through its own bits.
+// Against the descent of a hierarchy (domain_walk.cuh) that is more tests and
+// far fewer instructions, for the lanes of a warp stay together.
+template <class F>
+__device__ __forceinline__ void groupDomains(const float4* table, int n1, int n2, const BoxRay& r, float t1,
+                                             F&& consider) {
+  const float4* l2 = table + n1 * kNodeStride;
+  for (int q = 0; q < n1; ++q) {
+    const uint32_t groups = boxMask(table + q * kNodeStride, r, t1);
+    uint32_t bits[2] = {0u, 0u};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (!(groups & (1u << c))) continue;
+      const int first = 16 * q + 4 * c;
+      uint32_t m = 0;
+#pragma unroll 1
+      for (int j = 0; j < 4 && first + j < n2; ++j)
+        m |= boxMask(l2 + (first + j) * kNodeStride, r, t1) << (4 * j);
+      bits[c >> 1] |= m << (16 * (c & 1));
+    }
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+      for (uint32_t m = bits[w]; m; m &= m - 1) {
+        const int b = 32 * w + __ffs(m) - 1;
+        consider(reinterpret_cast<const int*>(l2 + (16 * q + (b >> 2)) * kNodeStride + 6)[b & 3]);
+      }
+  }
+}
+
+__device__ __forceinline__ uint32_t warpScan(uint32_t v, uint32_t* total) {
+  const int lane = threadIdx.x & 31;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  *total = __shfl_sync(0xffffffffu, x, 31);
+  return x - v;
+}
+
+__device__ __forceinline__ uint32_t lanesBelowMask() {
+  uint32_t m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
+
+enum ListKind { kListBounce, kListPrimary, kListShadow };
+
+}  // namespace
+
+// The sorted domain list of every ray, into the arena (one atomic per block of
+// 256 rays), the group table in shared memory (kNodeStride).
+template <int kKind>
+__global__ void __launch_bounds__(kWalkThreads) kListDomains(RayWalkArgs a) {
+  extern __shared__ float4 table[];
+  __shared__ uint32_t wsum[kWalkThreads / 32];
+  __shared__ unsigned long long wbase;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n1 = a.groups.l1, n2 = a.groups.l2, D = a.scene.num_domains;
+  if (kKind != kListPrimary) {
+    const float4* src = reinterpret_cast<const float4*>(a.groups.nodes);
+    for (int k = threadIdx.x; k < 8 * (n1 + n2); k += blockDim.x) table[(k >> 3) * kNodeStride + (k & 7)] = src[k];
+    __syncthreads();
+  }
+  const uint32_t n = *a.count;
+  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = base + threadIdx.x;
+    const bool active = i < n;
+    DomainList list;
+    int origin = -1;
+    uint32_t emit = 0;
+    if (active) {
+      const uint32_t rid = a.list[i];
+      V3 org, dir;
+      float t1 = INFINITY;
+      if (kKind == kListShadow) {
+        const float4 hp = a.sh.hitpos[rid / a.slots], d4 = a.sh.dir[rid];
+        org = v3(hp.x, hp.y, hp.z);
+        origin = __float_as_int(hp.w);
+        dir = v3(d4.x, d4.y, d4.z);
+        t1 = d4.w;
+      } else {
+        const float4 o4 = a.rays.org[rid], d4 = a.rays.dir[rid];
+        org = v3(o4.x, o4.y, o4.z);
+        dir = v3(d4.x, d4.y, d4.z);
+        a.ray_key[rid] = kNoHit;
+      }
+      const V3 inv = v3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
+      auto consider = [&](int d) {
+        float t;
+        if (slabTest(a.dboxes + 6 * d, a.dboxes + 6 * d + 3, org, inv, kRayEpsilon, t1, &t)) list.insert(t, d, a.ctr);
+      };
+      if (kKind == kListPrimary) {
+        // the domains whose projected box covers this pixel's bin
+        const int pid = a.rays.pixid[rid];
+        const ViewDev& vw = a.views[a.rays.view[rid]];
+        const int bx = (pid % vw.image_w) >> a.bin_shift, by = (pid / vw.image_w) >> a.bin_shift;
+        const int bin = vw.bin_base + by * vw.bins_x + bx;
+        const uint32_t c1 = a.bin_start[bin + 1];
+        for (uint32_t c = a.bin_start[bin]; c < c1; ++c) consider((int)a.bin_ids[c]);
+      } else if (n1 > 0) {
+        groupDomains(table, n1, n2, makeBoxRay(org, inv), t1, consider);
+      } else if (a.groups.tree_count > 0) {
+        descendDomains(reinterpret_cast<const float4*>(a.groups.tree), a.groups.tree_count, org, inv, t1, consider, a.ctr);
+      } else {
+        for (int d = 0; d < D; ++d) consider(d);
+      }
+      emit = (uint32_t)list.n;
+      if (kKind == kListShadow) {
+        emit += 1u;
+        for (int j = 0; j < list.n; ++j)
+          if ((int)(uint32_t)list.key[j] == origin) --emit;
+      }
+    }
+    uint32_t total;
+    uint32_t pos = warpScan(emit, &total);
+    if (lane == 31) wsum[warp] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t run = 0;
+      for (int w = 0; w < kWalkThreads / 32; ++w) {
+        const uint32_t v = wsum[w];
+        wsum[w] = run;
+        run += v;
+      }
+      unsigned long long b = run ? atomicAdd(a.arena_top, (unsigned long long)run) : 0ull;
+      if (b + run > a.arena_cap) {
+        atomicAdd(&a.ctr->arena_overflows, 1ull);  // the frame is traced again with a larger arena
+        b = ~0ull;
+      }
+      wbase = b;
+    }
+    __syncthreads();
+    const unsigned long long b = wbase;
+    pos += wsum[warp];
+    __syncthreads();  // wsum and wbase are rewritten by the next round
+    if (!active) continue;
+    const bool fits = b != ~0ull;
+    a.list_ref[i] = make_uint2(fits ? (uint32_t)(b + pos) : 0u, fits ? emit : 0u);
+    if (!fits) continue;
+    uint2* out = a.arena + b + pos;
+    if (kKind == kListShadow) *out++ = make_uint2((uint32_t)origin, 0u);
+    for (int j = 0; j < list.n; ++j) {
+      const uint64_t k = list.key[j];
+      if (kKind == kListShadow && (int)(uint32_t)k == origin) continue;
+      *out++ = make_uint2((uint32_t)k, __float_as_uint(orderedFloat((uint32_t)(k >> 32))));
+    }
+  }
+}
+
+namespace {
+
+// A ray against walk nodes.  Per axis a box spans tc -+ h with tc =
+// fma(c, inv, -org * inv) and h = fma(e, |inv|, pad): pad takes the rounding of
+// org * inv (BoxRay), and e was rounded up by more than the roundings of c, tc
+// and h that are relative to the box; what is left is relative to the plane's
+// own distance, kBoxSlack's part.
+struct WalkRay {
+  V3 org;
+  V3 inv, c, pad;
+  RayShear sh;
+};
+
+__device__ __forceinline__ WalkRay makeWalkRay(V3 org, V3 dir) {
+  const BoxRay b = makeBoxRay(org, v3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z));
+  WalkRay r;
+  r.org = org;
+  r.inv = b.inv;
+  r.c = v3(-(org.x * b.inv.x), -(org.y * b.inv.y), -(org.z * b.inv.z));
+  r.pad = v3(boxPad(org.x * b.inv.x, 1.0f / dir.x), boxPad(org.y * b.inv.y, 1.0f / dir.y),
+             boxPad(org.z * b.inv.z, 1.0f / dir.z));
+  r.sh = makeShear(dir);
+  return r;
+}
+
+// 32 bytes through the read-only cache in one request: a warp's lanes are at
+// different nodes, so the requests of a walk, not its bytes, load L1.
+__device__ __forceinline__ void load256(const float* p, float* v) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(p));
+}
+
+__device__ __forceinline__ unsigned long long f2add(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f2sub(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f2fmaPacked(unsigned long long a, unsigned long long b,
+                                                          unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// The four children of a walk node: entry distances, hits and references.
+__device__ __forceinline__ int4 testNode(const WalkNode* __restrict__ nodes, int node, const WalkRay& r, float tfar,
+                                         float tn[4], bool hit[4]) {
+  const WalkNode* p = nodes + node;
+  float x[8], y[8], z[8];
+  load256(p->cx, x);
+  load256(p->cy, y);
+  load256(p->cz, z);
+  const int4 ch = __ldg(reinterpret_cast<const int4*>(p->child));
+  auto span = [](const float* v, int h, float inv, float c, float pad, float2* near, float2* far) {
+    const unsigned long long tc = f2fmaPacked(f2pack(v[2 * h], v[2 * h + 1]), f2pack(inv, inv), f2pack(c, c));
+    const unsigned long long hw =
+        f2fmaPacked(f2pack(v[4 + 2 * h], v[5 + 2 * h]), f2pack(fabsf(inv), fabsf(inv)), f2pack(pad, pad));
+    *near = f2unpack(f2sub(tc, hw));
+    *far = f2unpack(f2add(tc, hw));
+  };
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float2 nx, fx, ny, fy, nz, fz;
+    span(x, h, r.inv.x, r.c.x, r.pad.x, &nx, &fx);
+    span(y, h, r.inv.y, r.c.y, r.pad.y, &ny, &fy);
+    span(z, h, r.inv.z, r.c.z, r.pad.z, &nz, &fz);
+    const float t00 = fmaxf(max3(nx.x, ny.x, nz.x), kRayEpsilon);
+    const float t01 = fmaxf(max3(nx.y, ny.y, nz.y), kRayEpsilon);
+    const float t10 = fminf(min3(fx.x, fy.x, fz.x), tfar) * kBoxSlack;
+    const float t11 = fminf(min3(fx.y, fy.y, fz.y), tfar) * kBoxSlack;
+    tn[2 * h] = t00;
+    tn[2 * h + 1] = t01;
+    hit[2 * h] = t00 <= t10;
+    hit[2 * h + 1] = t01 <= t11;
+  }
+  return ch;
+}
+
+__device__ __forceinline__ void addCounts(unsigned long long* dst, uint32_t v, int lane) {
+  unsigned long long s = v;
+  for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0 && s) atomicAdd(dst, s);
+}
+
+// Work indices for the idle lanes of a warp (mask), one atomic; n when the
+// counter has run out.  *exhausted is set once it has.
+__device__ __forceinline__ uint32_t fetchWork(unsigned int* work, uint32_t idle, uint32_t n, bool* exhausted) {
+  const uint32_t need = __popc(idle);
+  uint32_t base = 0;
+  if ((threadIdx.x & 31) == 0) base = atomicAdd(work, need);
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (base + need >= n) *exhausted = true;
+  return base + __popc(idle & lanesBelowMask());
+}
+
+}  // namespace
+
+// Closest hits.  The lanes of a warp walk independently: each is at an inner
+// node, at a triangle, at the end of a domain, or idle, and every round of the
+// warp runs the step most lanes are at.  Idle lanes fetch new rays once
+// kRefill of them have gathered.
+//
+// Rays walk 12 nodes and 4 triangles each, unevenly: lanes that take whole
+// leaves and node runs together leave two thirds of a warp idle (7 to 13 of 32
+// lanes, 5.8 ms a frame; with refilling but without the rounds 6.8 ms).  In
+// rounds 15 to 19 lanes are active, and L1's requests (a node in four, 32 bytes
+// each: seven of 16 bytes took 4.35 ms) and their latency bound the kernel.
+__global__ void __launch_bounds__(kWalkThreads, 4) kWalkClosest(RayWalkArgs a) {
+  const uint32_t n = *a.count;
+  const int lane = threadIdx.x & 31;
+  uint32_t visits = 0, culled = 0, nnodes = 0, ntris = 0;
+  bool has = false, exhausted = n == 0;
+  uint32_t rid = 0, next = 0, end = 0;
+  WalkRay r{};
+  uint64_t best_key = kNoHit;
+  float best_t = 0.f, best_u = 0.f, best_v = 0.f;
+  int best_dom = 0, dom = 0;
+  uint2 stack[kStack];
+  int sp = 0, cur = kDone;
+  uint32_t steps = 0;
+  auto pop = [&]() -> int {
+    while (sp > 0) {
+      const uint2 e = stack[--sp];
+      if (__uint_as_float(e.y) <= best_t) return (int)e.x;
+    }
+    return kDone;
+  };
+  while (true) {
+    const uint32_t inner = __ballot_sync(0xffffffffu, cur >= 0);
+    const uint32_t leaf = __ballot_sync(0xffffffffu, cur < 0 && cur != kDone);
+    const uint32_t idle = __ballot_sync(0xffffffffu, !has);
+    const int ni = __popc(inner), nl = __popc(leaf), nd = __popc(idle), ne = 32 - ni - nl - nd;
+    if (nd == 32 || (nd >= kRefill && !exhausted)) {
+      if (!has && best_key != kNoHit) {
+        // the finished ray's hit: TriMeshBuffer::updateIntersection
+        // (src/render/trimesh_buffer.cc:328-360)
+        const DomainDev* p = a.scene.domains + best_dom;
+        const uint32_t* f = a.scene.faces + 3 * ((size_t)p->face_base + ((uint32_t)best_key - p->gprim_base));
+        const uint32_t i0 = f[0], i1 = f[1], i2 = f[2];
+        const uint32_t* colors = a.scene.colors + p->vert_base;
+        const float* nb = a.scene.normals + 3 * (size_t)p->vert_base;
+        const uint32_t col = interpolateColor(colors[i0], colors[i1], colors[i2], best_u, best_v);
+        const V3 ns = interpolateNormal(
+            v3(nb[3 * (size_t)i0], nb[3 * (size_t)i0 + 1], nb[3 * (size_t)i0 + 2]),
+            v3(nb[3 * (size_t)i1], nb[3 * (size_t)i1 + 1], nb[3 * (size_t)i1 + 2]),
+            v3(nb[3 * (size_t)i2], nb[3 * (size_t)i2 + 1], nb[3 * (size_t)i2 + 2]), best_u, best_v);
+        a.ray_key[rid] = best_key;
+        a.hit_ns[rid] = make_float4(ns.x, ns.y, ns.z, __uint_as_float(col));
+        best_key = kNoHit;
+      }
+      if (exhausted) break;  // every lane is idle
+      __syncwarp();
+      const uint32_t i = fetchWork(a.work, idle, n, &exhausted);
+      if (!has && i < n) {
+        const uint2 ref = a.list_ref[i];
+        if (ref.y > 0) {
+          rid = a.list[i];
+          next = ref.x;
+          end = ref.x + ref.y;
+          const float4 o4 = a.rays.org[rid], d4 = a.rays.dir[rid];
+          r = makeWalkRay(v3(o4.x, o4.y, o4.z), v3(d4.x, d4.y, d4.z));
+          best_t = __int_as_float(0x7f800000);
+          steps = 0;
+          sp = 0;
+          cur = kDone;
+          has = true;
+        }
+      }
+    } else if (ne >= kSwitch || (ni == 0 && nl == 0)) {
+      if (has && cur == kDone) {
+        // the next domain of the list; the rest start beyond the hit once one does
+        has = next < end;
+        if (has) {
+          const uint2 e = a.arena[next];
+          if (__uint_as_float(e.y) > best_t) {
+            culled += end - next;
+            has = false;
+          } else {
+            ++next;
+            ++visits;
+            dom = (int)e.x;
+            cur = a.scene.domains[dom].node_base;
+          }
+        }
+        if (!has) nnodes += steps;
+      }
+    } else if (ni >= nl) {
+      if (cur >= 0) {
+        if (++steps > (uint32_t)kMaxSteps || (uint32_t)cur >= a.num_nodes || sp > kStack - 3) {
+          raise(a.ctr, (uint32_t)cur >= a.num_nodes ? kErrBadNode : kErrTraversalBound);
+          cur = kDone;
+          next = end;
+        } else {
+          float tn[4];
+          bool hit[4];
+          const int4 ch = testNode(a.nodes, cur, r, best_t, tn, hit);
+          // nearest child first, the others in slot order (as in traverseClosest)
+          uint32_t k[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) k[c] = hit[c] ? (__float_as_uint(tn[c]) & ~3u) | (uint32_t)c : 0xffffffffu;
+          const uint32_t kmin = min(__vimin3_u32(k[0], k[1], k[2]), k[3]);
+          if (kmin != 0xffffffffu) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (hit[c] && k[c] != kmin) stack[sp++] = make_uint2((uint32_t)childAt(ch, c), k[c] & ~3u);
+            cur = childAt(ch, (int)(kmin & 3u));
+          } else {
+            cur = pop();
+          }
+        }
+      }
+    } else if (cur < 0 && cur != kDone) {
+      // the leaf's first triangle; the leaf reference moves on to the rest
+      const uint32_t v = ~(uint32_t)cur;
+      const uint32_t first = v >> 3;
+      if (first >= a.num_tris) {
+        raise(a.ctr, kErrBadNode);
+        cur = kDone;
+        sp = 0;
+        next = end;
+      } else {
+        ++ntris;
+        const float4* tp = a.scene.tris + 3 * (size_t)first;
+        const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+        float t, u, vv;
+        if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
+                              kRayEpsilon, __int_as_float(0x7f800000), &t, &u, &vv)) {
+          const uint64_t key = packHitKey(t, a.scene.domains[dom].gprim_base + __float_as_uint(ta.w));
+          if (key < best_key) {
+            best_key = key;
+            best_t = t;
+            best_u = u;
+            best_v = vv;
+            best_dom = dom;
+          }
+        }
+        cur = (v & 7u) ? (int)~(v + 7u) : pop();
+      }
+    }
+  }
+  addCounts(&a.ctr->visits_radiance, visits, lane);
+  addCounts(&a.ctr->visits_culled, culled, lane);
+  addCounts(&a.ctr->nodes_radiance, nnodes, lane);
+  addCounts(&a.ctr->tris_radiance, ntris, lane);
+}
+
+// Occlusion, in the same rounds.
+__global__ void __launch_bounds__(kWalkThreads, 4) kWalkOccluded(RayWalkArgs a) {
+  const uint32_t n = *a.count;
+  const int lane = threadIdx.x & 31;
+  uint32_t visits = 0, nnodes = 0, ntris = 0;
+  bool has = false, exhausted = n == 0;
+  uint32_t rid = 0, next = 0, end = 0;
+  WalkRay r{};
+  float tfar = 0.f;
+  int stack[kStack];
+  int sp = 0, cur = kDone;
+  uint32_t steps = 0;
+  while (true) {
+    const uint32_t inner = __ballot_sync(0xffffffffu, cur >= 0);
+    const uint32_t leaf = __ballot_sync(0xffffffffu, cur < 0 && cur != kDone);
+    const uint32_t idle = __ballot_sync(0xffffffffu, !has);
+    const int ni = __popc(inner), nl = __popc(leaf), nd = __popc(idle), ne = 32 - ni - nl - nd;
+    if (nd == 32 && exhausted) break;
+    if (nd >= kRefill && !exhausted) {
+      const uint32_t i = fetchWork(a.work, idle, n, &exhausted);
+      if (!has && i < n) {
+        const uint2 ref = a.list_ref[i];
+        if (ref.y > 0) {
+          rid = a.list[i];
+          next = ref.x;
+          end = ref.x + ref.y;
+          const float4 hp = a.sh.hitpos[rid / a.slots], d4 = a.sh.dir[rid];
+          r = makeWalkRay(v3(hp.x, hp.y, hp.z), v3(d4.x, d4.y, d4.z));
+          tfar = d4.w;
+          steps = 0;
+          sp = 0;
+          has = true;
+          ++visits;
+          cur = a.scene.domains[a.arena[next++].x].node_base;
+        }
+      }
+    } else if (ne >= kSwitch || (ni == 0 && nl == 0)) {
+      if (has && cur == kDone) {
+        has = next < end;
+        if (has) {
+          ++visits;
+          cur = a.scene.domains[a.arena[next++].x].node_base;
+        } else {
+          nnodes += steps;
+          a.sh.occluded[rid] = 0;
+        }
+      }
+    } else if (ni >= nl) {
+      if (cur >= 0) {
+        if (++steps > (uint32_t)kMaxSteps || (uint32_t)cur >= a.num_nodes || sp > kStack - 3) {
+          raise(a.ctr, (uint32_t)cur >= a.num_nodes ? kErrBadNode : kErrTraversalBound);
+          cur = kDone;
+          sp = 0;
+          next = end;
+        } else {
+          float tn[4];
+          bool hit[4];
+          const int4 ch = testNode(a.nodes, cur, r, tfar, tn, hit);
+          int nx = kDone;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (!hit[c]) continue;
+            if (nx != kDone) stack[sp++] = nx;
+            nx = childAt(ch, c);
+          }
+          cur = nx != kDone ? nx : (sp > 0 ? stack[--sp] : kDone);
+        }
+      }
+    } else if (cur < 0 && cur != kDone) {
+      const uint32_t v = ~(uint32_t)cur;
+      const uint32_t first = v >> 3;
+      if (first >= a.num_tris) {
+        raise(a.ctr, kErrBadNode);
+        cur = kDone;
+        sp = 0;
+        next = end;
+      } else {
+        ++ntris;
+        const float4* tp = a.scene.tris + 3 * (size_t)first;
+        const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+        float t, u, vv;
+        if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
+                              kRayEpsilon, tfar, &t, &u, &vv)) {
+          nnodes += steps;
+          a.sh.occluded[rid] = 1;
+          has = false;
+          sp = 0;
+          cur = kDone;
+        } else {
+          cur = (v & 7u) ? (int)~(v + 7u) : (sp > 0 ? stack[--sp] : kDone);
+        }
+      }
+    }
+  }
+  addCounts(&a.ctr->visits_shadow, visits, lane);
+  addCounts(&a.ctr->nodes_shadow, nnodes, lane);
+  addCounts(&a.ctr->tris_shadow, ntris, lane);
+}
+
+// One thread per node.  The half extent is rounded up, then widened by 2^-21.
+__global__ void kWalkNodes(const BvhNode4* __restrict__ nodes, uint32_t num_nodes, const DomainDev* __restrict__ domains,
+                           int D, WalkNode* out) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= num_nodes) return;
+  int lo = 0, hi = D - 1;  // the last domain whose first node is <= k
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if ((uint32_t)domains[mid].node_base <= k) lo = mid;
+    else hi = mid - 1;
+  }
+  const int node_base = domains[lo].node_base;
+  const uint32_t tri_base = (uint32_t)domains[lo].tri_base;
+  const BvhNode4 nd = nodes[k];
+  WalkNode w;
+  auto axis = [&](const float* l, const float* h, float* c, float* e) {
+    for (int q = 0; q < 4; ++q) {
+      c[q] = 0.0f;
+      e[q] = -INFINITY;
+      if (nd.child[q] == kEmptyChild) continue;
+      c[q] = 0.5f * l[q] + 0.5f * h[q];
+      e[q] = __fmul_ru(fmaxf(__fsub_ru(h[q], c[q]), __fsub_ru(c[q], l[q])), 1.0000005f);
+      if (!isfinite(c[q]) || !isfinite(e[q])) {  // infinite or NaN planes: everything along this axis
+        c[q] = 0.0f;
+        e[q] = INFINITY;
+      }
+    }
+  };
+  axis(nd.lox, nd.hix, w.cx, w.ex);
+  axis(nd.loy, nd.hiy, w.cy, w.ey);
+  axis(nd.loz, nd.hiz, w.cz, w.ez);
+  for (int q = 0; q < 4; ++q) {
+    const int c = nd.child[q];
+    if (c == kEmptyChild) w.child[q] = kEmptyChild;
+    else if (c >= 0) w.child[q] = c + node_base;
+    else w.child[q] = (int)~(~(uint32_t)c + (tri_base << 3));
+    w.pad[q] = 0;
+  }
+  out[k] = w;
+}
+
+void launchWalkNodes(cudaStream_t s, const BvhNode4* nodes, uint32_t num_nodes, const DomainDev* domains, int D,
+                     WalkNode* out) {
+  if (num_nodes > 0) kWalkNodes<<<(num_nodes + 127) / 128, 128, 0, s>>>(nodes, num_nodes, domains, D, out);
+}
+
+template <int kKind>
+static void launchLists(cudaStream_t s, const RayWalkArgs& a, int num_sms) {
+  // the largest table (1024 domains) takes 39 KB; primary rays read their bin's domains instead
+  static_assert((kGroupMax / 64 + kGroupMax / 4) * kNodeStride * 16 <= 48 * 1024, "group table in shared memory");
+  const size_t bytes = kKind == kListPrimary ? 0 : (size_t)(a.groups.l1 + a.groups.l2) * kNodeStride * sizeof(float4);
+  kListDomains<kKind><<<num_sms * 8, kWalkThreads, bytes, s>>>(a);
+}
+
+void launchListDomains(cudaStream_t s, const RayWalkArgs& a, int num_sms) {
+  if (a.shadow) launchLists<kListShadow>(s, a, num_sms);
+  else if (a.bin_start) launchLists<kListPrimary>(s, a, num_sms);
+  else launchLists<kListBounce>(s, a, num_sms);
+}
+
+void launchWalkClosest(cudaStream_t s, const RayWalkArgs& a, int nblocks) {
+  kWalkClosest<<<nblocks, kWalkThreads, 0, s>>>(a);
+}
+
+void launchWalkOccluded(cudaStream_t s, const RayWalkArgs& a, int nblocks) {
+  kWalkOccluded<<<nblocks, kWalkThreads, 0, s>>>(a);
+}
+
+}  // namespace spray
