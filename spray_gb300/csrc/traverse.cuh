@@ -143,31 +143,6 @@ __device__ __forceinline__ void raise(Counters* ctr, unsigned long long bit) {
 
 // Marks the end of a traversal (never a child reference: empty slots are skipped).
 constexpr int kDone = (int)kEmptyChild;
-// Inner-node expansions a lane runs before its warp checks for idle lanes.
-constexpr int kNodeBudget = 8;
-
-// Traversal state of one (ray, domain) entry, kept across the rounds of the
-// persistent loop so that a lane can be refilled as soon as its entry ends.
-struct Walk {
-  const BvhNode4* nodes;
-  const float4* tris;
-  int num_nodes, num_tris;
-  int cur, sp, steps;
-};
-
-__device__ __forceinline__ Walk startWalk(const SceneDev& sc, const DomainDev& dom) {
-  Walk w;
-  const DomArrays g = domArrays(sc, dom);
-  w.nodes = g.nodes;
-  w.tris = g.tris;
-  w.num_nodes = dom.num_nodes;
-  w.num_tris = dom.num_tris;
-  w.cur = 0;
-  w.sp = 0;
-  w.steps = 0;
-  return w;
-}
-
 // Closest hit in one domain.  best_key enters as the key to beat and leaves as
 // the best found; returns true when this domain improved it.
 //
