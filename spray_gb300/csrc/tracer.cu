@@ -1252,7 +1252,7 @@ void Tracer::beginWave(const Wave& w) {
   launches += 1;
   if (cull.live) {
     launchCompact(stream, d_next_flag, nullptr, 1, (uint64_t)w.samples, d_alive_list, d_alive_count, nullptr,
-                  d_block_tmp, compact_blocks);
+                  d_block_tmp, std::min<int64_t>(compact_blocks, (w.samples + 255) / 256));
     launchCountCulled(stream, d_alive_count, w.samples, d_ctr);
     launches += 4;
   }
@@ -1287,13 +1287,17 @@ ShadeArgs Tracer::shadeArgs(int b, int S) {
 void Tracer::traceWaveWalks(const Wave& w) {
   const int S = std::max(slots(), 1);
   const int nb_total = maxBounces();
-  const int nblk = num_sms * kStreamBlocksPerSm;
+  // blocks of 256 threads for at most n items: the full grid of a large wave,
+  // fewer for a small one, whose launches would mostly start empty blocks
+  auto blocks = [&](int64_t n, int per_sm) { return (int)std::min<int64_t>((n + 255) / 256, num_sms * per_sm); };
+  const int nr = blocks(w.samples, kStreamBlocksPerSm), ns = blocks(w.samples * S, kStreamBlocksPerSm);
+  const int ncr = blocks(w.samples, kCompactBlocksPerSm);
   beginWave(w);
   for (int b = 0; b < nb_total; ++b) {
     cudaEvent_t s0 = poolEvent(), t0 = poolEvent(), t1 = poolEvent(), o0 = poolEvent(), o1 = poolEvent();
     const RayWalkArgs wr = walkArgs(false, b == 0, S);
     record(s0);
-    launchListDomains(stream, wr, num_sms);
+    launchListDomains(stream, wr, nr);
     record(t0);
     launchWalkClosest(stream, wr, traceBlocks());
     record(t1);
@@ -1302,20 +1306,20 @@ void Tracer::traceWaveWalks(const Wave& w) {
     ShadeArgs sa = shadeArgs(b, S);
     sa.blk_shadow = d_block_tmp;
     sa.blk_next = d_block_tmp2;
-    launchShade(stream, sa, compact_blocks);
+    launchShade(stream, sa, ncr);
     launchCompactCounted(stream, d_shadow_flag, d_alive_count, (uint32_t)S, d_shadow_list, d_shadow_count,
-                         nullptr, nullptr, d_block_tmp, compact_blocks);
+                         nullptr, nullptr, d_block_tmp, ncr);
     const RayWalkArgs ws = walkArgs(true, false, S);
-    launchListDomains(stream, ws, num_sms);
+    launchListDomains(stream, ws, ns);
     record(o0);
     launchWalkOccluded(stream, ws, traceBlocks());
     record(o1);
     occl_events.push_back({o0, o1});
-    launchRetire(stream, d_image, d_views, d_alive_list, d_alive_count, rays[cur], sh, d_shadow_flag, S, nblk);
+    launchRetire(stream, d_image, d_views, d_alive_list, d_alive_count, rays[cur], sh, d_shadow_flag, S, nr);
     launches += 7;
     if (b + 1 < nb_total) {
       launchCompactCounted(stream, d_next_flag, d_alive_count, 1, d_alive_list2, d_alive_count2, nullptr,
-                           d_alive_list, d_block_tmp2, compact_blocks);
+                           d_alive_list, d_block_tmp2, ncr);
       std::swap(d_alive_list, d_alive_list2);
       std::swap(d_alive_count, d_alive_count2);
       launches += 1;

@@ -329,6 +329,16 @@ __device__ __forceinline__ void addCounts(unsigned long long* dst, uint32_t v, i
   if (lane == 0 && s) atomicAdd(dst, s);
 }
 
+// Lanes of each warp that take rays.  With fewer rays than half the launch's
+// lanes they are spread over its warps, for a warp's rounds serve one step at a
+// time: 6144 rays in 192 full warps walk for 51 us, spread over all for 35 us.  Full
+// warps keep constants for the lane counts (variable ones cost 4 %).
+__device__ __forceinline__ int walkLanes(uint32_t n) {
+  const uint32_t warps = gridDim.x * (kWalkThreads / 32);
+  const uint32_t lanes = (n + warps - 1) / warps;
+  return lanes > 16u ? 32 : (int)lanes;
+}
+
 // Work indices for the idle lanes of a warp (mask), one atomic; n when the
 // counter has run out.  *exhausted is set once it has.
 __device__ __forceinline__ uint32_t fetchWork(unsigned int* work, uint32_t idle, uint32_t n, bool* exhausted) {
@@ -352,10 +362,13 @@ __device__ __forceinline__ uint32_t fetchWork(unsigned int* work, uint32_t idle,
 // lanes, 5.8 ms a frame; with refilling but without the rounds 6.8 ms).  In
 // rounds 15 to 19 lanes are active, and L1's requests (a node in four, 32 bytes
 // each: seven of 16 bytes took 4.35 ms) and their latency bound the kernel.
-__global__ void __launch_bounds__(kWalkThreads, 4) kWalkClosest(RayWalkArgs a) {
-  const uint32_t n = *a.count;
+template <bool kFull>
+__device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, int spread) {
   const int lane = threadIdx.x & 31;
   uint32_t visits = 0, culled = 0, nnodes = 0, ntris = 0;
+  const int lanes = kFull ? 32 : spread;
+  const int refill = kFull ? kRefill : (lanes * kRefill + 31) / 32, turn = kFull ? kSwitch : (lanes * kSwitch + 31) / 32;
+  const uint32_t used = kFull ? 0xffffffffu : (1u << lanes) - 1u;
   bool has = false, exhausted = n == 0;
   uint32_t rid = 0, next = 0, end = 0;
   WalkRay r{};
@@ -375,9 +388,9 @@ __global__ void __launch_bounds__(kWalkThreads, 4) kWalkClosest(RayWalkArgs a) {
   while (true) {
     const uint32_t inner = __ballot_sync(0xffffffffu, cur >= 0);
     const uint32_t leaf = __ballot_sync(0xffffffffu, cur < 0 && cur != kDone);
-    const uint32_t idle = __ballot_sync(0xffffffffu, !has);
-    const int ni = __popc(inner), nl = __popc(leaf), nd = __popc(idle), ne = 32 - ni - nl - nd;
-    if (nd == 32 || (nd >= kRefill && !exhausted)) {
+    const uint32_t idle = __ballot_sync(0xffffffffu, !has) & used;
+    const int ni = __popc(inner), nl = __popc(leaf), nd = __popc(idle), ne = lanes - ni - nl - nd;
+    if (nd == lanes || (nd >= refill && !exhausted)) {
       if (!has && best_key != kNoHit) {
         // the finished ray's hit: TriMeshBuffer::updateIntersection
         // (src/render/trimesh_buffer.cc:328-360)
@@ -398,7 +411,7 @@ __global__ void __launch_bounds__(kWalkThreads, 4) kWalkClosest(RayWalkArgs a) {
       if (exhausted) break;  // every lane is idle
       __syncwarp();
       const uint32_t i = fetchWork(a.work, idle, n, &exhausted);
-      if (!has && i < n) {
+      if ((kFull || lane < lanes) && !has && i < n) {
         const uint2 ref = a.list_ref[i];
         if (ref.y > 0) {
           rid = a.list[i];
@@ -413,7 +426,7 @@ __global__ void __launch_bounds__(kWalkThreads, 4) kWalkClosest(RayWalkArgs a) {
           has = true;
         }
       }
-    } else if (ne >= kSwitch || (ni == 0 && nl == 0)) {
+    } else if (ne >= turn || (ni == 0 && nl == 0)) {
       if (has && cur == kDone) {
         // the next domain of the list; the rest start beyond the hit once one does
         has = next < end;
@@ -492,10 +505,13 @@ __global__ void __launch_bounds__(kWalkThreads, 4) kWalkClosest(RayWalkArgs a) {
 }
 
 // Occlusion, in the same rounds.
-__global__ void __launch_bounds__(kWalkThreads, 4) kWalkOccluded(RayWalkArgs a) {
-  const uint32_t n = *a.count;
+template <bool kFull>
+__device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, int spread) {
   const int lane = threadIdx.x & 31;
   uint32_t visits = 0, nnodes = 0, ntris = 0;
+  const int lanes = kFull ? 32 : spread;
+  const int refill = kFull ? kRefill : (lanes * kRefill + 31) / 32, turn = kFull ? kSwitch : (lanes * kSwitch + 31) / 32;
+  const uint32_t used = kFull ? 0xffffffffu : (1u << lanes) - 1u;
   bool has = false, exhausted = n == 0;
   uint32_t rid = 0, next = 0, end = 0;
   WalkRay r{};
@@ -506,12 +522,12 @@ __global__ void __launch_bounds__(kWalkThreads, 4) kWalkOccluded(RayWalkArgs a) 
   while (true) {
     const uint32_t inner = __ballot_sync(0xffffffffu, cur >= 0);
     const uint32_t leaf = __ballot_sync(0xffffffffu, cur < 0 && cur != kDone);
-    const uint32_t idle = __ballot_sync(0xffffffffu, !has);
-    const int ni = __popc(inner), nl = __popc(leaf), nd = __popc(idle), ne = 32 - ni - nl - nd;
-    if (nd == 32 && exhausted) break;
-    if (nd >= kRefill && !exhausted) {
+    const uint32_t idle = __ballot_sync(0xffffffffu, !has) & used;
+    const int ni = __popc(inner), nl = __popc(leaf), nd = __popc(idle), ne = lanes - ni - nl - nd;
+    if (nd == lanes && exhausted) break;
+    if (nd >= refill && !exhausted) {
       const uint32_t i = fetchWork(a.work, idle, n, &exhausted);
-      if (!has && i < n) {
+      if ((kFull || lane < lanes) && !has && i < n) {
         const uint2 ref = a.list_ref[i];
         if (ref.y > 0) {
           rid = a.list[i];
@@ -527,7 +543,7 @@ __global__ void __launch_bounds__(kWalkThreads, 4) kWalkOccluded(RayWalkArgs a) 
           cur = a.scene.domains[a.arena[next++].x].node_base;
         }
       }
-    } else if (ne >= kSwitch || (ni == 0 && nl == 0)) {
+    } else if (ne >= turn || (ni == 0 && nl == 0)) {
       if (has && cur == kDone) {
         has = next < end;
         if (has) {
@@ -590,6 +606,20 @@ __global__ void __launch_bounds__(kWalkThreads, 4) kWalkOccluded(RayWalkArgs a) 
   addCounts(&a.ctr->tris_shadow, ntris, lane);
 }
 
+__global__ void __launch_bounds__(kWalkThreads, 4) kWalkClosest(RayWalkArgs a) {
+  const uint32_t n = *a.count;
+  const int lanes = walkLanes(n);
+  if (lanes == 32) walkClosest<true>(a, n, 32);
+  else walkClosest<false>(a, n, lanes);
+}
+
+__global__ void __launch_bounds__(kWalkThreads, 4) kWalkOccluded(RayWalkArgs a) {
+  const uint32_t n = *a.count;
+  const int lanes = walkLanes(n);
+  if (lanes == 32) walkOccluded<true>(a, n, 32);
+  else walkOccluded<false>(a, n, lanes);
+}
+
 // One thread per node.  The half extent is rounded up, then widened by 2^-21.
 __global__ void kWalkNodes(const BvhNode4* __restrict__ nodes, uint32_t num_nodes, const DomainDev* __restrict__ domains,
                            int D, WalkNode* out) {
@@ -637,17 +667,17 @@ void launchWalkNodes(cudaStream_t s, const BvhNode4* nodes, uint32_t num_nodes, 
 }
 
 template <int kKind>
-static void launchLists(cudaStream_t s, const RayWalkArgs& a, int num_sms) {
-  // the largest table (1024 domains) takes 39 KB; primary rays read their bin's domains instead
+static void launchLists(cudaStream_t s, const RayWalkArgs& a, int nblocks) {
+  // primary rays read their bin's domains instead
   static_assert((kGroupMax / 64 + kGroupMax / 4) * kNodeStride * 16 <= 48 * 1024, "group table in shared memory");
   const size_t bytes = kKind == kListPrimary ? 0 : (size_t)(a.groups.l1 + a.groups.l2) * kNodeStride * sizeof(float4);
-  kListDomains<kKind><<<num_sms * 8, kWalkThreads, bytes, s>>>(a);
+  kListDomains<kKind><<<nblocks, kWalkThreads, bytes, s>>>(a);
 }
 
-void launchListDomains(cudaStream_t s, const RayWalkArgs& a, int num_sms) {
-  if (a.shadow) launchLists<kListShadow>(s, a, num_sms);
-  else if (a.bin_start) launchLists<kListPrimary>(s, a, num_sms);
-  else launchLists<kListBounce>(s, a, num_sms);
+void launchListDomains(cudaStream_t s, const RayWalkArgs& a, int nblocks) {
+  if (a.shadow) launchLists<kListShadow>(s, a, nblocks);
+  else if (a.bin_start) launchLists<kListPrimary>(s, a, nblocks);
+  else launchLists<kListBounce>(s, a, nblocks);
 }
 
 void launchWalkClosest(cudaStream_t s, const RayWalkArgs& a, int nblocks) {

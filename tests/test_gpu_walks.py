@@ -3,8 +3,7 @@
 Frames without captures walk whole rays; bucket_launches = 4 keeps the
 per-domain queues.  Both must give the same image bit for bit and list the same
 (ray, domain) pairs, for domain counts around the sizes where the list pass
-changes (no groups below 16 domains, groups of 4, 16 and 64, the hierarchy above
-1024), with boxes that touch, overlap, are flat or inverted, and with rays
+changes (no groups below 16 domains, groups of 4, 16 and 64, the hierarchy above), with boxes that touch, overlap, are flat or inverted, and with rays
 parallel to their planes.
 """
 import numpy as np
