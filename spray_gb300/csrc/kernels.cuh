@@ -182,6 +182,7 @@ struct ViewDev {
   float ao_max_distance;
   int64_t pixel_base;   // first pixel of the view in the frame's image buffer
   double scale;         // retire weight scale, 1 / spp
+  float scale_hi, scale_lo;  // the same as a pair of floats
   int32_t bin_base;     // the view's first screen bin in the frame's bin table
   int32_t bins_x;       // screen bins per image row
 };

@@ -178,6 +178,7 @@ __device__ __forceinline__ void retirePixel(float4* image, const ViewDev* __rest
   const uint32_t send = s - (uint32_t)(rays.samid[s] % vw.spp) + (uint32_t)vw.spp;
   float4* px = image + vw.pixel_base + rays.pixid[s];
   const double scale = vw.scale;
+  const float hi = vw.scale_hi, lo = vw.scale_lo;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   bool touched = false;
   for (uint32_t q = j; q < n; ++q) {
@@ -187,9 +188,9 @@ __device__ __forceinline__ void retirePixel(float4* image, const ViewDev* __rest
       if (!flag[sid] || sh.occluded[sid]) continue;
       const float4 w = sh.wgt[sid];
       if (!touched) acc = *px;
-      acc.x = (float)((double)acc.x + scale * (double)w.x);
-      acc.y = (float)((double)acc.y + scale * (double)w.y);
-      acc.z = (float)((double)acc.z + scale * (double)w.z);
+      acc.x = addScaled(acc.x, w.x, scale, hi, lo);
+      acc.y = addScaled(acc.y, w.y, scale, hi, lo);
+      acc.z = addScaled(acc.z, w.z, scale, hi, lo);
       touched = true;
     }
   }

@@ -130,6 +130,45 @@ SPRAY_HD float powShininess(float x, float e) {
   return powf(x, e);
 }
 
+// ---------------------------------------------------------------- float-float
+// GB300 runs FP64 at 1/64 of its FP32 rate, so the two places where the
+// reference multiplies in double precision and rounds to float compute the
+// product (and sum) as a pair of floats t + lo with an error below 2^-47 of t.
+// The double expression differs from the exact value by less than 2^-52 of t:
+// when t + lo moved by 2^-45 of t either way rounds to the same float, that is
+// what the double expression rounds to as well; otherwise (a value that close
+// to a rounding boundary, or near the ends of the exponent range) *ok is false
+// and the caller evaluates the double expression.
+SPRAY_HD float roundPair(float t, float lo, bool* ok) {
+  const float eps = fabsf(t) * 2.8421709430404007e-14f;  // 2^-45
+  const float a = t + (lo + eps), b = t + (lo - eps);
+  *ok = a == b && fabsf(t) > 1e-30f && fabsf(t) < 1e37f;
+  return a;
+}
+
+// (float)((double)acc + scale * (double)w), scale = hi + lo to 2^-48 of it.
+SPRAY_HD float addScaled(float acc, float w, double scale, float hi, float lo) {
+  const float p = w * hi;
+  const float e = fmaf(w, hi, -p);  // exact: w * hi = p + e
+  const float t = acc + p;
+  const float q = t - acc;
+  const float z = (acc - (t - q)) + (p - q);  // exact: acc + p = t + z
+  const float r = e + w * lo;
+  if (r == 0.0f && (fabsf(p) > 1e-30f || w == 0.0f)) return t;  // an exact product: one rounding
+  bool ok;
+  const float v = roundPair(t, z + r, &ok);
+  return ok ? v : (float)((double)acc + scale * (double)w);
+}
+
+// (float)((double)x * (pi / 4))
+SPRAY_HD float timesQuarterPi(float x) {
+  const float hi = (float)(kPi / 4.0), lo = (float)(kPi / 4.0 - (double)hi);
+  const float p = x * hi;
+  bool ok;
+  const float v = roundPair(p, fmaf(x, lo, fmaf(x, hi, -p)), &ok);
+  return ok ? v : (float)((double)x * (kPi / 4.0));
+}
+
 // ---------------------------------------------------------------- sampling
 // Concentric disk mapping and cosine-weighted hemisphere sample about N
 // (src/render/sampler.h:49-120, sampler.cc:54-60).  theta is scaled by pi/4 in
@@ -162,7 +201,7 @@ SPRAY_HD void concentricDisk(float u1, float u2, float* dx, float* dy) {
       theta = 6.0f + sx / r;
     }
   }
-  theta = (float)((double)theta * (kPi / 4.0));
+  theta = timesQuarterPi(theta);
   float s, c;
   sincosPoly(theta, &s, &c);
   *dx = r * c;

@@ -977,6 +977,8 @@ void Tracer::planWaves() {
     d.ao_max_distance = f.ao_max_distance;
     d.pixel_base = frame_pixels;
     d.scale = 1.0 / (double)f.spp;
+    d.scale_hi = (float)d.scale;
+    d.scale_lo = (float)(d.scale - (double)d.scale_hi);
     frame_pixels += (int64_t)f.w * f.h;
     mix((uint64_t)f.ao_mode | ((uint64_t)f.bounces << 8) | ((uint64_t)f.ao_samples << 16));
   }
