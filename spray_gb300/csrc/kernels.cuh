@@ -16,6 +16,7 @@
 // Counts live in device memory so a bounce needs no host round trip.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -311,16 +312,23 @@ struct TraceArgs {
 };
 
 // A node as the whole-ray walks read it (made from BvhNode4 by
-// launchWalkNodes): the child boxes as centre c and half extent e per axis, so
-// that a 256-bit load brings both and the ray's direction signs select
-// nothing; children numbered scene-wide (inner nodes by node, leaves by
-// leaf-ordered triangle), so that a walk carries no per-domain base.
-struct alignas(128) WalkNode {
-  float cx[4], ex[4], cy[4], ey[4], cz[4], ez[4];
+// launchWalkNodes): 64 bytes, two 256-bit loads.  Child boxes are a centre c and
+// a half extent e per axis (so that the ray's direction signs select nothing),
+// halves relative to the domain's own centre and half size (WalkDomain), e
+// rounded up until c -+ e holds the box; children are numbered scene-wide (inner
+// nodes by node, leaves by leaf-ordered triangle).
+struct alignas(64) WalkNode {
+  __half cx[4], ex[4], cy[4], ey[4], cz[4], ez[4];
   int32_t child[4];
-  int32_t pad[4];
 };
-static_assert(sizeof(WalkNode) == 128, "walk node must be one 128-byte line");
+static_assert(sizeof(WalkNode) == 64, "walk node must be half a cache line");
+// A domain as the walks enter it, one 256-bit load.
+struct alignas(32) WalkDomain {
+  float centre[3], half[3];  // of the domain's triangles
+  int32_t root;              // its first node
+  uint32_t gprim_base;
+};
+static_assert(sizeof(WalkDomain) == 32, "walk domain must be one load");
 // Triangles a walk can number: leaf references keep 28 bits of the first one.
 constexpr uint64_t kMaxWalkTris = (uint64_t)1 << 28;
 
@@ -347,7 +355,7 @@ struct RayWalkArgs {
   unsigned long long arena_cap;
   uint2* list_ref;            // (first entry, entries)
   const WalkNode* nodes;
-  uint32_t num_nodes, num_tris;
+  const WalkDomain* domains;
   unsigned int* work;         // work counter of the walk (zeroed before launch)
   uint64_t* ray_key;          // per sample: closest hit
   float4* hit_ns;             // per sample: its Ns xyz, colour bits in w
@@ -420,8 +428,10 @@ void launchTraceClosest(cudaStream_t s, const TraceArgs& a, int nblocks);
 // the records after out-of-core and domain-parallel launches.
 void launchResolve(cudaStream_t s, const TraceArgs& a, float4* hit_ns, int nblocks, bool interpolate);
 void launchTraceOccluded(cudaStream_t s, const TraceArgs& a, int nblocks);
+// Sets *bad when a node references a child outside its domain's nodes (or before
+// itself) or triangles.
 void launchWalkNodes(cudaStream_t s, const BvhNode4* nodes, uint32_t num_nodes, const DomainDev* domains, int D,
-                     WalkNode* out);
+                     WalkDomain* wdomains, WalkNode* out, int* bad);
 void launchListDomains(cudaStream_t s, const RayWalkArgs& a, int nblocks);
 void launchWalkClosest(cudaStream_t s, const RayWalkArgs& a, int nblocks);
 void launchWalkOccluded(cudaStream_t s, const RayWalkArgs& a, int nblocks);

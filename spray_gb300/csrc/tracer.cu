@@ -369,6 +369,7 @@ void Tracer::freeScene() {
   devFree(d_domains);
   devFree(d_nodes);
   devFree(d_wnodes);
+  devFree(d_wdomains);
   devFree(d_tris);
   devFree(d_faces);
   devFree(d_colors);
@@ -596,7 +597,7 @@ void Tracer::installScene(std::vector<DomainPack>& packs, const spray_gpu_light*
   }
   if (max_bvh_depth * 3 + 4 > 64) throw std::runtime_error("BVH deeper than the traversal stack");
   total_tris = nt;
-  total_nodes = nn;
+  bad_hierarchy = false;
   scene_bytes = nn * sizeof(BvhNode4) + 3 * nt * sizeof(float4) + 3 * nt * 4 + nvv * 4 + 3 * nvv * 4;
   // out-of-core when the cache holds fewer domains than the scene has
   size_t max_nodes = 0, max_tris = 0, max_verts = 0;
@@ -674,8 +675,14 @@ void Tracer::installScene(std::vector<DomainPack>& packs, const spray_gpu_light*
   }
   if (walksRays()) {
     devAlloc(&d_wnodes, nn);
-    launchWalkNodes(stream, d_nodes, (uint32_t)nn, d_domains, nd, d_wnodes);
-    CK(cudaGetLastError());
+    devAlloc(&d_wdomains, nd);
+    int* bad = reinterpret_cast<int*>(d_ctr);  // a word that every frame clears
+    CK(cudaMemsetAsync(bad, 0, sizeof(int), stream));
+    launchWalkNodes(stream, d_nodes, (uint32_t)nn, d_domains, nd, d_wdomains, d_wnodes, bad);
+    int b = 0;
+    CK(cudaMemcpyAsync(&b, bad, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    bad_hierarchy = b != 0;
   }
   devAlloc(&d_lights, lf.size());
   CK(cudaMemcpy(d_lights, lf.data(), lf.size() * 4, cudaMemcpyHostToDevice));
@@ -1186,8 +1193,7 @@ RayWalkArgs Tracer::walkArgs(bool shadow, bool primary, int S) {
   a.arena_cap = cap_entries;
   a.list_ref = d_list_ref;
   a.nodes = d_wnodes;
-  a.num_nodes = (uint32_t)total_nodes;
-  a.num_tris = (uint32_t)total_tris;
+  a.domains = d_wdomains;
   a.work = d_walk_work + walk_launch++;
   a.ray_key = d_ray_key;
   a.hit_ns = d_hit_ns;
@@ -2231,7 +2237,7 @@ void Tracer::traceFrame(float* out, bool out_is_device, spray_gpu_stats* st) {
       continue;  // retrace with larger queues
     }
     if (ctr.list_overflows) throw OverflowError("a ray overlapped more than 32 domains");
-    if (ctr.error_flags & (kErrBadNode | kErrTraversalBound))
+    if ((ctr.error_flags & (kErrBadNode | kErrTraversalBound)) || (bad_hierarchy && walksRays()))
       throw std::runtime_error("BVH traversal left its bounds (corrupt hierarchy)");
     learn_ms = 0.0;
     if (learned() && !proposal_trained) {

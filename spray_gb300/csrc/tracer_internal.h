@@ -259,7 +259,8 @@ class Tracer {
   std::vector<spray_gpu_light> lights;
   DomainDev* d_domains = nullptr;
   BvhNode4* d_nodes = nullptr;
-  size_t total_nodes = 0;
+  bool bad_hierarchy = false;    // a node's child lies outside its domain
+  WalkDomain* d_wdomains = nullptr;
   WalkNode* d_wnodes = nullptr;  // d_nodes as the whole-ray walks read them
   float4* d_tris = nullptr;
   uint32_t* d_faces = nullptr;

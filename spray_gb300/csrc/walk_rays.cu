@@ -15,7 +15,7 @@
 // the resolve pass fall away, and a ray sets up its walk once instead of once
 // per domain.  Path tracing 64 domains at 1920x1080, 16 spp, 5 bounces: lists
 // 1.72 -> 0.87 ms a frame (with the partition), closest hits with their colours
-// and normals 4.48 + 0.39 -> 4.00 ms, occlusion 1.71 -> 1.47 ms.
+// and normals 4.48 + 0.39 -> 3.68 ms, occlusion 1.71 -> 1.37 ms.
 #include "domain_walk.cuh"
 #include "kernels.cuh"
 #include "spray_math.cuh"
@@ -25,6 +25,9 @@
 #define SPRAY_WALK_REFILL 20
 #endif
 
+#ifndef SPRAY_WALK_STAY
+#define SPRAY_WALK_STAY 12
+#endif
 #ifndef SPRAY_WALK_SWITCH
 #define SPRAY_WALK_SWITCH 8
 #endif
@@ -39,6 +42,9 @@ constexpr int kWalkThreads = 256;
 constexpr int kRefill = SPRAY_WALK_REFILL;
 // Lanes at the end of a domain that the warp gathers before it moves them on.
 constexpr int kSwitch = SPRAY_WALK_SWITCH;
+// Lanes at inner nodes with which a warp takes another node without weighing
+// the other steps.
+constexpr int kStay = SPRAY_WALK_STAY;
 // A node of the group table in shared memory takes 9 float4 instead of 8: the
 // four boxes of a node are read by all lanes at once, but near and far planes
 // differ by lane, and the exact tests read different nodes.
@@ -241,35 +247,55 @@ __global__ void __launch_bounds__(kWalkThreads) kListDomains(RayWalkArgs a) {
 
 namespace {
 
-// A ray against walk nodes.  Per axis a box spans tc -+ h with tc =
-// fma(c, inv, -org * inv) and h = fma(e, |inv|, pad): pad takes the rounding of
-// org * inv (BoxRay), and e was rounded up by more than the roundings of c, tc
-// and h that are relative to the box; what is left is relative to the plane's
-// own distance, kBoxSlack's part.
+// A ray in the domain it walks.  Per axis a box spans tc -+ h with tc =
+// fma(c, inv, o) and h = fma(e, |inv|, pad), where inv = half * (1 / dir) and o =
+// (centre - org) * (1 / dir) take the node's relative coordinates to distances.
+// The roundings of inv and o move a plane by at most 2^-22 of |inv| + |o|, which
+// pad exceeds (and by 1e12 for an axis the ray is parallel to, see BoxRay); what
+// is relative to the plane's own distance is kBoxSlack's part.
 struct WalkRay {
   V3 org;
-  V3 inv, c, pad;
+  V3 rinv;            // 1 / dir, held within [1e-30, 1e18]
+  V3 inv, o, pad;     // in the current domain
   RayShear sh;
 };
 
+__device__ __forceinline__ float walkInverse(float d) {
+  const float inv = 1.0f / d;
+  return copysignf(fminf(fmaxf(fabsf(inv), 1e-30f), 1e18f), inv);
+}
+
 __device__ __forceinline__ WalkRay makeWalkRay(V3 org, V3 dir) {
-  const BoxRay b = makeBoxRay(org, v3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z));
   WalkRay r;
   r.org = org;
-  r.inv = b.inv;
-  r.c = v3(-(org.x * b.inv.x), -(org.y * b.inv.y), -(org.z * b.inv.z));
-  r.pad = v3(boxPad(org.x * b.inv.x, 1.0f / dir.x), boxPad(org.y * b.inv.y, 1.0f / dir.y),
-             boxPad(org.z * b.inv.z, 1.0f / dir.z));
+  r.rinv = v3(walkInverse(dir.x), walkInverse(dir.y), walkInverse(dir.z));
+  r.inv = r.o = r.pad = v3(0.f, 0.f, 0.f);
   r.sh = makeShear(dir);
   return r;
 }
 
 // 32 bytes through the read-only cache in one request: a warp's lanes are at
 // different nodes, so the requests of a walk, not its bytes, load L1.
-__device__ __forceinline__ void load256(const float* p, float* v) {
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+__device__ __forceinline__ void load256(const void* p, uint32_t* v) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
       : "l"(p));
+}
+
+// Takes the ray to domain d; returns its root node.
+__device__ __forceinline__ int enterDomain(const RayWalkArgs& a, int d, WalkRay& r) {
+  uint32_t w[8];
+  load256(a.domains + d, w);
+  auto axis = [&](int k, float org, float rinv, float& inv, float& o, float& pad) {
+    const float c = __uint_as_float(w[k]), h = __uint_as_float(w[3 + k]);
+    inv = copysignf(fmaxf(fabsf(h * rinv), 1e-30f), rinv);
+    o = (c - org) * rinv;
+    pad = (fabsf(inv) + fabsf(o)) * 4.76837158203125e-7f + (fabsf(rinv) == 1e18f ? 1e12f : 0.0f);
+  };
+  axis(0, r.org.x, r.rinv.x, r.inv.x, r.o.x, r.pad.x);
+  axis(1, r.org.y, r.rinv.y, r.inv.y, r.o.y, r.pad.y);
+  axis(2, r.org.z, r.rinv.z, r.inv.z, r.o.z, r.pad.z);
+  return (int)w[6];
 }
 
 __device__ __forceinline__ unsigned long long f2add(unsigned long long a, unsigned long long b) {
@@ -288,29 +314,46 @@ __device__ __forceinline__ unsigned long long f2fmaPacked(unsigned long long a, 
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
+// two halves of a word as packed floats
+__device__ __forceinline__ unsigned long long f2half(uint32_t w) {
+  float lo, hi;
+  asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %2;\n cvt.f32.f16 %0, l;\n cvt.f32.f16 %1, h;\n}\n"
+      : "=f"(lo), "=f"(hi)
+      : "r"(w));
+  return f2pack(lo, hi);
+}
 
 // The four children of a walk node: entry distances, hits and references.
+// kPacked: multiply-adds two children at a time, fewer instructions but pairs of
+// registers for every constant of the ray.  It suits the occlusion walk (1.40
+// and 1.42 ms a frame, packed and scalar); the closest-hit walk spills with it
+// (4.01 and 3.73 ms).
+template <bool kPacked>
 __device__ __forceinline__ int4 testNode(const WalkNode* __restrict__ nodes, int node, const WalkRay& r, float tfar,
                                          float tn[4], bool hit[4]) {
-  const WalkNode* p = nodes + node;
-  float x[8], y[8], z[8];
-  load256(p->cx, x);
-  load256(p->cy, y);
-  load256(p->cz, z);
-  const int4 ch = __ldg(reinterpret_cast<const int4*>(p->child));
-  auto span = [](const float* v, int h, float inv, float c, float pad, float2* near, float2* far) {
-    const unsigned long long tc = f2fmaPacked(f2pack(v[2 * h], v[2 * h + 1]), f2pack(inv, inv), f2pack(c, c));
-    const unsigned long long hw =
-        f2fmaPacked(f2pack(v[4 + 2 * h], v[5 + 2 * h]), f2pack(fabsf(inv), fabsf(inv)), f2pack(pad, pad));
-    *near = f2unpack(f2sub(tc, hw));
-    *far = f2unpack(f2add(tc, hw));
+  uint32_t w[16];  // cx cx ex ex cy cy ey ey cz cz ez ez child x 4
+  load256(nodes + node, w);
+  load256(reinterpret_cast<const char*>(nodes + node) + 32, w + 8);
+  auto span = [](uint32_t c, uint32_t e, float inv, float o, float pad, float2* near, float2* far) {
+    if (kPacked) {
+      const unsigned long long tc = f2fmaPacked(f2half(c), f2pack(inv, inv), f2pack(o, o));
+      const unsigned long long hw = f2fmaPacked(f2half(e), f2pack(fabsf(inv), fabsf(inv)), f2pack(pad, pad));
+      *near = f2unpack(f2sub(tc, hw));
+      *far = f2unpack(f2add(tc, hw));
+    } else {
+      const float2 c2 = f2unpack(f2half(c)), e2 = f2unpack(f2half(e));
+      const float ta = fmaf(c2.x, inv, o), tb = fmaf(c2.y, inv, o);
+      const float ha = fmaf(e2.x, fabsf(inv), pad), hb = fmaf(e2.y, fabsf(inv), pad);
+      *near = make_float2(ta - ha, tb - hb);
+      *far = make_float2(ta + ha, tb + hb);
+    }
   };
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     float2 nx, fx, ny, fy, nz, fz;
-    span(x, h, r.inv.x, r.c.x, r.pad.x, &nx, &fx);
-    span(y, h, r.inv.y, r.c.y, r.pad.y, &ny, &fy);
-    span(z, h, r.inv.z, r.c.z, r.pad.z, &nz, &fz);
+    span(w[h], w[2 + h], r.inv.x, r.o.x, r.pad.x, &nx, &fx);
+    span(w[4 + h], w[6 + h], r.inv.y, r.o.y, r.pad.y, &ny, &fy);
+    span(w[8 + h], w[10 + h], r.inv.z, r.o.z, r.pad.z, &nz, &fz);
     const float t00 = fmaxf(max3(nx.x, ny.x, nz.x), kRayEpsilon);
     const float t01 = fmaxf(max3(nx.y, ny.y, nz.y), kRayEpsilon);
     const float t10 = fminf(min3(fx.x, fy.x, fz.x), tfar) * kBoxSlack;
@@ -320,7 +363,7 @@ __device__ __forceinline__ int4 testNode(const WalkNode* __restrict__ nodes, int
     hit[2 * h] = t00 <= t10;
     hit[2 * h + 1] = t01 <= t11;
   }
-  return ch;
+  return make_int4((int)w[12], (int)w[13], (int)w[14], (int)w[15]);
 }
 
 __device__ __forceinline__ void addCounts(unsigned long long* dst, uint32_t v, int lane) {
@@ -360,14 +403,17 @@ __device__ __forceinline__ uint32_t fetchWork(unsigned int* work, uint32_t idle,
 // Rays walk 12 nodes and 4 triangles each, unevenly: lanes that take whole
 // leaves and node runs together leave two thirds of a warp idle (7 to 13 of 32
 // lanes, 5.8 ms a frame; with refilling but without the rounds 6.8 ms).  In
-// rounds 15 to 19 lanes are active, and L1's requests (a node in four, 32 bytes
-// each: seven of 16 bytes took 4.35 ms) and their latency bound the kernel.
+// rounds 15 to 19 lanes are active; then L1's requests bound the walks (75 % of
+// its data pipe with 128-byte nodes in four requests, 4.02 ms; in seven, 4.35),
+// so nodes take 64 bytes in two, which leaves instruction issue (70 %) and
+// latency: 3.68 ms.
 template <bool kFull>
 __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, int spread) {
   const int lane = threadIdx.x & 31;
   uint32_t visits = 0, culled = 0, nnodes = 0, ntris = 0;
   const int lanes = kFull ? 32 : spread;
   const int refill = kFull ? kRefill : (lanes * kRefill + 31) / 32, turn = kFull ? kSwitch : (lanes * kSwitch + 31) / 32;
+  const int stay = kFull ? kStay : (lanes * kStay + 31) / 32;
   const uint32_t used = kFull ? 0xffffffffu : (1u << lanes) - 1u;
   bool has = false, exhausted = n == 0;
   uint32_t rid = 0, next = 0, end = 0;
@@ -439,53 +485,52 @@ __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, in
             ++next;
             ++visits;
             dom = (int)e.x;
-            cur = a.scene.domains[dom].node_base;
+            cur = enterDomain(a, dom, r);
           }
         }
         if (!has) nnodes += steps;
       }
     } else if (ni >= nl) {
-      if (cur >= 0) {
-        if (++steps > (uint32_t)kMaxSteps || (uint32_t)cur >= a.num_nodes || sp > kStack - 3) {
-          raise(a.ctr, (uint32_t)cur >= a.num_nodes ? kErrBadNode : kErrTraversalBound);
-          cur = kDone;
-          next = end;
-        } else {
-          float tn[4];
-          bool hit[4];
-          const int4 ch = testNode(a.nodes, cur, r, best_t, tn, hit);
-          // nearest child first, the others in slot order (as in traverseClosest)
-          uint32_t k[4];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) k[c] = hit[c] ? (__float_as_uint(tn[c]) & ~3u) | (uint32_t)c : 0xffffffffu;
-          const uint32_t kmin = min(__vimin3_u32(k[0], k[1], k[2]), k[3]);
-          if (kmin != 0xffffffffu) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if (hit[c] && k[c] != kmin) stack[sp++] = make_uint2((uint32_t)childAt(ch, c), k[c] & ~3u);
-            cur = childAt(ch, (int)(kmin & 3u));
+      do {
+        if (cur >= 0) {
+          ++steps;
+          if (sp > kStack - 3) {
+            raise(a.ctr, kErrTraversalBound);
+            cur = kDone;
+            sp = 0;
+            next = end;
           } else {
-            cur = pop();
+            float tn[4];
+            bool hit[4];
+            const int4 ch = testNode<false>(a.nodes, cur, r, best_t, tn, hit);
+            // nearest child first, the others in slot order (as in traverseClosest)
+            uint32_t k[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) k[c] = hit[c] ? (__float_as_uint(tn[c]) & ~3u) | (uint32_t)c : 0xffffffffu;
+            const uint32_t kmin = min(__vimin3_u32(k[0], k[1], k[2]), k[3]);
+            if (kmin != 0xffffffffu) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+                if (hit[c] && k[c] != kmin) stack[sp++] = make_uint2((uint32_t)childAt(ch, c), k[c] & ~3u);
+              cur = childAt(ch, (int)(kmin & 3u));
+            } else {
+              cur = pop();
+            }
           }
         }
-      }
+      } while (__popc(__ballot_sync(0xffffffffu, cur >= 0)) >= stay);
     } else if (cur < 0 && cur != kDone) {
       // the leaf's first triangle; the leaf reference moves on to the rest
       const uint32_t v = ~(uint32_t)cur;
       const uint32_t first = v >> 3;
-      if (first >= a.num_tris) {
-        raise(a.ctr, kErrBadNode);
-        cur = kDone;
-        sp = 0;
-        next = end;
-      } else {
+      {
         ++ntris;
         const float4* tp = a.scene.tris + 3 * (size_t)first;
         const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
         float t, u, vv;
         if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
                               kRayEpsilon, __int_as_float(0x7f800000), &t, &u, &vv)) {
-          const uint64_t key = packHitKey(t, a.scene.domains[dom].gprim_base + __float_as_uint(ta.w));
+          const uint64_t key = packHitKey(t, a.domains[dom].gprim_base + __float_as_uint(ta.w));
           if (key < best_key) {
             best_key = key;
             best_t = t;
@@ -511,6 +556,7 @@ __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, i
   uint32_t visits = 0, nnodes = 0, ntris = 0;
   const int lanes = kFull ? 32 : spread;
   const int refill = kFull ? kRefill : (lanes * kRefill + 31) / 32, turn = kFull ? kSwitch : (lanes * kSwitch + 31) / 32;
+  const int stay = kFull ? kStay : (lanes * kStay + 31) / 32;
   const uint32_t used = kFull ? 0xffffffffu : (1u << lanes) - 1u;
   bool has = false, exhausted = n == 0;
   uint32_t rid = 0, next = 0, end = 0;
@@ -540,7 +586,7 @@ __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, i
           sp = 0;
           has = true;
           ++visits;
-          cur = a.scene.domains[a.arena[next++].x].node_base;
+          cur = enterDomain(a, (int)a.arena[next++].x, r);
         }
       }
     } else if (ne >= turn || (ni == 0 && nl == 0)) {
@@ -548,42 +594,40 @@ __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, i
         has = next < end;
         if (has) {
           ++visits;
-          cur = a.scene.domains[a.arena[next++].x].node_base;
+          cur = enterDomain(a, (int)a.arena[next++].x, r);
         } else {
           nnodes += steps;
           a.sh.occluded[rid] = 0;
         }
       }
     } else if (ni >= nl) {
-      if (cur >= 0) {
-        if (++steps > (uint32_t)kMaxSteps || (uint32_t)cur >= a.num_nodes || sp > kStack - 3) {
-          raise(a.ctr, (uint32_t)cur >= a.num_nodes ? kErrBadNode : kErrTraversalBound);
-          cur = kDone;
-          sp = 0;
-          next = end;
-        } else {
-          float tn[4];
-          bool hit[4];
-          const int4 ch = testNode(a.nodes, cur, r, tfar, tn, hit);
-          int nx = kDone;
+      do {
+        if (cur >= 0) {
+          ++steps;
+          if (sp > kStack - 3) {
+            raise(a.ctr, kErrTraversalBound);
+            cur = kDone;
+            sp = 0;
+            next = end;
+          } else {
+            float tn[4];
+            bool hit[4];
+            const int4 ch = testNode<true>(a.nodes, cur, r, tfar, tn, hit);
+            int nx = kDone;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (!hit[c]) continue;
-            if (nx != kDone) stack[sp++] = nx;
-            nx = childAt(ch, c);
+            for (int c = 0; c < 4; ++c) {
+              if (!hit[c]) continue;
+              if (nx != kDone) stack[sp++] = nx;
+              nx = childAt(ch, c);
+            }
+            cur = nx != kDone ? nx : (sp > 0 ? stack[--sp] : kDone);
           }
-          cur = nx != kDone ? nx : (sp > 0 ? stack[--sp] : kDone);
         }
-      }
+      } while (__popc(__ballot_sync(0xffffffffu, cur >= 0)) >= stay);
     } else if (cur < 0 && cur != kDone) {
       const uint32_t v = ~(uint32_t)cur;
       const uint32_t first = v >> 3;
-      if (first >= a.num_tris) {
-        raise(a.ctr, kErrBadNode);
-        cur = kDone;
-        sp = 0;
-        next = end;
-      } else {
+      {
         ++ntris;
         const float4* tp = a.scene.tris + 3 * (size_t)first;
         const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
@@ -620,9 +664,35 @@ __global__ void __launch_bounds__(kWalkThreads, 4) kWalkOccluded(RayWalkArgs a) 
   else walkOccluded<false>(a, n, lanes);
 }
 
-// One thread per node.  The half extent is rounded up, then widened by 2^-21.
+// One thread per domain: the box of its root's children.
+__global__ void kWalkDomains(const BvhNode4* __restrict__ nodes, const DomainDev* __restrict__ domains, int D,
+                             WalkDomain* out) {
+  const int d = blockIdx.x * blockDim.x + threadIdx.x;
+  if (d >= D) return;
+  const BvhNode4& r = nodes[domains[d].node_base];
+  const float* planes[6] = {r.lox, r.hix, r.loy, r.hiy, r.loz, r.hiz};
+  WalkDomain w;
+  for (int k = 0; k < 3; ++k) {
+    float lo = INFINITY, hi = -INFINITY;
+    for (int q = 0; q < 4; ++q) {
+      if (r.child[q] == kEmptyChild) continue;
+      lo = fminf(lo, planes[2 * k][q]);
+      hi = fmaxf(hi, planes[2 * k + 1][q]);
+    }
+    const float c = 0.5f * lo + 0.5f * hi, h = 0.5f * hi - 0.5f * lo;
+    const bool ok = isfinite(c) && isfinite(h) && h > 0.0f;
+    w.centre[k] = isfinite(c) ? c : 0.0f;
+    w.half[k] = ok ? h : 1.0f;
+  }
+  w.root = domains[d].node_base;
+  w.gprim_base = domains[d].gprim_base;
+  out[d] = w;
+}
+
+// One thread per node: the boxes relative to the domain, in double so that the
+// only rounding that counts is that to half.
 __global__ void kWalkNodes(const BvhNode4* __restrict__ nodes, uint32_t num_nodes, const DomainDev* __restrict__ domains,
-                           int D, WalkNode* out) {
+                           int D, const WalkDomain* __restrict__ wdomains, WalkNode* out, int* bad) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= num_nodes) return;
   int lo = 0, hi = D - 1;  // the last domain whose first node is <= k
@@ -631,39 +701,50 @@ __global__ void kWalkNodes(const BvhNode4* __restrict__ nodes, uint32_t num_node
     if ((uint32_t)domains[mid].node_base <= k) lo = mid;
     else hi = mid - 1;
   }
-  const int node_base = domains[lo].node_base;
+  const WalkDomain wd = wdomains[lo];
   const uint32_t tri_base = (uint32_t)domains[lo].tri_base;
   const BvhNode4 nd = nodes[k];
   WalkNode w;
-  auto axis = [&](const float* l, const float* h, float* c, float* e) {
+  auto axis = [&](int x, const float* l, const float* h, __half* c, __half* e) {
+    const double centre = wd.centre[x], half = wd.half[x];
     for (int q = 0; q < 4; ++q) {
-      c[q] = 0.0f;
-      e[q] = -INFINITY;
+      c[q] = __ushort_as_half(0);
+      e[q] = __ushort_as_half(0xfc00);  // -inf: an unused slot is never entered
       if (nd.child[q] == kEmptyChild) continue;
-      c[q] = 0.5f * l[q] + 0.5f * h[q];
-      e[q] = __fmul_ru(fmaxf(__fsub_ru(h[q], c[q]), __fsub_ru(c[q], l[q])), 1.0000005f);
-      if (!isfinite(c[q]) || !isfinite(e[q])) {  // infinite or NaN planes: everything along this axis
-        c[q] = 0.0f;
-        e[q] = INFINITY;
-      }
+      const double a = ((double)l[q] - centre) / half, b = ((double)h[q] - centre) / half;
+      const __half m = __double2half(0.5 * a + 0.5 * b);
+      const double need = fmax(b - (double)__half2float(m), (double)__half2float(m) - a) * (1.0 + 1e-6);
+      // infinite or NaN planes: everything along this axis (+inf)
+      const bool ok = need >= 0.0 && need < 60000.0;
+      c[q] = ok ? m : __ushort_as_half(0);
+      e[q] = ok ? __float2half_ru(__double2float_ru(need)) : __ushort_as_half(0x7c00);
     }
   };
-  axis(nd.lox, nd.hix, w.cx, w.ex);
-  axis(nd.loy, nd.hiy, w.cy, w.ey);
-  axis(nd.loz, nd.hiz, w.cz, w.ez);
+  axis(0, nd.lox, nd.hix, w.cx, w.ex);
+  axis(1, nd.loy, nd.hiy, w.cy, w.ey);
+  axis(2, nd.loz, nd.hiz, w.cz, w.ez);
   for (int q = 0; q < 4; ++q) {
     const int c = nd.child[q];
-    if (c == kEmptyChild) w.child[q] = kEmptyChild;
-    else if (c >= 0) w.child[q] = c + node_base;
-    else w.child[q] = (int)~(~(uint32_t)c + (tri_base << 3));
-    w.pad[q] = 0;
+    const uint32_t leaf = ~(uint32_t)c;
+    // children follow their parent in the domain's nodes, leaves lie in its
+    // triangles: the walks rely on it and check nothing
+    const bool ok = c == kEmptyChild || (c >= 0 ? (uint32_t)c > k - (uint32_t)wd.root && c < domains[lo].num_nodes
+                                                : (leaf >> 3) + (leaf & 7u) < (uint32_t)domains[lo].num_tris);
+    if (!ok) {
+      *bad = 1;
+      w.child[q] = kEmptyChild;
+    } else if (c == kEmptyChild) w.child[q] = kEmptyChild;
+    else if (c >= 0) w.child[q] = c + wd.root;
+    else w.child[q] = (int)~(leaf + (tri_base << 3));
   }
   out[k] = w;
 }
 
 void launchWalkNodes(cudaStream_t s, const BvhNode4* nodes, uint32_t num_nodes, const DomainDev* domains, int D,
-                     WalkNode* out) {
-  if (num_nodes > 0) kWalkNodes<<<(num_nodes + 127) / 128, 128, 0, s>>>(nodes, num_nodes, domains, D, out);
+                     WalkDomain* wdomains, WalkNode* out, int* bad) {
+  if (num_nodes == 0) return;
+  kWalkDomains<<<(D + 127) / 128, 128, 0, s>>>(nodes, domains, D, wdomains);
+  kWalkNodes<<<(num_nodes + 127) / 128, 128, 0, s>>>(nodes, num_nodes, domains, D, wdomains, out, bad);
 }
 
 template <int kKind>
