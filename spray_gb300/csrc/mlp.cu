@@ -10,6 +10,7 @@
 // up sets Net::error, and the CTA frees its tensor memory and returns.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "mlp.cuh"
@@ -19,6 +20,7 @@ namespace spray {
 namespace mlp {
 namespace {
 
+constexpr int kReduceThreads = 256;          // threads per block of kReduceAdam
 constexpr uint64_t kWaitNs = 1000000000ull;  // bound of one mbarrier wait
 
 __device__ __forceinline__ uint32_t smemAddr(const void* p) {
@@ -392,7 +394,11 @@ static_assert(kGSmem <= 227 * 1024, "training shared memory");  // one CTA per S
 constexpr uint32_t kGCols = 512, kColLogit = 64, kColDw = 128;
 
 __global__ void __launch_bounds__(kTile, 1) kGrad(Net net, const Sample* batch, int64_t n, float inv_count,
-                                                  float* partial) {
+                                                  const uint32_t* labelled_rows, float* partial) {
+  if (labelled_rows) {
+    const uint32_t rows = *labelled_rows;
+    inv_count = rows > 0 ? 1.0f / (float)rows : 0.0f;
+  }
   extern __shared__ __align__(128) uint8_t sm[];
   const int t = threadIdx.x, warp = t >> 5;
   float* bias = reinterpret_cast<float*>(sm + kGBias);
@@ -587,13 +593,31 @@ __global__ void __launch_bounds__(kTile, 1) kGrad(Net net, const Sample* batch, 
   if (warp == 0) tmemDealloc(tm, kGCols);
 }
 
+// One thread per parameter: the partials in CTA order (16 loads in flight, the
+// additions one after the other), then Adam.
 __global__ void kReduceAdam(const float* __restrict__ partial, int nparts, float* grad, float* params,
-                            float* m, float* v, float lr, int step) {
+                            float* m, float* v, float lr, int step, float* mean_loss) {
+  __shared__ float tail[2];  // loss sum and labelled rows, the last two sums
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kPartial) return;
   float g = 0.0f;
-  for (int p = 0; p < nparts; ++p) g += partial[(size_t)p * kPartial + i];
-  grad[i] = g;
+  if (i < kPartial) {
+    int p = 0;
+    for (; p + 16 <= nparts; p += 16) {
+      float x[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) x[q] = partial[(size_t)(p + q) * kPartial + i];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) g += x[q];
+    }
+    for (; p < nparts; ++p) g += partial[(size_t)p * kPartial + i];
+    grad[i] = g;
+    if (i >= kParams) tail[i - kParams] = g;
+  }
+  static_assert(kParams / kReduceThreads == (kPartial - 1) / kReduceThreads, "the last block holds both sums");
+  if (mean_loss && blockIdx.x == gridDim.x - 1) {
+    __syncthreads();
+    if (threadIdx.x == 0) *mean_loss = tail[1] > 0.0f ? tail[0] / tail[1] : 0.0f;
+  }
   if (lr > 0.0f && i < kParams) {
     const float mi = 0.9f * m[i] + 0.1f * g;
     const float vi = 0.999f * v[i] + 0.001f * (g * g);
@@ -603,6 +627,20 @@ __global__ void kReduceAdam(const float* __restrict__ partial, int nparts, float
     const float vh = vi / (1.0f - powf(0.999f, (float)step));
     params[i] -= lr * mh / (sqrtf(vh) + 1e-8f);
   }
+}
+
+// Block column = step; its threads stride over the batch.
+__global__ void kCountLabelled(const Sample* __restrict__ samples, int64_t n, int64_t b, int64_t first,
+                               uint32_t* counts) {
+  const int64_t start = ((first + blockIdx.y) * b) % n;
+  const int64_t len = min(b, n - start);
+  uint32_t c = 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x) {
+    const Sample& q = samples[start + i];
+    c += q.label >= 0 && q.label < min(q.ncand, kCand) ? 1u : 0u;
+  }
+  for (int o = 16; o; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(&counts[blockIdx.y], c);
 }
 
 // Per alive ray: the list position of the candidate that holds its hit, when
@@ -709,15 +747,23 @@ void launchEvaluate(cudaStream_t s, const Net& net, const Sample* samples, int64
   kForward<EvalRows><<<nblocks, kTile, kFwdSmem, s>>>(net, r);
 }
 
-void launchGrad(cudaStream_t s, const Net& net, const Sample* batch, int64_t n, float inv_count, float* partial,
-                int nblocks) {
+void launchGrad(cudaStream_t s, const Net& net, const Sample* batch, int64_t n, float inv_count,
+                const uint32_t* labelled, float* partial, int nblocks) {
   cudaFuncSetAttribute(kGrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem);
-  kGrad<<<nblocks, kTile, kGSmem, s>>>(net, batch, n, inv_count, partial);
+  kGrad<<<nblocks, kTile, kGSmem, s>>>(net, batch, n, inv_count, labelled, partial);
+}
+
+void launchCountLabelled(cudaStream_t s, const Sample* samples, int64_t n, int64_t b, int64_t first, int steps,
+                         uint32_t* counts) {
+  cudaMemsetAsync(counts, 0, steps * sizeof(uint32_t), s);
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((b + 1023) / 1024, 256));
+  if (n > 0) kCountLabelled<<<dim3((unsigned)blocks, steps), 256, 0, s>>>(samples, n, b, first, counts);
 }
 
 void launchReduceAdam(cudaStream_t s, const float* partial, int nparts, float* grad, float* params, float* m,
-                      float* v, float lr, int step) {
-  kReduceAdam<<<(kPartial + 255) / 256, 256, 0, s>>>(partial, nparts, grad, params, m, v, lr, step);
+                      float* v, float lr, int step, float* mean_loss) {
+  kReduceAdam<<<(kPartial + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, s>>>(
+      partial, nparts, grad, params, m, v, lr, step, mean_loss);
 }
 
 void launchCollect(cudaStream_t s, const ArenaSource& src, const uint64_t* ray_key, const DomainDev* domains,

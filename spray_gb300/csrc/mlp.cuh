@@ -83,13 +83,19 @@ void launchEvaluate(cudaStream_t s, const Net& net, const Sample* samples, int64
                     int nblocks);
 // Gradient of the mean cross-entropy over the labelled rows of a batch:
 // every CTA writes a partial [kPartial] (gradient, loss sum, labelled rows).
-// `inv_count` scales the loss gradient (1 / labelled rows of the whole batch).
+// The loss gradient is scaled by 1 / *labelled (0 when there are none), or by
+// `inv_count` when `labelled` is null.
 void launchGrad(cudaStream_t s, const Net& net, const Sample* batch, int64_t n, float inv_count,
-                float* partial, int nblocks);
+                const uint32_t* labelled, float* partial, int nblocks);
+// counts[i] = labelled rows of step first + i, i < steps, whose batch is rows
+// [k * b mod n, + b) of the n samples, cut at the last (k the step).
+void launchCountLabelled(cudaStream_t s, const Sample* samples, int64_t n, int64_t b, int64_t first, int steps,
+                         uint32_t* counts);
 // Sums `nparts` partials in order into grad[kParams + 2] and, when lr > 0,
-// applies one Adam step (beta1 0.9, beta2 0.999, eps 1e-8) at step `step`.
+// applies one Adam step (beta1 0.9, beta2 0.999, eps 1e-8) at step `step`;
+// *mean_loss (optional) = loss sum / labelled rows.
 void launchReduceAdam(cudaStream_t s, const float* partial, int nparts, float* grad, float* params,
-                      float* m, float* v, float lr, int step);
+                      float* m, float* v, float lr, int step, float* mean_loss);
 // Training-pair emission after the hits of a depth are resolved: every alive
 // ray with at least two candidates and a hit appends (ray, candidates, label).
 // Pairs are appended in alive order (stable compaction), so the buffer's

@@ -1,8 +1,8 @@
 // C ABI of the learned proposal's kernels on caller-owned device buffers.
 #include <algorithm>
+#include <map>
 #include <stdexcept>
 #include <string>
-#include <vector>
 
 #include "../../include/spray_gpu.h"
 #include "mlp.cuh"
@@ -17,37 +17,71 @@ using spray::fail;
 namespace ml = spray::mlp;
 static_assert(sizeof(spray_mlp_sample) == sizeof(ml::Sample), "sample layout");
 
-struct Scope {
-  cudaStream_t s = nullptr;
-  int* err = nullptr;
+// A calling thread's workspace, kept between its calls (a call used to create a
+// stream and allocate and free its buffers, 140 us around a kernel of 20) and
+// freed when the thread ends: the per-CTA gradient partials (8 MB), a gradient,
+// the labelled rows of up to kCountSteps batches, and a pinned word that a
+// timed-out wait sets.  Work runs on the thread's own default stream, so threads
+// do not wait for one another; a call returns when its work is done, so one
+// workspace per thread and device is enough.
+constexpr int kCountSteps = 1024;
+
+struct Workspace {
+  int device = -1, nsms = 0;
+  int* err = nullptr;      // pinned, mapped
+  int* err_dev = nullptr;  // the same word as the device addresses it
   float* partial = nullptr;
-  int nsms = 0;
-  ~Scope() {
+  float* grad = nullptr;
+  uint32_t* counts = nullptr;
+  void release() {
+    if (err) cudaFreeHost(err);
     if (partial) cudaFree(partial);
-    if (err) cudaFree(err);
-    if (s) cudaStreamDestroy(s);
+    if (grad) cudaFree(grad);
+    if (counts) cudaFree(counts);
+    *this = Workspace{};
   }
 };
 
-int setup(Scope& sc, int32_t device, int nparts) {
+struct Workspaces {
+  std::map<int, Workspace> of;
+  ~Workspaces() {
+    for (auto& w : of)
+      if (cudaSetDevice(w.first) == cudaSuccess) w.second.release();
+  }
+};
+thread_local Workspaces t_workspaces;
+
+// The calling thread's workspace on `device`, with the gradient buffers when
+// training; makes the device current.
+int setup(Workspace** out, int32_t device, bool training) {
   cudaError_t e = cudaSetDevice(device);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sc.nsms, cudaDevAttrMultiProcessorCount, device);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&sc.s, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&sc.err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemsetAsync(sc.err, 0, sizeof(int), sc.s);
-  if (e == cudaSuccess && nparts > 0) e = cudaMalloc(&sc.partial, (size_t)nparts * ml::kPartial * sizeof(float));
   if (e != cudaSuccess) return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
+  Workspace& w = t_workspaces.of[device];
+  if (!w.err) {
+    e = cudaDeviceGetAttribute(&w.nsms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaHostAlloc(&w.err, sizeof(int), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&w.err_dev, w.err, 0);
+    w.device = device;
+  }
+  if (e == cudaSuccess && training && !w.counts) {
+    e = cudaMalloc(&w.partial, (size_t)ml::gradBlocks(w.nsms) * ml::kPartial * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&w.grad, ml::kPartial * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&w.counts, kCountSteps * sizeof(uint32_t));
+  }
+  if (e != cudaSuccess) {
+    w.release();
+    return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
+  }
+  *w.err = 0;
+  *out = &w;
   return SPRAY_GPU_OK;
 }
 
-int finish(Scope& sc) {
-  cudaError_t e = cudaStreamSynchronize(sc.s);
+int finish(const Workspace& w) {
+  cudaError_t e = cudaStreamSynchronize(cudaStreamPerThread);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
-  int err = 0;
-  e = cudaMemcpy(&err, sc.err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
-  if (err) return fail(SPRAY_GPU_ETIMEOUT, "a tensor-core wait gave up");
+  if (*(volatile int*)w.err) return fail(SPRAY_GPU_ETIMEOUT, "a tensor-core wait gave up");
   return SPRAY_GPU_OK;
 }
 
@@ -78,38 +112,37 @@ int spray_mlp_forward_dev(const float* params, const float* boxes, const float n
   if (!params || !boxes || !norm || (n > 0 && (!samples || !logits || !pred)))
     return fail(SPRAY_GPU_EINVAL, "null argument");
   if (n < 0) return fail(SPRAY_GPU_EINVAL, "negative sample count");
-  Scope sc;
-  if (int r = setup(sc, device, 0)) return r;
-  if (n == 0) return SPRAY_GPU_OK;
-  const int64_t tiles = (n + ml::kTile - 1) / ml::kTile;
-  const int grid = (int)std::min<int64_t>(tiles, 4 * sc.nsms);
-  ml::launchPredictSamples(sc.s, net(params, boxes, norm, sc.err), reinterpret_cast<const ml::Sample*>(samples),
-                           n, logits, pred, grid);
-  return finish(sc);
+  try {
+    Workspace* w = nullptr;
+    if (int r = setup(&w, device, false)) return r;
+    if (n == 0) return SPRAY_GPU_OK;
+    const int64_t tiles = (n + ml::kTile - 1) / ml::kTile;
+    const int grid = (int)std::min<int64_t>(tiles, 5 * w->nsms);
+    ml::launchPredictSamples(cudaStreamPerThread, net(params, boxes, norm, w->err_dev),
+                             reinterpret_cast<const ml::Sample*>(samples), n, logits, pred, grid);
+    return finish(*w);
+  } catch (const std::exception& ex) {
+    return fail(SPRAY_GPU_ECUDA, ex.what());
+  }
 }
 
 int spray_mlp_grad_dev(const float* params, const float* boxes, const float norm[4],
                        const spray_mlp_sample* samples, int64_t n, float* grad, int32_t device) {
   if (!params || !boxes || !norm || !grad || (n > 0 && !samples)) return fail(SPRAY_GPU_EINVAL, "null argument");
   if (n < 0) return fail(SPRAY_GPU_EINVAL, "negative sample count");
-  Scope sc;
-  if (int r = setup(sc, device, 0)) return r;
-  const int g = gradGrid(sc.nsms, n);
-  cudaError_t e = cudaMalloc(&sc.partial, (size_t)g * ml::kPartial * sizeof(float));
-  if (e != cudaSuccess) return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
-  // labelled rows, counted on the host copy of the labels
-  std::vector<spray_mlp_sample> h(n);
-  if (n > 0) {
-    e = cudaMemcpy(h.data(), samples, (size_t)n * sizeof(spray_mlp_sample), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
+  try {
+    Workspace* w = nullptr;
+    if (int r = setup(&w, device, true)) return r;
+    const int g = gradGrid(w->nsms, n);
+    const cudaStream_t st = cudaStreamPerThread;
+    const ml::Sample* q = reinterpret_cast<const ml::Sample*>(samples);
+    ml::launchCountLabelled(st, q, n, std::max<int64_t>(n, 1), 0, 1, w->counts);
+    ml::launchGrad(st, net(params, boxes, norm, w->err_dev), q, n, 0.0f, w->counts, w->partial, g);
+    ml::launchReduceAdam(st, w->partial, g, grad, nullptr, nullptr, nullptr, 0.0f, 0, nullptr);
+    return finish(*w);
+  } catch (const std::exception& ex) {
+    return fail(SPRAY_GPU_ECUDA, ex.what());
   }
-  int64_t labelled = 0;
-  for (auto& q : h) labelled += (q.label >= 0 && q.label < std::min(q.ncand, 8)) ? 1 : 0;
-  const float inv = labelled > 0 ? 1.0f / (float)labelled : 0.0f;
-  ml::Net nt = net(params, boxes, norm, sc.err);
-  ml::launchGrad(sc.s, nt, reinterpret_cast<const ml::Sample*>(samples), n, inv, sc.partial, g);
-  ml::launchReduceAdam(sc.s, sc.partial, g, grad, nullptr, nullptr, nullptr, 0.0f, 0);
-  return finish(sc);
 }
 
 int spray_mlp_train_dev(float* params, float* adam_m, float* adam_v, const float* boxes, const float norm[4],
@@ -118,50 +151,28 @@ int spray_mlp_train_dev(float* params, float* adam_m, float* adam_v, const float
   if (!params || !adam_m || !adam_v || !boxes || !norm || !samples) return fail(SPRAY_GPU_EINVAL, "null argument");
   if (n <= 0 || batch <= 0 || steps < 0 || first_step < 1 || !(lr > 0.0f))
     return fail(SPRAY_GPU_EINVAL, "need n > 0, batch > 0, steps >= 0, first_step >= 1, lr > 0");
-  Scope sc;
-  if (int r = setup(sc, device, 0)) return r;
-  const int64_t b = std::min<int64_t>(batch, n);
-  const int g = gradGrid(sc.nsms, b);
-  float* grad = nullptr;
-  cudaError_t e = cudaMalloc(&sc.partial, (size_t)g * ml::kPartial * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&grad, ml::kPartial * sizeof(float));
-  if (e != cudaSuccess) {
-    if (grad) cudaFree(grad);
-    return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
-  }
-  std::vector<spray_mlp_sample> h(n);
-  e = cudaMemcpy(h.data(), samples, (size_t)n * sizeof(spray_mlp_sample), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) {
-    cudaFree(grad);
-    return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
-  }
-  ml::Net nt = net(params, boxes, norm, sc.err);
-  std::vector<float> lossv(steps, 0.0f);
-  int rc = SPRAY_GPU_OK;
-  for (int k = 0; k < steps && rc == SPRAY_GPU_OK; ++k) {
-    const int64_t start = ((int64_t)k * b) % n;
-    const int64_t len = std::min<int64_t>(b, n - start);
-    int64_t labelled = 0;
-    for (int64_t i = start; i < start + len; ++i)
-      labelled += (h[i].label >= 0 && h[i].label < std::min(h[i].ncand, 8)) ? 1 : 0;
-    const float inv = labelled > 0 ? 1.0f / (float)labelled : 0.0f;
-    ml::launchGrad(sc.s, nt, reinterpret_cast<const ml::Sample*>(samples) + start, len, inv, sc.partial, g);
-    ml::launchReduceAdam(sc.s, sc.partial, g, grad, params, adam_m, adam_v, lr, first_step + k);
-    if (losses) {
-      float tail[2];
-      e = cudaMemcpyAsync(tail, grad + ml::kParams, 2 * sizeof(float), cudaMemcpyDeviceToHost, sc.s);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(sc.s);
-      if (e != cudaSuccess) rc = fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
-      else lossv[k] = tail[1] > 0.0f ? tail[0] / tail[1] : 0.0f;
+  try {
+    Workspace* w = nullptr;
+    if (int r = setup(&w, device, true)) return r;
+    const int64_t b = std::min<int64_t>(batch, n);
+    const int g = gradGrid(w->nsms, b);
+    const cudaStream_t st = cudaStreamPerThread;
+    const ml::Sample* q = reinterpret_cast<const ml::Sample*>(samples);
+    ml::Net nt = net(params, boxes, norm, w->err_dev);
+    for (int k = 0; k < steps; ++k) {
+      // the labelled rows of the next batches, on the device
+      if (k % kCountSteps == 0)
+        ml::launchCountLabelled(st, q, n, b, k, std::min(kCountSteps, steps - k), w->counts);
+      const int64_t start = ((int64_t)k * b) % n;
+      const int64_t len = std::min<int64_t>(b, n - start);
+      ml::launchGrad(st, nt, q + start, len, 0.0f, w->counts + k % kCountSteps, w->partial, g);
+      ml::launchReduceAdam(st, w->partial, g, w->grad, params, adam_m, adam_v, lr, first_step + k,
+                           losses ? losses + k : nullptr);
     }
+    return finish(*w);
+  } catch (const std::exception& ex) {
+    return fail(SPRAY_GPU_ECUDA, ex.what());
   }
-  if (rc == SPRAY_GPU_OK) rc = finish(sc);
-  cudaFree(grad);
-  if (rc == SPRAY_GPU_OK && losses && steps > 0) {
-    e = cudaMemcpy(losses, lossv.data(), steps * sizeof(float), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
-  }
-  return rc;
 }
 
 }  // extern "C"

@@ -1935,8 +1935,9 @@ void Tracer::trainProposal() {
     for (int64_t k = 0; k < per_epoch * cfg.learn_epochs; ++k) {
       const int64_t start = (k % per_epoch) * B;
       const int64_t len = std::min<int64_t>(B, n - start);
-      ml::launchGrad(stream, proposalNet(), d_pairs + start, len, 1.0f / (float)len, d_mlp_partial, grid);
-      ml::launchReduceAdam(stream, d_mlp_partial, grid, grad, params, m, v, cfg.learn_lr, ++adam_step);
+      ml::launchGrad(stream, proposalNet(), d_pairs + start, len, 1.0f / (float)len, nullptr, d_mlp_partial, grid);
+      ml::launchReduceAdam(stream, d_mlp_partial, grid, grad, params, m, v, cfg.learn_lr, ++adam_step,
+                           nullptr);
     }
   }
   CK(cudaEventRecord(e1, stream));
