@@ -423,7 +423,7 @@ int spray_gpu_insitu_partition(const float* domain_bounds, int32_t num_domains, 
  * device budget reserved at start-up, a host runtime that hands out GPU
  * memory from its own pool (a cudaMalloc behind its back breaks its
  * accounting; cudaFree synchronises the device).  All scratch lives in one
- * static device array (about 13 MB, kept on each device that used it until
+ * static device array (about 14 MB, kept on each device that used it until
  * exit); this call allocates nothing.
  *   domain_bounds  device, 6 floats per domain (min xyz, max xyz), <= 256 domains
  *   ray_org/dir    device, 4 floats per ray (xyz + unused), 16-byte aligned,

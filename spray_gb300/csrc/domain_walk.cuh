@@ -1,9 +1,13 @@
-// Descent of the 4-wide hierarchy over the domain boxes, shared by the
-// scheduler (sched.cu) and the non-speculative round loop (rounds.cu).
+// The domains a ray may enter: the descent of the 4-wide hierarchy over the
+// domain boxes (the scheduler, sched.cu, the non-speculative round loop,
+// rounds.cu, and scenes of many domains) and the test of their groups of 64, 16
+// and 4 with a ray's sorted list (the whole-ray walks, walk_rays.cu, and the
+// allocation-free scheduler, noalloc.cu).
 #pragma once
 
 #include "kernels.cuh"
 #include "spray_math.cuh"
+#include "traverse.cuh"
 
 namespace spray {
 
@@ -72,4 +76,97 @@ __device__ __forceinline__ void descendDomains(const float4* nodes, int NN, V3 o
   }
 }
 
+namespace {
+
+// A node of the group table in shared memory takes 9 float4 instead of 8: the
+// four boxes of a node are read by all lanes at once, but near and far planes
+// differ by lane, and the exact tests read different nodes.
+constexpr int kNodeStride = 9;
+// Slack of the group test: the exact slab test rounds (plane - org) * inv and
+// this one fma(plane, inv, -org * inv); 2e-6 covers both by far.
+constexpr float kGroupSlack = 1.000002f;
+
+// Floats as integers that order like them (negative t: the ray starts inside
+// the box; -0 was made +0 by the caller).
+__device__ __forceinline__ uint32_t orderedBits(float t) {
+  const uint32_t u = __float_as_uint(t);
+  return u ^ ((u & 0x80000000u) ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ float orderedFloat(uint32_t k) {
+  return __uint_as_float(k ^ ((k & 0x80000000u) ? 0x80000000u : 0xffffffffu));
+}
+
+// Per-lane sorted list of (entry t, domain), 64-bit keys in local memory.
+struct DomainList {
+  uint64_t key[kMaxList];
+  int n = 0;
+  __device__ __forceinline__ void insert(float t, int d, Counters* ctr) {
+    const uint64_t k = ((uint64_t)orderedBits(t + 0.0f) << 32) | (uint32_t)d;
+    if (n == kMaxList) {
+      atomicAdd(&ctr->list_overflows, 1ull);
+      return;  // the frame is refused
+    }
+    int j = n++;
+    while (j > 0 && key[j - 1] > k) {
+      key[j] = key[j - 1];
+      --j;
+    }
+    key[j] = k;
+  }
+};
+
+// The four boxes of a table node against the ray: bit k set when box k may be hit.
+__device__ __forceinline__ uint32_t boxMask(const float4* p, const BoxRay& r, float t1) {
+  float tn[4];
+  bool h[4];
+  testBoxes(p[r.sx], p[r.sx ^ 1], p[2 + r.sy], p[3 - r.sy], p[4 + r.sz], p[5 - r.sz], r, kRayEpsilon, t1, kGroupSlack,
+            tn, h);
+  return (h[0] ? 1u : 0u) | (h[1] ? 2u : 0u) | (h[2] ? 4u : 0u) | (h[3] ? 8u : 0u);
+}
+
+// Calls consider(d) for a superset of the domains whose boxes the ray enters
+// within (1e-3, t1], 64 at a time: every group of 16 is tested, the four nodes
+// of a group some lane may enter are tested by all of the warp's lanes that
+// may, at the same addresses, and then each lane goes through its own bits.
+// Against the descent of a hierarchy (domain_walk.cuh) that is more tests and
+// far fewer instructions, for the lanes of a warp stay together.
+template <class F>
+__device__ __forceinline__ void groupDomains(const float4* table, int n1, int n2, const BoxRay& r, float t1,
+                                             F&& consider) {
+  const float4* l2 = table + n1 * kNodeStride;
+  for (int q = 0; q < n1; ++q) {
+    const uint32_t groups = boxMask(table + q * kNodeStride, r, t1);
+    uint32_t bits[2] = {0u, 0u};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (!(groups & (1u << c))) continue;
+      const int first = 16 * q + 4 * c;
+      uint32_t m = 0;
+#pragma unroll 1
+      for (int j = 0; j < 4 && first + j < n2; ++j)
+        m |= boxMask(l2 + (first + j) * kNodeStride, r, t1) << (4 * j);
+      bits[c >> 1] |= m << (16 * (c & 1));
+    }
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+      for (uint32_t m = bits[w]; m; m &= m - 1) {
+        const int b = 32 * w + __ffs(m) - 1;
+        consider(reinterpret_cast<const int*>(l2 + (16 * q + (b >> 2)) * kNodeStride + 6)[b & 3]);
+      }
+  }
+}
+
+__device__ __forceinline__ uint32_t warpScan(uint32_t v, uint32_t* total) {
+  const int lane = threadIdx.x & 31;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  *total = __shfl_sync(0xffffffffu, x, 31);
+  return x - v;
+}
+
+}  // namespace
 }  // namespace spray

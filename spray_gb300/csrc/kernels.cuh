@@ -215,7 +215,7 @@ struct SchedArgs {
   uint64_t* ray_key;          // radiance: reset to kNoHit per scheduled ray
   const BvhNode4* dnodes;     // 4-wide hierarchy over the domain boxes (null: test every domain)
   int dnode_count;
-  const float* dboxes;        // domain boxes, 6 floats each (null: staged from the domain table)
+  const float* dboxes;        // domain boxes, 6 floats each
   // primary rays: candidate domains per screen bin (null: not primary rays);
   // a ray's bins are those of its view (ViewDev::bin_base, bins_x)
   const uint32_t* bin_start;  // [all views' bins + 1]
@@ -241,6 +241,7 @@ struct SchedArgs {
   // with order_by_depth the entries at or before it form bucket 0 and the
   // later ones buckets 1, 2, 3+ (null: bucket = list position, capped at 3)
   const uint8_t* pred;
+  int key_relative;           // scatter: hist holds positions relative to key_start
   int defer_hist;             // kSchedLists leaves the histogram to the partition step
   int pack_depth;             // entries in the packed format (kPackedIdBits)
   uint8_t* dbg_depth;         // debug capture: list position of every entry (or null)
@@ -420,6 +421,9 @@ void launchSchedLists(cudaStream_t s, const SchedArgs& a, const DomainDev* domai
                       int nwarps, int nblocks);
 void launchSchedPartition(cudaStream_t s, const SchedArgs& a, int ndomains, int nwarps,
                           uint32_t* scan_tmp, size_t scan_words);
+// The scatter alone, for a histogram scanned by the caller: a.hist holds each
+// chunk's first position per key (key_relative: within its key's entries).
+void launchSchedScatter(cudaStream_t s, const SchedArgs& a, int ndomains, int nwarps);
 // Resident blocks per SM of the scheduling kernel for this shared-memory use.
 int schedBlocksPerSm(int D, int nkeys, int dnode_count);
 void launchTraceClosest(cudaStream_t s, const TraceArgs& a, int nblocks);

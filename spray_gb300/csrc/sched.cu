@@ -485,7 +485,8 @@ __global__ void __launch_bounds__(128) kSchedScatter(SchedArgs a, int D, int nke
   const uint64_t r1 = min((uint64_t)n, r0 + csize);
   if (r0 >= r1) break;
   __syncwarp();
-  for (int k = lane; k < nkeys; k += 32) running[k] = a.hist[(size_t)ch * nkeys + k];
+  for (int k = lane; k < nkeys; k += 32)
+    running[k] = a.hist[(size_t)ch * nkeys + k] + (a.key_relative ? a.key_start[k] : 0u);
   __syncwarp();
   // the next group's list sizes, offsets, ray ids and predictions load while
   // this group is flattened and ranked
@@ -645,8 +646,7 @@ static void launchLists(cudaStream_t s, const SchedArgs& a, const DomainDev* dom
 
 void launchSchedLists(cudaStream_t s, const SchedArgs& a, const DomainDev* domains, int D, int nwarps,
                       int nblocks) {
-  // without a box array (the allocation-free entry point) the tables are staged
-  if (!a.dboxes || tablesShared(D, a.dnode_count)) launchLists<true>(s, a, domains, D, nwarps, nblocks);
+  if (tablesShared(D, a.dnode_count)) launchLists<true>(s, a, domains, D, nwarps, nblocks);
   else launchLists<false>(s, a, domains, D, nwarps, nblocks);
 }
 
@@ -676,6 +676,11 @@ void launchSchedPartition(cudaStream_t s, const SchedArgs& a, int D, int nwarps,
   kHistKeyScan<<<(nkeys + 31) / 32, 1024, 0, s>>>(colsum, G, nkeys, keybase, ticket, a.key_start,
                                                    a.num_entries, a.entry_cap, a.ctr);
   kHistApply<<<grid, bt, 0, s>>>(a.hist, a.count, nch, nwarps, nkeys, colsum, keybase);
+  launchSchedScatter(s, a, D, nwarps);
+}
+
+void launchSchedScatter(cudaStream_t s, const SchedArgs& a, int D, int nwarps) {
+  const int nkeys = a.order_by_depth ? kDepthBuckets * D : D;
   const int wpb = 4;
   size_t smem3 = (size_t)wpb * nkeys * 4 + (size_t)wpb * kScatterWindow * 3 * 4;
   cudaFuncSetAttribute(kSchedScatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
