@@ -599,8 +599,9 @@ __global__ void kWalkDomains(const BvhNode4* __restrict__ nodes, const DomainDev
   out[d] = w;
 }
 
-// One thread per node: the boxes relative to the domain, in double so that the
-// only rounding that counts is that to half.
+// One thread per node: the boxes relative to the domain.  The relative planes
+// are within 2^-22 of their true values (a subtraction and a product of values
+// of at most 1), which 1e-6 more extent covers; e is rounded up to half.
 __global__ void kWalkNodes(const BvhNode4* __restrict__ nodes, uint32_t num_nodes, const DomainDev* __restrict__ domains,
                            int D, const WalkDomain* __restrict__ wdomains, WalkNode* out, int* bad) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -616,18 +617,18 @@ __global__ void kWalkNodes(const BvhNode4* __restrict__ nodes, uint32_t num_node
   const BvhNode4 nd = nodes[k];
   WalkNode w;
   auto axis = [&](int x, const float* l, const float* h, __half* c, __half* e) {
-    const double centre = wd.centre[x], half = wd.half[x];
+    const float centre = wd.centre[x], scale = 1.0f / wd.half[x];
     for (int q = 0; q < 4; ++q) {
       c[q] = __ushort_as_half(0);
       e[q] = __ushort_as_half(0xfc00);  // -inf: an unused slot is never entered
       if (nd.child[q] == kEmptyChild) continue;
-      const double a = ((double)l[q] - centre) / half, b = ((double)h[q] - centre) / half;
-      const __half m = __double2half(0.5 * a + 0.5 * b);
-      const double need = fmax(b - (double)__half2float(m), (double)__half2float(m) - a) * (1.0 + 1e-6);
-      // infinite or NaN planes: everything along this axis (+inf)
-      const bool ok = need >= 0.0 && need < 60000.0;
+      const float a = (l[q] - centre) * scale, b = (h[q] - centre) * scale;
+      const __half m = __float2half_rn(0.5f * a + 0.5f * b);
+      const float need = fmaxf(b - __half2float(m), __half2float(m) - a) + 1e-6f;
+      // infinite or NaN planes, or outside the domain: everything along this axis (+inf)
+      const bool ok = need >= 0.0f && fabsf(a) <= 1.0001f && fabsf(b) <= 1.0001f;
       c[q] = ok ? m : __ushort_as_half(0);
-      e[q] = ok ? __float2half_ru(__double2float_ru(need)) : __ushort_as_half(0x7c00);
+      e[q] = ok ? __float2half_ru(need) : __ushort_as_half(0x7c00);
     }
   };
   axis(0, nd.lox, nd.hix, w.cx, w.ex);
