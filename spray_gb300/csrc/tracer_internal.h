@@ -94,6 +94,19 @@ inline void devFree(T*& p) {
   p = nullptr;
 }
 
+// A device array for the length of a scope.
+template <class T>
+struct DeviceBuffer {
+  T* p = nullptr;
+  explicit DeviceBuffer(size_t n) { devAlloc(&p, n); }
+  ~DeviceBuffer() { devFree(p); }
+  DeviceBuffer(const DeviceBuffer&) = delete;
+  DeviceBuffer& operator=(const DeviceBuffer&) = delete;
+};
+
+// Bytes of domains packed into one upload.
+constexpr size_t kUploadBytes = (size_t)64 << 20;
+
 // Ray pool of the non-speculative round loop (rounds.cu), one entry per ray.
 struct RoundRays {
   float4* org;  // xyz; w = occlusion range of a shadow ray (infinite for radiance)
@@ -127,6 +140,16 @@ void buildPack(const spray_gpu_domain& src, int d, DomainPack& p, bool bvh = tru
 // `src`, built on the current device (bvh_build.cu).
 void buildBvhsOnDevice(const spray_gpu_domain* src, const std::vector<int>& which, std::vector<DomainPack>& packs,
                        cudaStream_t stream, uint64_t batch_tris);
+// The same for meshes on the device: leaf-ordered triangles into `tris` (3 float4
+// per triangle, meshes back to back), the nodes back to back into a new device
+// allocation *nodes, each mesh's node count and the deepest tree.
+struct DeviceMesh {
+  const float* v;
+  const uint32_t* f;
+  uint32_t nf;
+};
+void buildBvhsInPlace(const std::vector<DeviceMesh>& meshes, cudaStream_t stream, uint64_t batch_tris, float4* tris,
+                      BvhNode4** nodes, std::vector<uint32_t>* counts, int* max_depth);
 // Prepared-domain blobs: one file per domain holding everything buildPack
 // makes, so that a scene is prepared once and loaded without rebuilding.
 std::string domainBlobPath(const std::string& dir, int d);
@@ -203,6 +226,8 @@ class Tracer {
   void captureHits(int b);
   void captureShadows(int b, int S);
   void installScene(std::vector<DomainPack>& packs, const spray_gpu_light* ls, int nl);
+  void setResidentScene(const spray_gpu_domain* doms, int nd);
+  void finishScene(const spray_gpu_light* ls, int nl);
   void setupOutOfCore(std::vector<DomainPack>& packs, int capacity, size_t max_nodes, size_t max_tris,
                       size_t max_verts, size_t slot_bytes);
   void loadDomain(int d, int slot, cudaStream_t s);
@@ -278,6 +303,7 @@ class Tracer {
   // in-core frame captured as a CUDA graph; recaptured when buffers change
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t buf_gen = 1, graph_gen = 0;
+  uint64_t first_gen = 0;        // buf_gen of the last frame launched without a graph
   int64_t graph_launches = 0;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> graph_sched, graph_trace, graph_occl;
   void captureFrame();
@@ -318,6 +344,9 @@ class Tracer {
 
   // wave buffers
   int64_t cap_samples = 0;
+  int cap_slots = 0;
+  char* h_upload = nullptr;      // pinned, packs the domains of a resident scene's upload
+  size_t h_upload_cap = 0;
   uint64_t cap_entries = 0, needed_entries = 0;
   int sched_blocks = 0, sched_warps = 0, sched_chunks = 0, compact_blocks = 0;
   int cur = 0;

@@ -1,0 +1,73 @@
+"""One tracer through a sequence of scenes, views and failed updates: the buffers
+and captured launches it keeps between them must never show the last scene."""
+import numpy as np
+import pytest
+
+import spray_gb300 as sg
+from spray_gb300 import scenes
+from conftest import small_config
+
+pytestmark = pytest.mark.gpu
+
+
+def bits(a):
+    return a.view(np.uint32)
+
+
+def _fresh(cfg, scene, cam):
+    t = sg.Tracer(cfg)
+    t.set_scene(scene)
+    t.set_camera(*cam)
+    return t.trace()[0]
+
+
+@pytest.mark.parametrize("shader", ["pt", "ao"])
+def test_scenes_one_after_the_other(lib_built, shader):
+    cfg = small_config(image_w=53, image_h=41, ao_mode=int(shader == "ao"), ao_samples=3, pixel_samples=2,
+                       bounces=1 if shader == "ao" else 3)
+    t = sg.Tracer(cfg)
+    # domain counts, meshes and lights (shadow rays per hit) grow and shrink
+    for grid, mesh, light in ((2, 24, "point"), (3, 20, "point+diffuse"), (1, 32, "quad"), (3, 28, "point+diffuse"),
+                              (2, 24, "point")):
+        sc = scenes.wavelet_grid(grid, mesh, colors="albedo", light=light)
+        cam = scenes.orbit_camera(sc, frame=grid)
+        t.set_scene(sc)
+        t.set_camera(*cam)
+        want = _fresh(cfg, sc, cam)
+        for _ in range(3):  # launched directly, captured, replayed
+            assert np.array_equal(bits(t.trace()[0]), bits(want))
+
+
+def test_more_shadow_rays_per_hit_than_the_last_frame(lib_built):
+    sc = scenes.wavelet_grid(2, 24, colors="albedo", light="point")
+    cfg = small_config(image_w=64, image_h=48, ao_mode=0, pixel_samples=2, bounces=2)
+    pos, look, up = scenes.orbit_camera(sc)
+    t = sg.Tracer(cfg)
+    t.set_scene(sc)
+    t.set_camera(pos, look, up)
+    first = t.trace()[0]
+    view = dict(position=pos, lookat=look, up=up, image_w=64, image_h=48, pixel_samples=2, ao_mode=1, ao_samples=16,
+                bounces=1)
+    got = t.trace_views([view])[0][0]
+    want = _fresh(dict(cfg, ao_mode=1, ao_samples=16, bounces=1), sc, (pos, look, up))
+    assert np.array_equal(bits(got), bits(want))
+    assert np.array_equal(bits(t.trace()[0]), bits(first))
+
+
+def test_a_failed_update_leaves_no_scene(lib_built):
+    sc = scenes.wavelet_grid(2, 24, colors="albedo", light="point")
+    cam = scenes.orbit_camera(sc)
+    t = sg.Tracer(small_config(image_w=32, image_h=32))
+    t.set_scene(sc)
+    t.set_camera(*cam)
+    want = t.trace()[0]
+    t.trace()
+    bad = sg.Scene([sg.Domain(np.zeros((3, 3), np.float32), [[0, 1, 7]])], sc.lights)
+    with pytest.raises(sg.SprayError) as e:
+        t.set_scene(bad)
+    assert e.value.code == sg.EINVAL and "face index" in str(e.value)
+    with pytest.raises(sg.SprayError) as e:
+        t.trace()
+    assert e.value.code == sg.ESTATE
+    t.set_scene(sc)
+    assert np.array_equal(bits(t.trace()[0]), bits(want))
