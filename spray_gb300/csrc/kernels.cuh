@@ -48,12 +48,13 @@ struct DomainDev {
   int32_t face_base;       // first index triple (original face order)
   int32_t bsdf;
   float bsdf_p[3];
-  int32_t resident;        // 1: geometry in a device slot (the *_base offsets); 2: traced in
-                           // place from pinned host memory (the src_* pointers); 0: neither
+  int32_t resident;        // 1: in core (the *_base offsets); out of core 2: traced in place from
+                           // pinned host memory, 3: in a device cache slot (the src_* pointers);
+                           // 0: nowhere
   int32_t num_nodes;       // BVH nodes of the domain
   int32_t num_tris;        // triangles of the domain
-  // out of core: the domain's arrays in mapped pinned host memory, read over
-  // the host link when the domain is traced in place
+  // out of core: the domain's arrays, in its cache slot or in mapped pinned host
+  // memory, which is read over the host link
   const BvhNode4* src_nodes;
   const float4* src_tris;
   const uint32_t* src_faces;
@@ -88,7 +89,7 @@ struct DomArrays {
 
 __device__ __forceinline__ DomArrays domArrays(const SceneDev& sc, const DomainDev& d) {
   DomArrays a;
-  if (d.resident == 2) {
+  if (d.resident >= 2) {
     a.nodes = d.src_nodes;
     a.tris = d.src_tris;
     a.faces = d.src_faces;
@@ -493,5 +494,13 @@ struct LiveArgs {
   uint32_t cap;
 };
 void launchCountLive(cudaStream_t s, const LiveArgs& a);
+// Copies of whole domains into their cache slots, read from pinned host memory
+// (mapped) by a kernel; sizes are in 16-byte words.
+struct CopySeg {
+  const uint4* src;
+  uint4* dst;
+  uint64_t words;
+};
+void launchCopySegs(cudaStream_t s, const CopySeg* segs, int nseg);
 
 }  // namespace spray

@@ -633,7 +633,8 @@ void Tracer::traceRounds() {
         logLoad(id, hit ? 1 : 0, hit ? -1 : evicted);
         if (!hit) {
           if (evicted >= 0) hdoms[evicted].resident = 0;
-          loadDomain(id, slot, stream);
+          const CopySeg c = loadDomain(id, slot);
+          CK(cudaMemcpyAsync(c.dst, h_pinned + host_off[id], c.words * 16, cudaMemcpyHostToDevice, stream));
           DomainDev* sd = reinterpret_cast<DomainDev*>(h_stage);
           std::memcpy(sd, hdoms.data(), D * sizeof(DomainDev));
           CK(cudaMemcpyAsync(d_domains, sd, D * sizeof(DomainDev), cudaMemcpyHostToDevice, stream));

@@ -9,6 +9,8 @@
 // A closest hit is folded into the ray's packed (t | triangle) key with a
 // 64-bit atomicMin, so the winner does not depend on the order in which the
 // domains were visited.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "spray_math.cuh"
 #include "traverse.cuh"
@@ -525,6 +527,33 @@ __global__ void __launch_bounds__(256) kCountLive(LiveArgs a) {
 
 void launchCountLive(cudaStream_t s, const LiveArgs& a) {
   if (a.ndomains > 0) kCountLive<<<a.ndomains, 256, 0, s>>>(a);
+}
+
+// 16 blocks per domain, four 16-byte loads in flight per thread.  The host link
+// gives 211 GB/s to a kernel as to one large copy; domains of 1.6 MB copied one by
+// one reach 166 GB/s, and their five arrays one by one 87.  A running traversal
+// fills the SMs' registers, so this serves only passes that load before they
+// trace; passes that load beside a running batch use the copy engine.
+constexpr int kCopyBlocks = 16;
+
+__global__ void __launch_bounds__(256) kCopySegs(const CopySeg* __restrict__ segs) {
+  const CopySeg c = segs[blockIdx.y];
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  for (; i + 3 * stride < c.words; i += 4 * stride) {
+    const uint4 v0 = __ldcs(c.src + i), v1 = __ldcs(c.src + i + stride);
+    const uint4 v2 = __ldcs(c.src + i + 2 * stride), v3 = __ldcs(c.src + i + 3 * stride);
+    c.dst[i] = v0;
+    c.dst[i + stride] = v1;
+    c.dst[i + 2 * stride] = v2;
+    c.dst[i + 3 * stride] = v3;
+  }
+  for (; i < c.words; i += stride) c.dst[i] = __ldcs(c.src + i);
+}
+
+void launchCopySegs(cudaStream_t s, const CopySeg* segs, int nseg) {
+  for (int k = 0; k < nseg; k += 65535)  // grid height
+    kCopySegs<<<dim3(kCopyBlocks, std::min(nseg - k, 65535)), 256, 0, s>>>(segs + k);
 }
 
 }  // namespace spray

@@ -358,6 +358,9 @@ void Tracer::freeScene() {
   h_stage = nullptr;
   if (h_live) cudaFreeHost(h_live);
   h_live = nullptr;
+  if (h_copies) cudaFreeHost(h_copies);
+  h_copies = d_copies = nullptr;
+  devFree(d_cache);
   devFree(d_live);
   devFree(d_live_doms);
   ooc = false;
@@ -829,48 +832,39 @@ void Tracer::finishScene(const spray_gpu_light* ls, int nl) {
 void Tracer::setupOutOfCore(std::vector<DomainPack>& packs, int capacity, size_t max_nodes,
                             size_t max_tris, size_t max_verts, size_t slot_bytes) {
   cache_capacity = capacity;
-  slot_nodes = max_nodes;
-  slot_tris = max_tris;
-  slot_verts = max_verts;
   cache_slot_bytes = slot_bytes;
-  // one pinned arena: per domain nodes | tris | faces | colours | normals
+  slot_stride = (blockOf(max_nodes, max_tris, max_verts).bytes + 255) & ~(size_t)255;
+  // one pinned arena: a block per domain
   host_off.assign(D, 0);
   size_t total = 0;
   for (int d = 0; d < D; ++d) {
     host_off[d] = total;
-    const DomainPack& p = packs[d];
-    total += p.nodes.size() * sizeof(BvhNode4) + p.tris.size() * sizeof(float4) + p.faces.size() * 4 +
-             p.colors.size() * 4 + p.normals.size() * 4;
-    total = (total + 255) & ~(size_t)255;
+    total += (blockOf(d).bytes + 255) & ~(size_t)255;
   }
   // mapped, so that a domain can also be traced in place over the host link
   CK(cudaHostAlloc((void**)&h_pinned, std::max<size_t>(total, 256), cudaHostAllocMapped));
-  char* dev_pinned = nullptr;
   CK(cudaHostGetDevicePointer((void**)&dev_pinned, h_pinned, 0));
+#pragma omp parallel for schedule(dynamic, 1)
   for (int d = 0; d < D; ++d) {
     const DomainPack& p = packs[d];
     char* q = h_pinned + host_off[d];
+    const Block b = blockOf(d);
+    std::memcpy(q, p.nodes.data(), p.nodes.size() * sizeof(BvhNode4));
+    std::memcpy(q + b.tris, p.tris.data(), p.tris.size() * sizeof(float4));
+    std::memcpy(q + b.faces, p.faces.data(), p.faces.size() * 4);
+    std::memcpy(q + b.colors, p.colors.data(), p.colors.size() * 4);
+    std::memcpy(q + b.normals, p.normals.data(), p.normals.size() * 4);
+  }
+  for (int d = 0; d < D; ++d) {
     DomainDev& dd = hdoms[d];
-    auto put = [&](const void* src, size_t n) {
-      const char* at = dev_pinned + (q - h_pinned);
-      std::memcpy(q, src, n);
-      q += n;
-      return at;
-    };
-    dd.src_nodes = reinterpret_cast<const BvhNode4*>(put(p.nodes.data(), p.nodes.size() * sizeof(BvhNode4)));
-    dd.src_tris = reinterpret_cast<const float4*>(put(p.tris.data(), p.tris.size() * sizeof(float4)));
-    dd.src_faces = reinterpret_cast<const uint32_t*>(put(p.faces.data(), p.faces.size() * 4));
-    dd.src_colors = reinterpret_cast<const uint32_t*>(put(p.colors.data(), p.colors.size() * 4));
-    dd.src_normals = reinterpret_cast<const float*>(put(p.normals.data(), p.normals.size() * 4));
     dd.resident = 0;
     dd.node_base = dd.tri_base = dd.vert_base = dd.face_base = 0;
+    pointTo(d, dev_pinned + host_off[d]);
   }
   devAlloc(&d_domains, D);
-  devAlloc(&d_nodes, (size_t)capacity * max_nodes);
-  devAlloc(&d_tris, 3 * (size_t)capacity * max_tris);
-  devAlloc(&d_faces, 3 * (size_t)capacity * max_tris);
-  devAlloc(&d_colors, (size_t)capacity * max_verts);
-  devAlloc(&d_normals, 3 * (size_t)capacity * max_verts);
+  devAlloc(&d_cache, (size_t)capacity * slot_stride);
+  CK(cudaHostAlloc((void**)&h_copies, capacity * sizeof(CopySeg), cudaHostAllocMapped));
+  CK(cudaHostGetDevicePointer((void**)&d_copies, h_copies, 0));
   // segment tables (one per radiance depth bucket, one for shadows) of D + 1
   // begins and D + 1 prefixes each
   devAlloc(&d_segs, (kDepthBuckets + 1) * (2 * (size_t)D + 2));
@@ -916,30 +910,38 @@ bool LruSlots::load(int domain, int* slot, int* evicted) {
   return false;
 }
 
-// Copies a domain into a device slot (ordered on stream s, from pinned memory).
-void Tracer::loadDomain(int d, int slot, cudaStream_t s) {
+Tracer::Block Tracer::blockOf(size_t nodes, size_t ntris, size_t nverts) {
+  auto up = [](size_t n) { return (n + 15) & ~(size_t)15; };
+  Block b;
+  b.tris = nodes * sizeof(BvhNode4);
+  b.faces = b.tris + 3 * ntris * sizeof(float4);
+  b.colors = b.faces + up(12 * ntris);
+  b.normals = b.colors + up(4 * nverts);
+  b.bytes = b.normals + up(12 * nverts);
+  return b;
+}
+
+void Tracer::pointTo(int d, char* base) {
+  const Block b = blockOf(d);
   DomainDev& dd = hdoms[d];
-  const size_t nn = (size_t)dd.num_nodes, nt = (size_t)dd.num_tris;
-  // vertex count: colours + normals follow the faces in the pinned block
-  const char* q = h_pinned + host_off[d];
-  size_t nv = domain_verts[d];
-  dd.node_base = (int32_t)(slot * slot_nodes);
-  dd.tri_base = (int32_t)(slot * slot_tris);
-  dd.face_base = (int32_t)(slot * slot_tris);
-  dd.vert_base = (int32_t)(slot * slot_verts);
-  dd.resident = 1;
-  size_t b_nodes = nn * sizeof(BvhNode4), b_tris = 3 * nt * sizeof(float4), b_faces = 3 * nt * 4;
-  CK(cudaMemcpyAsync(d_nodes + dd.node_base, q, b_nodes, cudaMemcpyHostToDevice, s));
-  q += b_nodes;
-  CK(cudaMemcpyAsync(d_tris + 3 * (size_t)dd.tri_base, q, b_tris, cudaMemcpyHostToDevice, s));
-  q += b_tris;
-  CK(cudaMemcpyAsync(d_faces + 3 * (size_t)dd.face_base, q, b_faces, cudaMemcpyHostToDevice, s));
-  q += b_faces;
-  CK(cudaMemcpyAsync(d_colors + dd.vert_base, q, nv * 4, cudaMemcpyHostToDevice, s));
-  q += nv * 4;
-  CK(cudaMemcpyAsync(d_normals + 3 * (size_t)dd.vert_base, q, 3 * nv * 4, cudaMemcpyHostToDevice, s));
-  h2d_bytes += b_nodes + b_tris + b_faces + nv * 16;
+  dd.src_nodes = reinterpret_cast<const BvhNode4*>(base);
+  dd.src_tris = reinterpret_cast<const float4*>(base + b.tris);
+  dd.src_faces = reinterpret_cast<const uint32_t*>(base + b.faces);
+  dd.src_colors = reinterpret_cast<const uint32_t*>(base + b.colors);
+  dd.src_normals = reinterpret_cast<const float*>(base + b.normals);
+}
+
+// Gives domain d a device slot and counts its load; the caller copies the
+// returned block (whole, 16-byte words) before it is traced.
+CopySeg Tracer::loadDomain(int d, int slot) {
+  char* to = d_cache + (size_t)slot * slot_stride;
+  pointTo(d, to);
+  hdoms[d].resident = 3;
+  const size_t nn = (size_t)hdoms[d].num_nodes, nt = (size_t)hdoms[d].num_tris, nv = domain_verts[d];
+  h2d_bytes += nn * sizeof(BvhNode4) + 3 * nt * sizeof(float4) + 12 * nt + 16 * nv;
   ++domain_loads;
+  return CopySeg{reinterpret_cast<const uint4*>(dev_pinned + host_off[d]), reinterpret_cast<uint4*>(to),
+                 blockOf(d).bytes / 16};
 }
 
 // Traces the queues of an out-of-core scene: domains in `order` that have
@@ -965,14 +967,19 @@ void Tracer::traceOutOfCore(bool shadow, const std::vector<int>& order, int S) {
   size_t i = 0;
   while (i < todo.size()) {
     size_t j = std::min(todo.size(), i + (size_t)cache_capacity);
+    int nload = 0;
     for (size_t k = i; k < j; ++k) {
       int slot, evicted;
       const bool hit = lru.load(todo[k], &slot, &evicted);
       logLoad(todo[k], hit ? 1 : 0, hit ? -1 : evicted);
       if (!hit) {
         if (evicted >= 0) hdoms[evicted].resident = 0;
-        loadDomain(todo[k], slot, stream);
+        h_copies[nload++] = loadDomain(todo[k], slot);
       }
+    }
+    if (nload > 0) {
+      launchCopySegs(stream, d_copies, nload);
+      launches += 1;
     }
     // stage the domain table and the segment table (begin, prefix) of this batch
     DomainDev* sd = reinterpret_cast<DomainDev*>(h_stage);
@@ -1707,7 +1714,7 @@ void Tracer::oocPass(bool with_r, bool with_s, int S, int rb, int rb_first, int 
   // rest stay in `remaining`, domains without live entries are dropped
   // traced in place: not resident, and few live entries (by the counts in hlive)
   auto inPlace = [&](int d) {
-    return hdoms[d].resident != 1 && cfg.ooc_inplace > 0 &&
+    return hdoms[d].resident != 3 && cfg.ooc_inplace > 0 &&
            (uint64_t)(with_r ? hlive[d] : 0) + (with_s ? hlive[D + d] : 0) <= (uint64_t)cfg.ooc_inplace;
   };
   // B bounds the domains that go through the cache (resident or copied); those
@@ -1746,6 +1753,7 @@ void Tracer::oocPass(bool with_r, bool with_s, int S, int rb, int rb_first, int 
     for (int d : batch) {
       if (inPlace(d)) {
         hdoms[d].resident = 2;
+        pointTo(d, dev_pinned + host_off[d]);
         inplace.push_back(d);
         logLoad(d, 2, -1);
         continue;
@@ -1755,7 +1763,8 @@ void Tracer::oocPass(bool with_r, bool with_s, int S, int rb, int rb_first, int 
       logLoad(d, hit ? 1 : 0, hit ? -1 : evicted);
       if (!hit) {
         if (evicted >= 0) hdoms[evicted].resident = 0;
-        loadDomain(d, slot, cstream);
+        const CopySeg c = loadDomain(d, slot);
+        CK(cudaMemcpyAsync(c.dst, h_pinned + host_off[d], c.words * 16, cudaMemcpyHostToDevice, cstream));
       }
     }
     CK(cudaEventRecord(loaded, cstream));

@@ -230,7 +230,16 @@ class Tracer {
   void finishScene(const spray_gpu_light* ls, int nl);
   void setupOutOfCore(std::vector<DomainPack>& packs, int capacity, size_t max_nodes, size_t max_tris,
                       size_t max_verts, size_t slot_bytes);
-  void loadDomain(int d, int slot, cudaStream_t s);
+  // A domain's arrays in the pinned arena and, the same way, in a cache slot:
+  // byte offsets of triangles, faces, colours and normals after the nodes, and
+  // the size, all multiples of 16.
+  struct Block {
+    size_t tris, faces, colors, normals, bytes;
+  };
+  static Block blockOf(size_t nodes, size_t ntris, size_t nverts);
+  Block blockOf(int d) const { return blockOf(hdoms[d].num_nodes, hdoms[d].num_tris, domain_verts[d]); }
+  void pointTo(int d, char* base);  // hdoms[d]'s arrays
+  CopySeg loadDomain(int d, int slot);
   void traceOutOfCore(bool shadow, const std::vector<int>& order, int S);
   // domain-parallel (in-situ) execution (insitu.cu)
   bool situ() const { return insitu_ranks > 1; }
@@ -315,7 +324,11 @@ class Tracer {
   // out-of-core cache
   bool ooc = false;
   int cache_capacity = 0;
-  size_t slot_nodes = 0, slot_tris = 0, slot_verts = 0, cache_slot_bytes = 0;
+  char* d_cache = nullptr;        // cache_capacity slots of slot_stride bytes
+  char* dev_pinned = nullptr;     // the arena as the device addresses it
+  CopySeg* h_copies = nullptr;    // pinned, mapped: the loads of a pass that loads before it traces
+  CopySeg* d_copies = nullptr;    // the same list as the device addresses it
+  size_t slot_stride = 0, cache_slot_bytes = 0;
   char* h_pinned = nullptr;       // prepared domains, pinned
   std::vector<size_t> host_off;   // per domain offset into h_pinned
   char* h_stage = nullptr;        // pinned staging of the domain and segment tables
