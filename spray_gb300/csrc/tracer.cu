@@ -1799,44 +1799,52 @@ void Tracer::oocPass(bool with_r, bool with_s, int S, int rb, int rb_first, int 
   nextBatch(batch);
   cudaEvent_t loaded = poolEvent();
   if (!batch.empty()) issueLoads(batch, loaded);
-  const size_t tbl = 2 * (size_t)D + 2;  // words per segment table
+  // A batch's radiance entries go in one launch, its buckets one after the other
+  // in the segment table: nearer list positions are still taken first, and one
+  // launch has one tail (2048x2048, 8 spp, 216 domains: closest hits 19.2 -> 17.0 ms a
+  // frame against a launch per bucket).  With so many domains that the tables
+  // would crowd the traversal's shared memory, a launch per bucket.
+  const bool merge = rb_count > 1 && (size_t)(rb * D + 2 * (rb_count * D) + 2) * 4 <= kMergedTables;
+  const int nr_tables = merge ? 1 : rb_count;             // radiance tables, then the shadows'
+  const size_t per = (size_t)(merge ? rb_count : 1) * D;  // segments a radiance table may hold
   while (!batch.empty()) {
-    // domain table, then segment tables: radiance bucket 0..rb-1, shadows
+    // domain table, then segment tables (begins, prefixes): radiance, shadows
     DomainDev* sd = reinterpret_cast<DomainDev*>(h_stage);
     std::memcpy(sd, hdoms.data(), D * sizeof(DomainDev));
     // the device table of this batch marks them in place; later batches decide anew
     inplace_domains += (int64_t)inplace.size();
     for (int d : inplace) hdoms[d].resident = 0;
     uint32_t* seg = reinterpret_cast<uint32_t*>(h_stage + D * sizeof(DomainDev));
-    std::vector<int> nseg(rb + 1, 0);
-    for (int q = 0; q <= rb; ++q) {
-      const bool shadow = q == rb;
-      const bool on = shadow ? with_s : (with_r && q >= rb_first && q < rb_end);
-      uint32_t* beg = seg + q * tbl;
-      uint32_t* pre = beg + D + 1;
+    const size_t tbl = 2 * per + 1;  // words per table
+    std::vector<int> nseg(nr_tables + 1, 0);
+    for (int k = 0; k <= nr_tables; ++k) {
+      const bool shadow = k == nr_tables;
+      uint32_t* beg = seg + k * tbl;
+      uint32_t* pre = beg + (shadow ? (size_t)D : per);
       uint32_t run = 0;
-      if (on)
+      const int q0 = merge ? rb_first : rb_first + k, q1 = merge ? rb_end : q0 + 1;
+      for (int q = q0; q < (shadow ? q0 + 1 : q1) && (shadow ? with_s : with_r); ++q)
         for (int d : batch) {
           if (hlive[(shadow ? D : 0) + d] == 0) continue;
           const uint32_t b0 = shadow ? sk[d] : rk[q * D + d], b1 = shadow ? sk[d + 1] : rk[q * D + d + 1];
           if (b1 == b0) continue;
-          beg[nseg[q]] = b0;
-          pre[nseg[q]] = run;
+          beg[nseg[k]] = b0;
+          pre[nseg[k]] = run;
           run += b1 - b0;
-          ++nseg[q];
+          ++nseg[k];
         }
-      pre[nseg[q]] = run;
+      pre[nseg[k]] = run;
     }
     CK(cudaMemcpyAsync(d_domains, sd, D * sizeof(DomainDev), cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(d_segs, seg, (rb + 1) * tbl * 4, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(d_segs, seg, (nr_tables * tbl + 2 * (size_t)D + 1) * 4, cudaMemcpyHostToDevice, stream));
     // counts for the batch after this one, taken before this one traces
     counted = poolEvent();
     countLive(window(remaining), counted);
     CK(cudaStreamWaitEvent(stream, loaded, 0));
     // radiance buckets front to back (or predicted first), then the shadows
-    for (int q = 0; q <= rb; ++q) {
-      if (nseg[q] == 0) continue;
-      const bool shadow = q == rb;
+    for (int k = 0; k <= nr_tables; ++k) {
+      if (nseg[k] == 0) continue;
+      const bool shadow = k == nr_tables;
       CK(cudaMemsetAsync(d_work, 0, 4, stream));
       TraceArgs ta = traceArgs(shadow ? 0 : (rb > 1 ? 1 : 0), S);
       if (shadow) {
@@ -1844,9 +1852,9 @@ void Tracer::oocPass(bool with_r, bool with_s, int S, int rb, int rb_first, int 
         ta.key_start = d_skey_start;
         ta.num_entries = d_snum_entries;
       }
-      ta.seg_begin = d_segs + q * tbl;
-      ta.seg_prefix = ta.seg_begin + D + 1;
-      ta.nseg = nseg[q];
+      ta.seg_begin = d_segs + k * tbl;
+      ta.seg_prefix = ta.seg_begin + (shadow ? (size_t)D : per);
+      ta.nseg = nseg[k];
       cudaEvent_t e0 = poolEvent(), e1 = poolEvent();
       CK(cudaEventRecord(e0, stream));
       if (shadow) launchTraceOccluded(stream, ta, traceBlocks());

@@ -104,6 +104,9 @@ struct DeviceBuffer {
   DeviceBuffer& operator=(const DeviceBuffer&) = delete;
 };
 
+// Key and segment tables of a merged traversal launch (shared memory per block).
+constexpr size_t kMergedTables = (size_t)40 << 10;
+
 // Bytes of domains packed into one upload.
 constexpr size_t kUploadBytes = (size_t)64 << 20;
 
