@@ -30,6 +30,7 @@ constexpr int kW3 = kB2 + kHid, kB3 = kW3 + kHid * kHid;
 constexpr int kW4 = kB3 + kHid, kB4 = kW4 + kOutPad * kHid;
 constexpr int kParams = kB4 + kOutPad;  // 13520
 constexpr int kPartial = kParams + 2;   // per-CTA gradient, loss sum, labelled rows
+constexpr int kPartialPitch = (kPartial + 3) / 4 * 4;  // floats between the CTAs' partials
 
 // A training pair: the ray, its candidate domains in (t, id) order and the
 // position of the candidate that holds the closest hit (-1: none).
@@ -62,6 +63,8 @@ struct ArenaSource {
 struct Net {
   const float* params;       // kParams floats
   const float* boxes;        // 6 floats per domain: min xyz, max xyz
+  int num_boxes;             // boxes that may be read ahead of use,
+  const uint32_t* more_boxes;  // or their number on the device (null: num_boxes)
   Norm norm;
   int* error;                // set to nonzero when a bounded wait gave up
 };
@@ -82,15 +85,16 @@ void launchPredictSamples(cudaStream_t s, const Net& net, const Sample* samples,
 void launchEvaluate(cudaStream_t s, const Net& net, const Sample* samples, int64_t n, unsigned long long* counts,
                     int nblocks);
 // Gradient of the mean cross-entropy over the labelled rows of a batch:
-// every CTA writes a partial [kPartial] (gradient, loss sum, labelled rows).
+// CTA k writes partial[k * kPartialPitch ..] (gradient, loss sum, labelled rows).
 // The loss gradient is scaled by 1 / *labelled (0 when there are none), or by
 // `inv_count` when `labelled` is null.
 void launchGrad(cudaStream_t s, const Net& net, const Sample* batch, int64_t n, float inv_count,
                 const uint32_t* labelled, float* partial, int nblocks);
 // counts[i] = labelled rows of step first + i, i < steps, whose batch is rows
-// [k * b mod n, + b) of the n samples, cut at the last (k the step).
+// [k * b mod n, + b) of the n samples, cut at the last (k the step); *num_boxes =
+// 1 + the highest domain among the candidates of those rows.
 void launchCountLabelled(cudaStream_t s, const Sample* samples, int64_t n, int64_t b, int64_t first, int steps,
-                         uint32_t* counts);
+                         uint32_t* counts, uint32_t* num_boxes);
 // Sums `nparts` partials in order into grad[kParams + 2] and, when lr > 0,
 // applies one Adam step (beta1 0.9, beta2 0.999, eps 1e-8) at step `step`;
 // *mean_loss (optional) = loss sum / labelled rows.

@@ -20,7 +20,7 @@ static_assert(sizeof(spray_mlp_sample) == sizeof(ml::Sample), "sample layout");
 // A calling thread's workspace, kept between its calls (a call used to create a
 // stream and allocate and free its buffers, 140 us around a kernel of 20) and
 // freed when the thread ends: the per-CTA gradient partials (8 MB), a gradient,
-// the labelled rows of up to kCountSteps batches, and a pinned word that a
+// the labelled rows of up to kCountSteps batches and the boxes they name, and a pinned word that a
 // timed-out wait sets.  Work runs on the thread's own default stream, so threads
 // do not wait for one another; a call returns when its work is done, so one
 // workspace per thread and device is enough.
@@ -64,9 +64,9 @@ int setup(Workspace** out, int32_t device, bool training) {
     w.device = device;
   }
   if (e == cudaSuccess && training && !w.counts) {
-    e = cudaMalloc(&w.partial, (size_t)ml::gradBlocks(w.nsms) * ml::kPartial * sizeof(float));
+    e = cudaMalloc(&w.partial, (size_t)ml::gradBlocks(w.nsms) * ml::kPartialPitch * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&w.grad, ml::kPartial * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&w.counts, kCountSteps * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&w.counts, (kCountSteps + 1) * sizeof(uint32_t));
   }
   if (e != cudaSuccess) {
     w.release();
@@ -85,10 +85,12 @@ int finish(const Workspace& w) {
   return SPRAY_GPU_OK;
 }
 
-ml::Net net(const float* params, const float* boxes, const float norm[4], int* err) {
+ml::Net net(const float* params, const float* boxes, const uint32_t* num_boxes, const float norm[4], int* err) {
   ml::Net n;
   n.params = params;
   n.boxes = boxes;
+  n.num_boxes = 0;
+  n.more_boxes = num_boxes;
   for (int c = 0; c < 3; ++c) n.norm.centre[c] = norm[c];
   n.norm.scale = norm[3];
   n.error = err;
@@ -117,8 +119,8 @@ int spray_mlp_forward_dev(const float* params, const float* boxes, const float n
     if (int r = setup(&w, device, false)) return r;
     if (n == 0) return SPRAY_GPU_OK;
     const int64_t tiles = (n + ml::kTile - 1) / ml::kTile;
-    const int grid = (int)std::min<int64_t>(tiles, 5 * w->nsms);
-    ml::launchPredictSamples(cudaStreamPerThread, net(params, boxes, norm, w->err_dev),
+    const int grid = (int)std::min<int64_t>(tiles, w->nsms);
+    ml::launchPredictSamples(cudaStreamPerThread, net(params, boxes, nullptr, norm, w->err_dev),
                              reinterpret_cast<const ml::Sample*>(samples), n, logits, pred, grid);
     return finish(*w);
   } catch (const std::exception& ex) {
@@ -136,8 +138,8 @@ int spray_mlp_grad_dev(const float* params, const float* boxes, const float norm
     const int g = gradGrid(w->nsms, n);
     const cudaStream_t st = cudaStreamPerThread;
     const ml::Sample* q = reinterpret_cast<const ml::Sample*>(samples);
-    ml::launchCountLabelled(st, q, n, std::max<int64_t>(n, 1), 0, 1, w->counts);
-    ml::launchGrad(st, net(params, boxes, norm, w->err_dev), q, n, 0.0f, w->counts, w->partial, g);
+    ml::launchCountLabelled(st, q, n, std::max<int64_t>(n, 1), 0, 1, w->counts, w->counts + kCountSteps);
+    ml::launchGrad(st, net(params, boxes, w->counts + kCountSteps, norm, w->err_dev), q, n, 0.0f, w->counts, w->partial, g);
     ml::launchReduceAdam(st, w->partial, g, grad, nullptr, nullptr, nullptr, 0.0f, 0, nullptr);
     return finish(*w);
   } catch (const std::exception& ex) {
@@ -158,11 +160,12 @@ int spray_mlp_train_dev(float* params, float* adam_m, float* adam_v, const float
     const int g = gradGrid(w->nsms, b);
     const cudaStream_t st = cudaStreamPerThread;
     const ml::Sample* q = reinterpret_cast<const ml::Sample*>(samples);
-    ml::Net nt = net(params, boxes, norm, w->err_dev);
+    ml::Net nt = net(params, boxes, w->counts + kCountSteps, norm, w->err_dev);
     for (int k = 0; k < steps; ++k) {
       // the labelled rows of the next batches, on the device
       if (k % kCountSteps == 0)
-        ml::launchCountLabelled(st, q, n, b, k, std::min(kCountSteps, steps - k), w->counts);
+        ml::launchCountLabelled(st, q, n, b, k, std::min(kCountSteps, steps - k), w->counts,
+                                w->counts + kCountSteps);
       const int64_t start = ((int64_t)k * b) % n;
       const int64_t len = std::min<int64_t>(b, n - start);
       ml::launchGrad(st, nt, q + start, len, 0.0f, w->counts + k % kCountSteps, w->partial, g);

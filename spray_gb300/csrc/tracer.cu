@@ -1278,7 +1278,7 @@ void Tracer::schedule(bool shadow, int order_by_depth, uint32_t* count, uint32_t
     mlp::ArenaSource src = arenaSource();
     src.count = count;
     src.list = list;
-    mlp::launchPredictArena(stream, proposalNet(), src, d_pred, num_sms * 5);  // 5 CTAs per SM
+    mlp::launchPredictArena(stream, proposalNet(), src, d_pred, num_sms);
     a.pred = d_pred;
     launchSchedPartition(stream, a, D, sched_warps, d_scan_tmp, scan_words);
     launches += 7;
@@ -1989,7 +1989,7 @@ void Tracer::setupProposal() {
   put(ml::kW4, ml::kOutPad, ml::kHid, ml::kCand, ml::kHid, ml::kHid);
   devAlloc(&d_mlp, p.size());
   CK(cudaMemcpy(d_mlp, p.data(), p.size() * 4, cudaMemcpyHostToDevice));
-  devAlloc(&d_mlp_partial, (size_t)ml::gradBlocks(num_sms) * ml::kPartial);
+  devAlloc(&d_mlp_partial, (size_t)ml::gradBlocks(num_sms) * ml::kPartialPitch);
   // domain boxes and the normalisation of positions to the scene box
   std::vector<float> bx(6 * (size_t)D);
   float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -2034,6 +2034,8 @@ mlp::Net Tracer::proposalNet() const {
   mlp::Net n;
   n.params = d_mlp;
   n.boxes = d_boxes;
+  n.num_boxes = D;
+  n.more_boxes = nullptr;
   n.norm = mlp_norm;
   n.error = d_mlp_err;
   return n;
@@ -2055,7 +2057,7 @@ void Tracer::predictDomainCounts(bool run_predict) {
   // (atomics folded into the inference epilogue measured slower: they stall
   // the tensor-core tile loop more than this pass costs)
   if (run_predict) {
-    mlp::launchPredictArena(stream, proposalNet(), arenaSource(), d_pred, num_sms * 5);
+    mlp::launchPredictArena(stream, proposalNet(), arenaSource(), d_pred, num_sms);
     launches += 1;
   }
   mlp::launchPredCount(stream, arenaSource(), d_pred, d_predcount, num_sms * 4);
@@ -2094,7 +2096,7 @@ void Tracer::trainProposal() {
   unsigned long long ev[3] = {0ull, 0ull, 0ull};
   if (held > 0) {
     CK(cudaMemsetAsync(d_mlp_eval, 0, 3 * sizeof(unsigned long long), stream));
-    ml::launchEvaluate(stream, proposalNet(), d_pairs + n, held, d_mlp_eval, num_sms * 5);
+    ml::launchEvaluate(stream, proposalNet(), d_pairs + n, held, d_mlp_eval, num_sms);
     CK(cudaMemcpyAsync(ev, d_mlp_eval, sizeof(ev), cudaMemcpyDeviceToHost, stream));
   }
   CK(cudaStreamSynchronize(stream));
