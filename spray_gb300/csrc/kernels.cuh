@@ -407,8 +407,6 @@ struct EyeCull {
 void launchGenPrimary(cudaStream_t s, const ViewDev* views, const TileDev* tiles, int ntiles,
                       int64_t nsamples, RayBuf rays, uint32_t* alive_list, uint32_t* alive_count,
                       const EyeCull& cull, Counters* ctr);
-// Adds nsamples - *alive_count to Counters::eyes_culled (after the live flags' compaction).
-void launchCountCulled(cudaStream_t s, const uint32_t* alive_count, int64_t nsamples, Counters* ctr);
 // scan_tmp holds scan_words words, at least scanTmpWords(nkeys, nchunks) for
 // the fastest scan (fewer give a scan over fewer chunk groups).  Launches 5
 // kernels.
@@ -454,12 +452,27 @@ void launchCompact(cudaStream_t s, const uint8_t* flag, const uint32_t* n_dev, u
 // list must not alias src.
 void launchCompactList(cudaStream_t s, const uint32_t* src, const uint32_t* n_dev, const uint8_t* flag,
                        uint32_t* list, uint32_t* count, int32_t* index_of, uint32_t* block_tmp, int nblocks);
+// The write pass of a compaction.
+struct CompactArgs {
+  const uint8_t* flag;
+  const uint32_t* n_dev;   // elements: *n_dev * n_mul, or n_host when null
+  uint32_t n_mul;
+  uint64_t n_host;
+  const uint32_t* block_tmp;
+  uint32_t* list;
+  uint32_t* count;         // set: block_tmp holds kept counts, *count is written
+  int32_t* index_of;       // optional
+  const uint32_t* src;     // element k is src[k] (null: k)
+  unsigned long long* dropped;  // optional, with count: += elements not kept
+};
+// launchCompact of n flags in two launches; *dropped += flags not set.
+void launchCompactAlive(cudaStream_t s, const uint8_t* flag, uint64_t n, uint32_t* list, uint32_t* count,
+                        unsigned long long* dropped, uint32_t* block_tmp, int nblocks);
 // The write pass of launchCompact / launchCompactList when block_tmp already
 // holds each block's kept count (kShade's block counts): each block adds the
-// counts before its own, the last writes *count.  One launch.
-void launchCompactCounted(cudaStream_t s, const uint8_t* flag, const uint32_t* n_dev, uint32_t n_mul,
-                          uint32_t* list, uint32_t* count, int32_t* index_of, const uint32_t* src,
-                          uint32_t* block_tmp, int nblocks);
+// counts before its own, the last writes *count.  One launch, also for two.
+void launchCompactCounted(cudaStream_t s, const CompactArgs& a, int nblocks);
+void launchCompactPair(cudaStream_t s, const CompactArgs& a, const CompactArgs& b, int nblocks);
 // Adds the unoccluded shadow rays of the alive list's samples (*count of them,
 // shadow slot k of entry j at j * slots + k) to their pixels.
 void launchRetire(cudaStream_t s, float4* image, const ViewDev* views, const uint32_t* list, const uint32_t* count,

@@ -87,14 +87,6 @@ __global__ void kGenPrimary(const ViewDev* __restrict__ views, const TileDev* __
 // The culled eye rays of a wave: its samples less the live ones the
 // compaction kept (one thread; a counter per culled warp would serialise
 // hundreds of thousands of atomics on one address).
-__global__ void kCountCulled(const uint32_t* alive_count, int64_t nsamples, Counters* ctr) {
-  ctr->eyes_culled += (unsigned long long)(nsamples - (int64_t)*alive_count);
-}
-
-void launchCountCulled(cudaStream_t s, const uint32_t* alive_count, int64_t nsamples, Counters* ctr) {
-  kCountCulled<<<1, 1, 0, s>>>(alive_count, nsamples, ctr);
-}
-
 void launchGenPrimary(cudaStream_t s, const ViewDev* views, const TileDev* tiles, int ntiles, int64_t nsamples,
                       RayBuf rays, uint32_t* alive_list, uint32_t* alive_count, const EyeCull& cull,
                       Counters* ctr) {
@@ -740,76 +732,84 @@ __global__ void __launch_bounds__(1024) kCompactScan(uint32_t* block_tmp, int nb
 
 // block_tmp holds each block's first output position, or with `count` set,
 // each block's kept count: the block then adds the counts before its own and
-// the last block writes the total to *count (no separate scan launch).
-__global__ void kCompactWrite(const uint8_t* __restrict__ flag, const uint32_t* n_dev,
-                              uint32_t n_mul, uint64_t n_host, const uint32_t* block_tmp,
-                              uint32_t* list, int32_t* index_of, const uint32_t* __restrict__ src,
-                              uint32_t* count = nullptr) {
-  __shared__ uint32_t ws[33];
-  const uint64_t n = n_dev ? (uint64_t)(*n_dev) * n_mul : n_host;
-  const uint64_t per = compactPer(n_dev ? *n_dev : n_host, n_dev ? n_mul : 1u, gridDim.x);
+// the last block writes the total to *count (no separate scan launch) and adds
+// what was dropped to *dropped.  Blocks of kCompactThreads.
+constexpr int kCompactThreads = 256;
+__device__ __forceinline__ void compactWrite(const CompactArgs& a) {
+  constexpr int kWarps = kCompactThreads / 32;
+  __shared__ uint32_t ws[kWarps + 1];
+  const uint64_t n = a.n_dev ? (uint64_t)(*a.n_dev) * a.n_mul : a.n_host;
+  const uint64_t per = compactPer(a.n_dev ? *a.n_dev : a.n_host, a.n_dev ? a.n_mul : 1u, gridDim.x);
   const uint64_t b0 = min(n, per * blockIdx.x), b1 = min(n, b0 + per);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t base;
-  if (count) {
+  if (a.count) {
     uint32_t sum = 0;
-    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) sum += block_tmp[k];
-    for (int o = 16; o; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
+    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += kCompactThreads) sum += a.block_tmp[k];
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) ws[w] = sum;
     __syncthreads();
     base = 0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) base += ws[k];
+    for (int k = 0; k < kWarps; ++k) base += ws[k];
     __syncthreads();
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count = base + block_tmp[blockIdx.x];
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+      const uint32_t kept = base + a.block_tmp[blockIdx.x];
+      *a.count = kept;
+      if (a.dropped) *a.dropped += n - kept;
+    }
   } else {
-    base = block_tmp[blockIdx.x];
+    base = a.block_tmp[blockIdx.x];
   }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const uint32_t lt = laneMaskLt();
   // four elements per thread per round (element s + k * blockDim + thread:
   // order row k, warp, lane), so that a round's loads overlap and its two
-  // barriers cover 4 x blockDim elements
-  __shared__ uint32_t wk[4][8];
-  for (uint64_t s = b0; s < b1; s += 4 * (uint64_t)blockDim.x) {
+  // barriers cover 4 x blockDim elements; the round's 32 warp counts are scanned by
+  // a warp (one thread that walked them took a third of the pass)
+  __shared__ uint32_t wk[4 * kWarps];
+  static_assert(4 * kWarps == 32, "a warp scans a round's counts");
+  for (uint64_t s = b0; s < b1; s += 4 * kCompactThreads) {
     uint32_t id[4], bal[4];
     bool f[4], valid[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const uint64_t i = s + (uint64_t)k * blockDim.x + threadIdx.x;
+      const uint64_t i = s + (uint64_t)k * kCompactThreads + threadIdx.x;
       valid[k] = i < b1;
-      id[k] = valid[k] ? (src ? src[i] : (uint32_t)i) : 0u;
+      id[k] = valid[k] ? (a.src ? a.src[i] : (uint32_t)i) : 0u;
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      f[k] = valid[k] && flag[id[k]] != 0;
+      f[k] = valid[k] && a.flag[id[k]] != 0;
       bal[k] = __ballot_sync(0xffffffffu, f[k]);
-      if (lane == 0) wk[k][w] = __popc(bal[k]);
+      if (lane == 0) wk[k * kWarps + w] = __popc(bal[k]);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t run = 0;
-      for (int k = 0; k < 4; ++k)
-        for (int q = 0; q < nw; ++q) {
-          const uint32_t v = wk[k][q];
-          wk[k][q] = run;
-          run += v;
-        }
-      ws[32] = run;
+    if (w == 0) {
+      uint32_t total;
+      wk[lane] = warpScan(wk[lane], &total);
+      if (lane == 0) ws[kWarps] = total;
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       if (!valid[k]) continue;
       if (f[k]) {
-        const uint32_t p = base + wk[k][w] + __popc(bal[k] & lt);
-        list[p] = id[k];
-        if (index_of) index_of[id[k]] = (int32_t)p;
-      } else if (index_of) {
-        index_of[id[k]] = -1;
+        const uint32_t p = base + wk[k * kWarps + w] + __popc(bal[k] & lt);
+        a.list[p] = id[k];
+        if (a.index_of) a.index_of[id[k]] = (int32_t)p;
+      } else if (a.index_of) {
+        a.index_of[id[k]] = -1;
       }
     }
-    base += ws[32];
+    base += ws[kWarps];
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(kCompactThreads) kCompactWrite(CompactArgs a) { compactWrite(a); }
+
+// Two independent compactions with the same grid.
+__global__ void __launch_bounds__(kCompactThreads) kCompactPair(CompactArgs a, CompactArgs b) {
+  compactWrite(blockIdx.y == 0 ? a : b);
 }
 
 void launchCompact(cudaStream_t s, const uint8_t* flag, const uint32_t* n_dev, uint32_t n_mul,
@@ -817,20 +817,31 @@ void launchCompact(cudaStream_t s, const uint8_t* flag, const uint32_t* n_dev, u
                    uint32_t* block_tmp, int nblocks) {
   kCompactCount<<<nblocks, 256, 0, s>>>(flag, n_dev, n_mul, n_host, block_tmp, nullptr);
   kCompactScan<<<1, 1024, 0, s>>>(block_tmp, nblocks, count);
-  kCompactWrite<<<nblocks, 256, 0, s>>>(flag, n_dev, n_mul, n_host, block_tmp, list, index_of, nullptr);
+  kCompactWrite<<<nblocks, kCompactThreads, 0, s>>>(
+      CompactArgs{flag, n_dev, n_mul, n_host, block_tmp, list, nullptr, index_of, nullptr, nullptr});
 }
 
-void launchCompactCounted(cudaStream_t s, const uint8_t* flag, const uint32_t* n_dev, uint32_t n_mul,
-                          uint32_t* list, uint32_t* count, int32_t* index_of, const uint32_t* src,
-                          uint32_t* block_tmp, int nblocks) {
-  kCompactWrite<<<nblocks, 256, 0, s>>>(flag, n_dev, n_mul, 0, block_tmp, list, index_of, src, count);
+void launchCompactAlive(cudaStream_t s, const uint8_t* flag, uint64_t n, uint32_t* list, uint32_t* count,
+                        unsigned long long* dropped, uint32_t* block_tmp, int nblocks) {
+  kCompactCount<<<nblocks, 256, 0, s>>>(flag, nullptr, 1, n, block_tmp, nullptr);
+  kCompactWrite<<<nblocks, kCompactThreads, 0, s>>>(
+      CompactArgs{flag, nullptr, 1, n, block_tmp, list, count, nullptr, nullptr, dropped});
+}
+
+void launchCompactCounted(cudaStream_t s, const CompactArgs& a, int nblocks) {
+  kCompactWrite<<<nblocks, kCompactThreads, 0, s>>>(a);
+}
+
+void launchCompactPair(cudaStream_t s, const CompactArgs& a, const CompactArgs& b, int nblocks) {
+  kCompactPair<<<dim3(nblocks, 2), kCompactThreads, 0, s>>>(a, b);
 }
 
 void launchCompactList(cudaStream_t s, const uint32_t* src, const uint32_t* n_dev, const uint8_t* flag,
                        uint32_t* list, uint32_t* count, int32_t* index_of, uint32_t* block_tmp, int nblocks) {
   kCompactCount<<<nblocks, 256, 0, s>>>(flag, n_dev, 1, 0, block_tmp, src);
   kCompactScan<<<1, 1024, 0, s>>>(block_tmp, nblocks, count);
-  kCompactWrite<<<nblocks, 256, 0, s>>>(flag, n_dev, 1, 0, block_tmp, list, index_of, src);
+  kCompactWrite<<<nblocks, kCompactThreads, 0, s>>>(
+      CompactArgs{flag, n_dev, 1, 0, block_tmp, list, nullptr, index_of, src, nullptr});
 }
 
 // ---------------------------------------------------------------- scores

@@ -1399,10 +1399,9 @@ void Tracer::beginWave(const Wave& w) {
                    d_alive_count, cull, d_ctr);
   launches += 1;
   if (cull.live) {
-    launchCompact(stream, d_next_flag, nullptr, 1, (uint64_t)w.samples, d_alive_list, d_alive_count, nullptr,
-                  d_block_tmp, std::min<int64_t>(compact_blocks, (w.samples + 255) / 256));
-    launchCountCulled(stream, d_alive_count, w.samples, d_ctr);
-    launches += 4;
+    launchCompactAlive(stream, d_next_flag, (uint64_t)w.samples, d_alive_list, d_alive_count, &d_ctr->eyes_culled,
+                       d_block_tmp, std::min<int64_t>(compact_blocks, (w.samples + 255) / 256));
+    launches += 2;
   }
 }
 
@@ -1429,9 +1428,20 @@ ShadeArgs Tracer::shadeArgs(int b, int S) {
   return sa;
 }
 
+// The compactions behind the shader, which left their block counts.
+CompactArgs Tracer::shadowCompaction(int S) const {
+  return CompactArgs{d_shadow_flag, d_alive_count, (uint32_t)S, 0, d_block_tmp, d_shadow_list, d_shadow_count,
+                     nullptr, nullptr, nullptr};
+}
+
+CompactArgs Tracer::nextCompaction() const {
+  return CompactArgs{d_next_flag, d_alive_count, 1, 0, d_block_tmp2, d_alive_list2, d_alive_count2,
+                     nullptr, d_alive_list, nullptr};
+}
+
 // A wave whose rays walk their domains themselves: per depth closest hits
-// (with the hits' colours and normals), shading, the shadow rays' compaction,
-// occlusion, retire and the next depth's alive list.
+// (with the hits' colours and normals), shading, the compactions (shadow rays,
+// the next depth's alive list), occlusion and retire.
 void Tracer::traceWaveWalks(const Wave& w) {
   const int S = std::max(slots(), 1);
   const int nb_total = maxBounces();
@@ -1455,8 +1465,10 @@ void Tracer::traceWaveWalks(const Wave& w) {
     sa.blk_shadow = d_block_tmp;
     sa.blk_next = d_block_tmp2;
     launchShade(stream, sa, ncr);
-    launchCompactCounted(stream, d_shadow_flag, d_alive_count, (uint32_t)S, d_shadow_list, d_shadow_count,
-                         nullptr, nullptr, d_block_tmp, ncr);
+    // this depth's shadow rays, and the next depth's alive rays
+    const bool more = b + 1 < nb_total;
+    if (more) launchCompactPair(stream, shadowCompaction(S), nextCompaction(), ncr);
+    else launchCompactCounted(stream, shadowCompaction(S), ncr);
     const RayWalkArgs ws = walkArgs(true, false, S);
     launchListDomains(stream, ws, ns);
     record(o0);
@@ -1465,12 +1477,9 @@ void Tracer::traceWaveWalks(const Wave& w) {
     occl_events.push_back({o0, o1});
     launchRetire(stream, d_image, d_views, d_alive_list, d_alive_count, rays[cur], sh, d_shadow_flag, S, nr);
     launches += 7;
-    if (b + 1 < nb_total) {
-      launchCompactCounted(stream, d_next_flag, d_alive_count, 1, d_alive_list2, d_alive_count2, nullptr,
-                           d_alive_list, d_block_tmp2, ncr);
+    if (more) {
       std::swap(d_alive_list, d_alive_list2);
       std::swap(d_alive_count, d_alive_count2);
-      launches += 1;
       cur ^= 1;
     }
   }
@@ -1563,8 +1572,7 @@ void Tracer::traceWave(const Wave& w, bool capture) {
     launchShade(stream, sa, compact_blocks);
     launches += 1;
     // shadow rays -> queues -> occlusion
-    launchCompactCounted(stream, d_shadow_flag, d_alive_count, (uint32_t)S, d_shadow_list, d_shadow_count,
-                         nullptr, nullptr, d_block_tmp, compact_blocks);
+    launchCompactCounted(stream, shadowCompaction(S), compact_blocks);
     launches += 1;
     // In core the shadow entries are sorted by list position (the ray's own
     // domain first): the occlusion walk takes them in that order, so an
@@ -1599,8 +1607,7 @@ void Tracer::traceWave(const Wave& w, bool capture) {
     // next depth
     if (b + 1 < nb_total) {
       // compact this depth's alive list (not every sample of the wave)
-      launchCompactCounted(stream, d_next_flag, d_alive_count, 1, d_alive_list2, d_alive_count2, nullptr,
-                           d_alive_list, d_block_tmp2, compact_blocks);
+      launchCompactCounted(stream, nextCompaction(), compact_blocks);
       std::swap(d_alive_list, d_alive_list2);
       std::swap(d_alive_count, d_alive_count2);
       launches += 1;

@@ -193,6 +193,8 @@ class Tracer {
   void freeBuffers();
   void traceWave(const Wave& w, bool capture);
   void traceWaveBatched(const Wave& w);
+  CompactArgs shadowCompaction(int S) const;
+  CompactArgs nextCompaction() const;
   void traceWaveWalks(const Wave& w);
   void beginWave(const Wave& w);
   ShadeArgs shadeArgs(int b, int S);
