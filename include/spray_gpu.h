@@ -185,7 +185,8 @@ typedef struct spray_gpu_stats {
   int64_t kernel_launches;  /* kernels this library launched during the frame */
   int64_t list_overflows;   /* rays whose domain list exceeded list_size */
   double frame_ms;          /* device time of the frame (CUDA events) */
-  double trace_ms;          /* device time inside the closest-hit kernel */
+  double trace_ms;          /* device time inside the closest-hit kernel; in core it shares the device with the
+                               last depth's occlusion, so these times can add up to more than the frame's */
   double occlude_ms;        /* device time inside the occlusion kernel */
   double schedule_ms;       /* device time inside the scheduling kernels */
   int64_t trace_launches;

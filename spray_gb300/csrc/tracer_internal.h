@@ -106,6 +106,9 @@ struct DeviceBuffer {
 
 // Key and segment tables of a merged traversal launch (shared memory per block).
 constexpr size_t kMergedTables = (size_t)40 << 10;
+// Side lists (occlusion beside the next closest hits) of more bytes than this are
+// given back before a scene is loaded.
+constexpr size_t kSideKept = (size_t)256 << 20;
 
 // Bytes of domains packed into one upload.
 constexpr size_t kUploadBytes = (size_t)64 << 20;
@@ -195,6 +198,7 @@ class Tracer {
   void traceWaveBatched(const Wave& w);
   CompactArgs shadowCompaction(int S) const;
   CompactArgs nextCompaction() const;
+  void chain(cudaStream_t from, cudaStream_t to);
   void traceWaveWalks(const Wave& w);
   void beginWave(const Wave& w);
   ShadeArgs shadeArgs(int b, int S);
@@ -212,7 +216,7 @@ class Tracer {
     return !ooc && !situ() && !learned() && !rounded() && cfg.cull && !cfg.debug_capture &&
            cfg.bucket_launches != kDepthBuckets && total_tris < kMaxWalkTris;
   }
-  RayWalkArgs walkArgs(bool shadow, bool primary, int S);
+  RayWalkArgs walkArgs(bool shadow, bool primary, int S, bool side);
   void setupProposal();
   void freeProposal();
   mlp::ArenaSource arenaSource() const;
@@ -282,7 +286,7 @@ class Tracer {
   spray_gpu_config cfg;
   int num_sms = 0;
   cudaStream_t stream = nullptr;
-  cudaStream_t cstream = nullptr;  // out-of-core domain copies, ahead of the traces
+  cudaStream_t cstream = nullptr;  // side stream: out-of-core domain copies ahead of the traces; occlusion in core
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   std::vector<cudaEvent_t> ev_pool;
   size_t ev_used = 0;
@@ -322,6 +326,7 @@ class Tracer {
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> graph_sched, graph_trace, graph_occl;
   void captureFrame();
   void record(cudaEvent_t e);
+  void record(cudaEvent_t e, cudaStream_t s);
   bool capturing = false;
   void dropGraph();
   std::vector<size_t> domain_verts;
@@ -430,6 +435,11 @@ class Tracer {
   unsigned int* d_walk_work = nullptr;
   unsigned long long* d_walk_top = nullptr;  // and an arena cursor
   uint2* d_list_ref = nullptr;
+  uint2* d_side_arena = nullptr;  // of the shadow rays' lists beside the next closest hits
+  uint2* d_side_ref = nullptr;
+  size_t side_bytes = 0;
+  bool side_refused = false;  // there was no memory for them
+  void freeSide();
   size_t walk_work_cap = 0, walk_launch = 0;
   size_t walkLaunches() const { return walksRays() ? waves.size() * (size_t)maxBounces() * 2 : 0; }
   void clearFrame();
