@@ -326,6 +326,7 @@ Tracer::Tracer(const spray_gpu_config& c) : cfg(c) {
   CK(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, cfg.device));
   CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&cstream, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&ostream, cudaStreamNonBlocking));
   CK(cudaEventCreate(&ev_start));
   CK(cudaEventCreate(&ev_stop));
   devAlloc(&d_ctr, 1);
@@ -344,6 +345,7 @@ Tracer::~Tracer() {
   if (ev_stop) cudaEventDestroy(ev_stop);
   if (stream) cudaStreamDestroy(stream);
   if (cstream) cudaStreamDestroy(cstream);
+  if (ostream) cudaStreamDestroy(ostream);
   if (h_reduce) cudaFreeHost(h_reduce);
   if (h_upload) cudaFreeHost(h_upload);
 }
@@ -1487,7 +1489,7 @@ void Tracer::traceWaveWalks(const Wave& w) {
   const int nr = blocks(w.samples, kStreamBlocksPerSm), ns = blocks(w.samples * S, kStreamBlocksPerSm);
   const int ncr = blocks(w.samples, kCompactBlocksPerSm);
   const bool side = nb_total > 1 && d_side_ref;
-  const cudaStream_t sst = side ? cstream : stream;
+  const cudaStream_t sst = side ? ostream : stream;
   beginWave(w);
   for (int b = 0; b < nb_total; ++b) {
     const bool more = b + 1 < nb_total;
@@ -1889,11 +1891,17 @@ void Tracer::oocPass(bool with_r, bool with_s, int S, int rb, int rb_first, int 
     counted = poolEvent();
     countLive(window(remaining), counted);
     CK(cudaStreamWaitEvent(stream, loaded, 0));
-    // radiance buckets front to back (or predicted first), then the shadows
+    // radiance buckets front to back (or predicted first), and beside them the
+    // shadows on a stream of their own: one launch's tail leaves the chip to the
+    // other (1600x900, 4 spp, 216 domains, learned order: 8.08 -> 7.75 ms a frame; 2048x2048, 8 spp:
+    // 34.7 -> 34.3)
+    const bool both = nseg[nr_tables] > 0 && *std::max_element(nseg.begin(), nseg.end() - 1) > 0;
+    const cudaStream_t ss = both ? ostream : stream;
+    if (both) chain(stream, ss);
     for (int k = 0; k <= nr_tables; ++k) {
       if (nseg[k] == 0) continue;
       const bool shadow = k == nr_tables;
-      CK(cudaMemsetAsync(d_work, 0, 4, stream));
+      const cudaStream_t st = shadow ? ss : stream;
       TraceArgs ta = traceArgs(shadow ? 0 : (rb > 1 ? 1 : 0), S);
       if (shadow) {
         ta.entries = d_sentries;
@@ -1903,14 +1911,17 @@ void Tracer::oocPass(bool with_r, bool with_s, int S, int rb, int rb_first, int 
       ta.seg_begin = d_segs + k * tbl;
       ta.seg_prefix = ta.seg_begin + (shadow ? (size_t)D : per);
       ta.nseg = nseg[k];
+      if (shadow) ta.work = d_work + 1;
+      CK(cudaMemsetAsync(ta.work, 0, 4, st));
       cudaEvent_t e0 = poolEvent(), e1 = poolEvent();
-      CK(cudaEventRecord(e0, stream));
-      if (shadow) launchTraceOccluded(stream, ta, traceBlocks());
-      else launchTraceClosest(stream, ta, traceBlocks());
-      CK(cudaEventRecord(e1, stream));
+      CK(cudaEventRecord(e0, st));
+      if (shadow) launchTraceOccluded(st, ta, traceBlocks());
+      else launchTraceClosest(st, ta, traceBlocks());
+      CK(cudaEventRecord(e1, st));
       (shadow ? occl_events : trace_events).push_back({e0, e1});
       launches += 1;
     }
+    if (both) chain(ss, stream);
     // the counts (and every trace before this batch's) have completed: the
     // staging buffers are free and the next batch's copies can start
     CK(cudaEventSynchronize(counted));

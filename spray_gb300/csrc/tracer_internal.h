@@ -286,7 +286,8 @@ class Tracer {
   spray_gpu_config cfg;
   int num_sms = 0;
   cudaStream_t stream = nullptr;
-  cudaStream_t cstream = nullptr;  // side stream: out-of-core domain copies ahead of the traces; occlusion in core
+  cudaStream_t cstream = nullptr;  // out-of-core domain copies, ahead of the traces
+  cudaStream_t ostream = nullptr;  // occlusion beside closest hits
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   std::vector<cudaEvent_t> ev_pool;
   size_t ev_used = 0;

@@ -84,6 +84,15 @@ def test_walks_equal_queues_at_odd_sizes(lib_built, w, h, spp):
     _pair(sc, scenes.orbit_camera(sc), image_w=w, image_h=h, ao_mode=0, pixel_samples=spp, bounces=3)
 
 
+@pytest.mark.parametrize("bounces", [1, 2, 6])
+@pytest.mark.parametrize("wave", [0, 5000])
+def test_walks_equal_queues_over_depths_and_waves(lib_built, bounces, wave):
+    """One depth runs on one stream, more beside each other's shadow rays; several waves share the buffers."""
+    sc = _boxes_scene(27, 5)
+    _pair(sc, scenes.orbit_camera(sc), image_w=131, image_h=77, ao_mode=0, ao_samples=2, pixel_samples=3,
+          bounces=bounces, wave_samples=wave, max_samples_per_rank=3000)
+
+
 @pytest.mark.parametrize("axis", [0, 1, 2])
 def test_walks_equal_queues_for_axis_parallel_rays(lib_built, axis):
     """A camera on a shared plane of the grid looking along an axis: the middle
