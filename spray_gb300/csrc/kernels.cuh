@@ -403,10 +403,11 @@ struct EyeCull {
   const uint32_t* bin_start = nullptr;
   int bin_shift = 0;
   uint8_t* live = nullptr;
+  uint32_t* block_live = nullptr;  // live samples of each block's range (the compaction's blocks)
 };
 void launchGenPrimary(cudaStream_t s, const ViewDev* views, const TileDev* tiles, int ntiles,
                       int64_t nsamples, RayBuf rays, uint32_t* alive_list, uint32_t* alive_count,
-                      const EyeCull& cull, Counters* ctr);
+                      const EyeCull& cull, Counters* ctr, int nblocks);
 // scan_tmp holds scan_words words, at least scanTmpWords(nkeys, nchunks) for
 // the fastest scan (fewer give a scan over fewer chunk groups).  Launches 5
 // kernels.
@@ -465,9 +466,6 @@ struct CompactArgs {
   const uint32_t* src;     // element k is src[k] (null: k)
   unsigned long long* dropped;  // optional, with count: += elements not kept
 };
-// launchCompact of n flags in two launches; *dropped += flags not set.
-void launchCompactAlive(cudaStream_t s, const uint8_t* flag, uint64_t n, uint32_t* list, uint32_t* count,
-                        unsigned long long* dropped, uint32_t* block_tmp, int nblocks);
 // The write pass of launchCompact / launchCompactList when block_tmp already
 // holds each block's kept count (kShade's block counts): each block adds the
 // counts before its own, the last writes *count.  One launch, also for two.

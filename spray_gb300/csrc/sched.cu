@@ -28,6 +28,13 @@ __device__ __forceinline__ uint32_t warpExclusiveScan(uint32_t v, uint32_t* tota
   return x - v;
 }
 
+// Elements per block of the compaction passes: whole groups of n_mul (the
+// shadow slots of one alive ray), so that a block's range is the range of
+// alive rays a shader block with the same grid covered (kShade's block counts).
+__host__ __device__ __forceinline__ uint64_t compactPer(uint64_t units, uint32_t n_mul, uint32_t blocks) {
+  return (units + blocks - 1) / blocks * n_mul;
+}
+
 // ---------------------------------------------------------------- primary rays
 // Eye rays of SpRay's Tracer::genSingleEyes / genMultiEyes
 // (src/ooc/ooc_tracer.inl:84-172) with Camera::generateRay
@@ -39,62 +46,80 @@ __device__ __forceinline__ uint32_t warpExclusiveScan(uint32_t v, uint32_t* tota
 // exact slab test of every domain fails for it): its record is not written,
 // live[i] = 0, and a compaction of `live` makes the alive list.  It still
 // counts as a primary ray.
-__global__ void kGenPrimary(const ViewDev* __restrict__ views, const TileDev* __restrict__ tiles, int ntiles,
-                            int64_t nsamples, RayBuf rays, uint32_t* alive_list, uint32_t* alive_count,
-                            EyeCull cull, Counters* ctr) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) {
+//
+// A block takes the contiguous range of samples that its block of the compaction
+// takes and leaves it the number of live ones, which saves the compaction's
+// counting pass (33 million samples, a third of them live: 270 us, with
+// that pass and a thread per sample, -> 132).
+__global__ void __launch_bounds__(256) kGenPrimary(const ViewDev* __restrict__ views,
+                                                   const TileDev* __restrict__ tiles, int ntiles, int64_t nsamples,
+                                                   RayBuf rays, uint32_t* alive_list, uint32_t* alive_count,
+                                                   EyeCull cull, Counters* ctr) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (!cull.live) *alive_count = (uint32_t)nsamples;
     atomicAdd(&ctr->rays_primary, (unsigned long long)nsamples);
   }
-  if (i >= nsamples) return;
-  // last tile with sample_base <= i
-  int lo = 0, hi = ntiles - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tiles[mid].sample_base <= i) lo = mid;
-    else hi = mid - 1;
+  const int64_t per = (int64_t)compactPer((uint64_t)nsamples, 1, gridDim.x);
+  const int64_t b0 = min(nsamples, per * blockIdx.x), b1 = min(nsamples, b0 + per);
+  uint32_t kept = 0;
+  int64_t tile_end = -1;  // of the tile in tl
+  TileDev tl{};
+  for (int64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
+    if (i >= tile_end) {
+      // last tile with sample_base <= i
+      int lo = 0, hi = ntiles - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tiles[mid].sample_base <= i) lo = mid;
+        else hi = mid - 1;
+      }
+      tl = tiles[lo];
+      tile_end = lo + 1 < ntiles ? tiles[lo + 1].sample_base : nsamples;
+    }
+    const ViewDev& vw = views[tl.view];
+    const CameraDev& cam = vw.cam;
+    const int spp = tl.spp;
+    const uint32_t bufid = (uint32_t)(i - tl.sample_base);
+    const uint32_t lp = spp > 1 ? bufid / (uint32_t)spp : bufid;
+    const uint32_t ly = lp / (uint32_t)tl.w;
+    const int x = tl.x + (int)(lp - ly * (uint32_t)tl.w);
+    const int y = tl.y + (int)ly;
+    if (cull.live) {
+      const int bin = vw.bin_base + (y >> cull.bin_shift) * vw.bins_x + (x >> cull.bin_shift);
+      const bool live = cull.bin_start[bin] != cull.bin_start[bin + 1];
+      cull.live[i] = live;
+      if (!live) continue;
+      ++kept;
+    }
+    float fx = (float)x, fy = (float)y;
+    if (spp > 1) {
+      uint32_t st = rngSeed((int32_t)bufid);
+      fx = (float)x + rngNext(st);
+      fy = (float)y + rngNext(st);
+    }
+    const V3 d = cameraRay(cam, fx, fy);
+    rays.org[i] = make_float4(cam.pos[0], cam.pos[1], cam.pos[2], 0.f);
+    rays.dir[i] = make_float4(d.x, d.y, d.z, 0.f);
+    rays.pixid[i] = y * vw.image_w + x;
+    rays.samid[i] = (int32_t)bufid;
+    rays.view[i] = (uint16_t)tl.view;
+    if (!cull.live) alive_list[i] = (uint32_t)i;
   }
-  const TileDev tl = tiles[lo];
-  const ViewDev& vw = views[tl.view];
-  const CameraDev& cam = vw.cam;
-  const int spp = tl.spp;
-  int32_t bufid = (int32_t)(i - tl.sample_base);
-  int32_t lp = spp > 1 ? bufid / spp : bufid;
-  int x = tl.x + lp % tl.w;
-  int y = tl.y + lp / tl.w;
   if (cull.live) {
-    const int bin = vw.bin_base + (y >> cull.bin_shift) * vw.bins_x + (x >> cull.bin_shift);
-    const bool live = cull.bin_start[bin] != cull.bin_start[bin + 1];
-    cull.live[i] = live;
-    if (!live) return;
+    __shared__ uint32_t sum;
+    if (threadIdx.x == 0) sum = 0;
+    __syncthreads();
+    kept = __reduce_add_sync(0xffffffffu, kept);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&sum, kept);
+    __syncthreads();
+    if (threadIdx.x == 0) cull.block_live[blockIdx.x] = sum;
   }
-  float fx = (float)x, fy = (float)y;
-  if (spp > 1) {
-    uint32_t st = rngSeed(bufid);
-    fx = (float)x + rngNext(st);
-    fy = (float)y + rngNext(st);
-  }
-  const V3 d = cameraRay(cam, fx, fy);
-  rays.org[i] = make_float4(cam.pos[0], cam.pos[1], cam.pos[2], 0.f);
-  rays.dir[i] = make_float4(d.x, d.y, d.z, 0.f);
-  rays.pixid[i] = y * vw.image_w + x;
-  rays.samid[i] = bufid;
-  rays.view[i] = (uint16_t)tl.view;
-  if (!cull.live) alive_list[i] = (uint32_t)i;
 }
 
-// The culled eye rays of a wave: its samples less the live ones the
-// compaction kept (one thread; a counter per culled warp would serialise
-// hundreds of thousands of atomics on one address).
 void launchGenPrimary(cudaStream_t s, const ViewDev* views, const TileDev* tiles, int ntiles, int64_t nsamples,
                       RayBuf rays, uint32_t* alive_list, uint32_t* alive_count, const EyeCull& cull,
-                      Counters* ctr) {
-  int threads = 256;
-  int64_t blocks = (nsamples + threads - 1) / threads;
-  if (blocks < 1) blocks = 1;
-  kGenPrimary<<<(unsigned)blocks, threads, 0, s>>>(views, tiles, ntiles, nsamples, rays, alive_list, alive_count,
-                                                   cull, ctr);
+                      Counters* ctr, int nblocks) {
+  kGenPrimary<<<nblocks, 256, 0, s>>>(views, tiles, ntiles, nsamples, rays, alive_list, alive_count, cull, ctr);
 }
 
 // ---------------------------------------------------------------- schedule
@@ -680,13 +705,6 @@ void launchSchedScatter(cudaStream_t s, const SchedArgs& a, int D, int nwarps) {
 }
 
 // ---------------------------------------------------------------- compaction
-// Elements per block of the compaction passes: whole groups of n_mul (the
-// shadow slots of one alive ray), so that a block's range is the range of
-// alive rays a shader block with the same grid covered (kShade's block counts).
-__host__ __device__ __forceinline__ uint64_t compactPer(uint64_t units, uint32_t n_mul, uint32_t blocks) {
-  return (units + blocks - 1) / blocks * n_mul;
-}
-
 __global__ void kCompactCount(const uint8_t* __restrict__ flag, const uint32_t* n_dev,
                               uint32_t n_mul, uint64_t n_host, uint32_t* block_tmp,
                               const uint32_t* __restrict__ src) {
@@ -819,13 +837,6 @@ void launchCompact(cudaStream_t s, const uint8_t* flag, const uint32_t* n_dev, u
   kCompactScan<<<1, 1024, 0, s>>>(block_tmp, nblocks, count);
   kCompactWrite<<<nblocks, kCompactThreads, 0, s>>>(
       CompactArgs{flag, n_dev, n_mul, n_host, block_tmp, list, nullptr, index_of, nullptr, nullptr});
-}
-
-void launchCompactAlive(cudaStream_t s, const uint8_t* flag, uint64_t n, uint32_t* list, uint32_t* count,
-                        unsigned long long* dropped, uint32_t* block_tmp, int nblocks) {
-  kCompactCount<<<nblocks, 256, 0, s>>>(flag, nullptr, 1, n, block_tmp, nullptr);
-  kCompactWrite<<<nblocks, kCompactThreads, 0, s>>>(
-      CompactArgs{flag, nullptr, 1, n, block_tmp, list, count, nullptr, nullptr, dropped});
 }
 
 void launchCompactCounted(cudaStream_t s, const CompactArgs& a, int nblocks) {

@@ -1417,14 +1417,16 @@ void Tracer::beginWave(const Wave& w) {
     cull.bin_start = d_bin_start;
     cull.bin_shift = kBinShift;
     cull.live = d_next_flag;
+    cull.block_live = d_block_tmp;
   }
+  const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(compact_blocks, (w.samples + 255) / 256));
   launchGenPrimary(stream, d_views, d_tiles + w.first_tile, w.num_tiles, w.samples, rays[0], d_alive_list,
-                   d_alive_count, cull, d_ctr);
+                   d_alive_count, cull, d_ctr, nb);
   launches += 1;
   if (cull.live) {
-    launchCompactAlive(stream, d_next_flag, (uint64_t)w.samples, d_alive_list, d_alive_count, &d_ctr->eyes_culled,
-                       d_block_tmp, std::min<int64_t>(compact_blocks, (w.samples + 255) / 256));
-    launches += 2;
+    launchCompactCounted(stream, CompactArgs{d_next_flag, nullptr, 1, (uint64_t)w.samples, d_block_tmp, d_alive_list,
+                                             d_alive_count, nullptr, nullptr, &d_ctr->eyes_culled}, nb);
+    launches += 1;
   }
 }
 
