@@ -106,6 +106,15 @@ __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t
       : "memory");
 }
 
+// The same with A in tensor memory: lane = row, a column = two elements along K.
+__device__ __forceinline__ void mmaTmem(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc, uint32_t on) {
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d),
+      "r"(a), "l"(b), "r"(idesc), "r"(acc), "r"(on)
+      : "memory");
+}
+
 __device__ __forceinline__ void commit(uint32_t bar, uint32_t on) {
   asm volatile(
       "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
@@ -133,6 +142,20 @@ __device__ __forceinline__ void gemm(uint32_t d, Operand a, Operand b, int K, in
 #pragma unroll
   for (int k = 0; k < K / 16; ++k) mma(d, a.at(k), b.at(k), id, (accumulate || k > 0) ? 1u : 0u, on);
 }
+
+__device__ __forceinline__ void gemmTmem(uint32_t d, uint32_t a, Operand b, int K, int N, uint32_t on) {
+  const uint32_t id = idescBf16(128, N, false, b.transposed);
+#pragma unroll
+  for (int k = 0; k < K / 16; ++k) mmaTmem(d, a + 8 * k, b.at(k), id, k > 0 ? 1u : 0u, on);
+}
+
+// N consecutive columns of this thread's lane, written.
+__device__ __forceinline__ void tmemSt8(uint32_t taddr, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmemStWait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // N consecutive fp32 accumulator columns of this thread's lane.
 __device__ __forceinline__ void tmemLd8(uint32_t taddr, float* v) {
@@ -366,20 +389,9 @@ __device__ __forceinline__ void candFeatures(const float* on, const float* d, co
   }
 }
 
-// The 64 features of a row -> its operand row x (128 bytes apart in 16-byte pieces).
-// Columns come in pairs, in order: 16 bytes are stored when complete.
-__device__ __forceinline__ void features(const Row& r, int t, const Net& net, const BoxCache& cache, uint8_t* x) {
-  uint4 q;
-  auto put = [&](int c, float a, float b) {
-    const uint32_t p = packBf16(a, b);
-    if ((c & 7) == 0) q.x = p;
-    else if ((c & 7) == 2) q.y = p;
-    else if ((c & 7) == 4) q.z = p;
-    else {
-      q.w = p;
-      *reinterpret_cast<uint4*>(x + opOff(t, c & ~7, 8)) = q;
-    }
-  };
+// The 64 features of a row, in order: put(column, value, value of column + 1).
+template <class Put>
+__device__ __forceinline__ void rowFeatures(const Row& r, const Net& net, const BoxCache& cache, Put&& put) {
   float on[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) on[c] = (r.o[c] - net.norm.centre[c]) * net.norm.scale;
@@ -390,6 +402,21 @@ __device__ __forceinline__ void features(const Row& r, int t, const Net& net, co
   for (int j = 0; j < kCand; j += 2) candFeatures(on, r.d, r.cand + j, j, r.ncand, net, cache, put);
 #pragma unroll
   for (int c = kIn; c < kK; c += 2) put(c, 0.0f, 0.0f);
+}
+
+// Row t of the operand x: 16 bytes are stored when complete.
+__device__ __forceinline__ void features(const Row& r, int t, const Net& net, const BoxCache& cache, uint8_t* x) {
+  uint4 q;
+  rowFeatures(r, net, cache, [&](int c, float a, float b) {
+    const uint32_t p = packBf16(a, b);
+    if ((c & 7) == 0) q.x = p;
+    else if ((c & 7) == 2) q.y = p;
+    else if ((c & 7) == 4) q.z = p;
+    else {
+      q.w = p;
+      *reinterpret_cast<uint4*>(x + opOff(t, c & ~7, 8)) = q;
+    }
+  });
 }
 __device__ __forceinline__ void noFeatures(int t, uint8_t* x) {
 #pragma unroll
@@ -513,25 +540,31 @@ struct ArenaRows {
   }
 };
 
-// Inference.  A CTA per SM of eight groups of 128 threads, each with its own tile
-// of rows, activation buffer, 64 tensor-memory columns and barriers; they share
-// the weights and the box records.  A tile's own chain (rows, features, four
-// products with a read-back each) is serial, so the groups fill each other's
-// waits.  Before, five CTAs of one group each held their own weights, and every
-// candidate read six scattered words of its box and took a square root and a
-// division from it: 1048576 rows 157 -> 81 us.
-constexpr int kFwdGroups = 8, kFwdThreads = kFwdGroups * kTile;
+// Inference.  A CTA per SM of five groups of 128 threads, each with its own tile of
+// rows, 96 tensor-memory columns and barriers; they share the weights and the box
+// records.  A tile's own chain (rows, features, four products with a read-back
+// each) is serial, so the groups fill each other's waits.  The activations stay in
+// tensor memory, written there as the next product's A: through shared memory they
+// were half of its traffic, which bound the kernel (80 % of its data pipe), although
+// eight groups fitted then.  1048576 rows: 157 us with five CTAs of one group that
+// held their own weights and read six scattered words of every candidate's box,
+// 81 us with eight groups and the activations in shared memory, now 71 us (four groups 79, three
+// 89); issue bounds it, 63 %.
+constexpr int kFwdGroups = 5, kFwdThreads = kFwdGroups * kTile;
 // Shared memory: W1 W2 W3 (8 KB each), W4 (2 KB), box records, biases, mbarriers,
-// the tensor-memory address; per group activations (16 KB) and staged samples.
+// the tensor-memory address; per group the staged samples.
 constexpr int kFwdW = 0, kFwdBox = 3 * 8192 + 2048, kFwdBias = kFwdBox + kBoxBytes;
 constexpr int kFwdBar = kFwdBias + (3 * kHid + kOutPad) * 4, kFwdSlot = kFwdBar + 8 * kFwdGroups;
-constexpr int kFwdAct = (kFwdSlot + 4 + 127) / 128 * 128, kFwdStage = kFwdAct + kFwdGroups * 16384;
-constexpr int kFwdSmem = kFwdStage + kFwdGroups * kStageBytes;
-static_assert(kFwdSmem <= 227 * 1024, "forward shared memory");  // one CTA per SM: 512 columns
-// D0 of group g: columns 64 g .. + 63; the logits reuse the first 16 once layer 3's
-// output has been read back (the tcgen05 fences around the barrier order the read
-// before the next MMA, as between the hidden layers)
-constexpr uint32_t kFwdCols = 64;
+constexpr int kFwdStage = (kFwdSlot + 4 + 15) / 16 * 16, kFwdSmem = 116 * 1024;
+static_assert(kFwdStage + kFwdGroups * kStageBytes <= kFwdSmem, "forward shared memory");
+// (more than half of an SM's, so that one CTA has it and its tensor memory alone)
+static_assert(2 * kFwdSmem > 227 * 1024, "one CTA per SM: 512 columns");
+// Group g: its accumulators in 64 columns from 96 g (the logits reuse the first 16
+// once layer 3's output has been read back; the tcgen05 fences around the barrier
+// order the read before the next MMA, as between the hidden layers), its
+// activations in the 32 after them.
+constexpr uint32_t kFwdCols = 96, kFwdAct = 64;
+static_assert(kFwdGroups * kFwdCols <= 512, "tensor memory");
 
 template <class Rows>
 __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
@@ -541,7 +574,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
   const int g = __shfl_sync(0xffffffffu, (int)threadIdx.x / kTile, 0), warp = __shfl_sync(0xffffffffu, t >> 5, 0);
   float* bias = reinterpret_cast<float*>(sm + kFwdBias);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kFwdSlot);
-  uint8_t* act = sm + kFwdAct + 16384 * g;
   uint8_t* stage = sm + kFwdStage + kStageBytes * g;
   BoxCache cache(sm + kFwdBox);
   const uint32_t mbar = smemAddr(sm + kFwdBar + 8 * g), stage_to = smemAddr(stage);
@@ -553,7 +585,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
   weights.load(net.params);
   cache.init(net, threadIdx.x, kFwdThreads);
   weights.store(sm + kFwdW, bias);
-  if (threadIdx.x < 32) tmemAlloc(smemAddr(tslot), kFwdCols * kFwdGroups);
+  if (threadIdx.x < 32) tmemAlloc(smemAddr(tslot), 512);
   if (t == 0) mbarInit(mbar, 1);
   fenceProxyAsync();
   fenceBeforeSync();
@@ -561,7 +593,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
   fenceAfterSync();
   const uint32_t tm = __shfl_sync(0xffffffffu, *tslot, 0) + kFwdCols * g;
   const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-  const Operand a_act{smemAddr(act), 1024u, false};
   const uint32_t b_w = smemAddr(sm + kFwdW);
   uint32_t phase = 0;
   bool ok = true;
@@ -572,14 +603,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
       barSync(1 + g, kTile);
     }
     int ncand = 0;
-    if (i < n) {
-      const Row r = rows.load(i, stage, t);
-      ncand = r.ncand;
-      features(r, t, net, cache, act);
-    } else {
-      noFeatures(t, act);
+    {
+      uint32_t x[kK / 2];
+      if (i < n) {
+        const Row r = rows.load(i, stage, t);
+        ncand = r.ncand;
+        rowFeatures(r, net, cache, [&](int c, float a, float b) { x[c / 2] = packBf16(a, b); });
+      } else {
+#pragma unroll
+        for (int c = 0; c < kK / 2; ++c) x[c] = 0u;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < kK / 2; c += 8) tmemSt8(tm + lane_base + kFwdAct + c, x + c);
     }
-    fenceProxyAsync();
+    tmemStWait();
     fenceBeforeSync();
     barSync(1 + g, kTile);
     const int64_t next = tile + (int64_t)gridDim.x * kFwdGroups;
@@ -589,8 +627,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
       if (warp == 0) {
         fenceAfterSync();
         const Operand w{b_w + 8192 * l, 1024u, false};
-        if (l < 3) gemm(tm, a_act, w, kK, kHid, false, t == 0);
-        else gemm(tm, a_act, w, kHid, kOutPad, false, t == 0);
+        if (l < 3) gemmTmem(tm, tm + kFwdAct, w, kK, kHid, t == 0);
+        else gemmTmem(tm, tm + kFwdAct, w, kHid, kOutPad, t == 0);
         commit(mbar, t == 0);
       }
       ok = ok && mbarWait(mbar, phase);
@@ -602,11 +640,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
         for (int h = 0; h < 4; ++h) {
           float z[16];
           tmemLd16(tm + lane_base + 16 * h, z);
-#pragma unroll
-          for (int c = 0; c < 16; c += 8)
-            *reinterpret_cast<uint4*>(act + opOff(t, 16 * h + c, 8)) = activate8(z + c, bias + l * kHid + 16 * h + c);
+          const uint4 a = activate8(z, bias + l * kHid + 16 * h), b = activate8(z + 8, bias + l * kHid + 16 * h + 8);
+          const uint32_t x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+          tmemSt8(tm + lane_base + kFwdAct + 8 * h, x);
         }
-        fenceProxyAsync();
+        tmemStWait();
         fenceBeforeSync();
         barSync(1 + g, kTile);
       } else {
@@ -632,7 +670,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
   fenceBeforeSync();
   __syncthreads();
   fenceAfterSync();
-  if (threadIdx.x < 32) tmemDealloc(*tslot, kFwdCols * kFwdGroups);
+  if (threadIdx.x < 32) tmemDealloc(*tslot, 512);
 }
 
 // Training.  A CTA per SM and 128 rows a tile as the partial sums have it.  The
