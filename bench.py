@@ -53,6 +53,16 @@ POLICIES = {"plain": (0, "plain speculative"), "resident": (1, "resident domains
 MEASURED_PEAKS = ROOT / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6800.0
 NODE_BYTES, TRI_BYTES, ENTRY_BYTES, RAY_BYTES, HIT_BYTES = 128, 48, 8, 32, 24
+WALK_NODE_BYTES = 64  # half-precision nodes of the in-core whole-ray walks
+
+
+def node_bytes(cfg: dict, num_domains: int) -> int:
+    """Bytes of a node as the frame's traversal reads it: whole-ray walks in core,
+    the queue kernels otherwise (out of core, learned order, round loop, captures)."""
+    size = cfg.get("cache_size", -1)
+    in_core = not cfg.get("cache_bytes") and (size <= 0 or size >= num_domains)
+    queues = cfg.get("debug_capture") or cfg.get("schedule_policy", 0) in (3, 5) or not cfg.get("cull", 1)
+    return WALK_NODE_BYTES if in_core and not queues and cfg.get("bucket_launches", 0) != 4 else NODE_BYTES
 
 
 def describe(name: str, spec: dict, cfg: dict) -> str:
@@ -262,12 +272,21 @@ def accuracy_report(scene, cfg, cam, mode_a_img, oracle_obj, device: int) -> dic
         hits[str(b)] = A.hit_agreement(rays, h, oracle_obj)
         shadows[str(b)] = A.shadow_agreement(t.debug(sg.DBG_SHADOWS, b), h, oracle_obj)
     t.close()
+    # the counts of the kernels that render the frame when nothing is captured,
+    # which must give the same image
+    t = sg.Tracer(cfg, device=device)
+    t.set_scene(scene)
+    t.set_camera(*cam)
+    plain, st = t.trace()
+    t.close()
     rep = A.frame_report(img, mode_a_img, mode_b, hits, shadows)
     rep["frame"] = [c["image_w"], c["image_h"]]
+    rep["captured_frame_equals_plain_frame"] = bool(np.array_equal(plain.view(np.uint32), img.view(np.uint32)))
+    nb = node_bytes(cfg, len(scene.domains))
     gpu_bytes = (st["visits_radiance"] * (RAY_BYTES + ENTRY_BYTES + HIT_BYTES)
-                 + st["nodes_radiance"] * NODE_BYTES + st["tris_radiance"] * TRI_BYTES)
+                 + st["nodes_radiance"] * nb + st["tris_radiance"] * TRI_BYTES)
     orc_bytes = (ost["bvh4_visits"] * (RAY_BYTES + ENTRY_BYTES + HIT_BYTES)
-                 + ost["bvh4_nodes"] * NODE_BYTES + ost["bvh4_tris"] * TRI_BYTES)
+                 + ost["bvh4_nodes"] * nb + ost["bvh4_tris"] * TRI_BYTES)
     rep["closest_hit_traversal"] = {
         "gpu": {"visits": st["visits_radiance"], "nodes": st["nodes_radiance"], "tris": st["tris_radiance"]},
         "oracle": {"visits": ost["bvh4_visits"], "nodes": ost["bvh4_nodes"], "tris": ost["bvh4_tris"],
@@ -597,10 +616,11 @@ def main():
 
     s0 = stats[-1]
     peak, peak_kind = hbm_peak()
+    nb = node_bytes(cfg, len(scene.domains))
     trace_bytes = (s0["visits_radiance"] * (RAY_BYTES + ENTRY_BYTES + HIT_BYTES)
-                   + s0["nodes_radiance"] * NODE_BYTES + s0["tris_radiance"] * TRI_BYTES)
+                   + s0["nodes_radiance"] * nb + s0["tris_radiance"] * TRI_BYTES)
     occl_bytes = (s0["visits_shadow"] * (RAY_BYTES + ENTRY_BYTES)
-                  + s0["nodes_shadow"] * NODE_BYTES + s0["tris_shadow"] * TRI_BYTES)
+                  + s0["nodes_shadow"] * nb + s0["tris_shadow"] * TRI_BYTES)
     if s0["trace_ms"] >= s0["occlude_ms"]:
         kname, kbytes, kms, klaunch = "closest-hit traversal", trace_bytes, s0["trace_ms"], s0["trace_launches"]
         kvisits = s0["visits_radiance"]
@@ -645,7 +665,9 @@ def main():
         # is the algorithmic bytes the walk requested (its own node and
         # triangle counts) per second against the HBM copy peak;
         # `achieved_floor` counts only the bytes every visit must move (ray,
-        # queue entry, hit record), a lower bound independent of the walk.
+        # queue entry, hit record), a lower bound independent of the walk.  In core
+        # a depth's occlusion runs beside the next depth's closest hits, and the
+        # kernel time includes what they take from each other.
         "roofline": {"bound": "latency", "peak_kind": "hbm", "kernel": kname, "achieved": achieved,
                      "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                      "traffic": traffic, "algorithmic_bytes_per_frame": kbytes,
