@@ -26,10 +26,13 @@
 #endif
 
 #ifndef SPRAY_WALK_STAY
-#define SPRAY_WALK_STAY 12
+#define SPRAY_WALK_STAY 8
 #endif
 #ifndef SPRAY_WALK_SWITCH
-#define SPRAY_WALK_SWITCH 8
+#define SPRAY_WALK_SWITCH 4
+#endif
+#ifndef SPRAY_WALK_LEAVES
+#define SPRAY_WALK_LEAVES 4
 #endif
 
 namespace spray {
@@ -40,11 +43,18 @@ constexpr int kWalkThreads = 256;
 // Idle lanes a warp gathers before it fetches new rays for them (closest hits
 // of that frame at 12, 16, 20 and 24: 4.13, 4.05, 4.00 and 4.17 ms).
 constexpr int kRefill = SPRAY_WALK_REFILL;
-// Lanes at the end of a domain that the warp gathers before it moves them on.
+// Lanes at the end of a domain that the warp gathers before it moves them on (24
+// views at 5, 8 and 12 before the runs of triangles below: 115.0, 115.9 and 119.7
+// ms; at 3 and 4 with them 112.3 and 112.2).
 constexpr int kSwitch = SPRAY_WALK_SWITCH;
 // Lanes at inner nodes with which a warp takes another node without weighing
-// the other steps.
+// the other steps (8, 12 and 16: 115.1, 115.9 and 116.6 ms; with the runs of
+// triangles 8 and 10: 112.2 and 112.7).
 constexpr int kStay = SPRAY_WALK_STAY;
+// And lanes at triangles with which it takes another triangle: leaves hold up to
+// eight, and weighing the steps is dear beside one test (one a round: 113.8 ms; 16,
+// 8, 5, 4, 3, 1: 114.4, 113.3, 112.3, 112.2, 112.3, 113.1 ms).
+constexpr int kLeaves = SPRAY_WALK_LEAVES;
 __device__ __forceinline__ uint32_t lanesBelowMask() {
   uint32_t m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -316,14 +326,15 @@ __device__ __forceinline__ uint32_t fetchWork(unsigned int* work, uint32_t idle,
 // rounds 15 to 19 lanes are active; then L1's requests bound the walks (75 % of
 // its data pipe with 128-byte nodes in four requests, 4.02 ms; in seven, 4.35),
 // so nodes take 64 bytes in two, which leaves instruction issue (70 %) and
-// latency: 3.68 ms.
+// latency: 3.68 ms.  Runs of triangles as well as of nodes take another 3 % off the
+// frame (7.05 -> 6.83 ms).
 template <bool kFull>
 __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, int spread) {
   const int lane = threadIdx.x & 31;
   uint32_t visits = 0, culled = 0, nnodes = 0, ntris = 0;
   const int lanes = kFull ? 32 : spread;
   const int refill = kFull ? kRefill : (lanes * kRefill + 31) / 32, turn = kFull ? kSwitch : (lanes * kSwitch + 31) / 32;
-  const int stay = kFull ? kStay : (lanes * kStay + 31) / 32;
+  const int stay = kFull ? kStay : (lanes * kStay + 31) / 32, leaves = kFull ? kLeaves : (lanes * kLeaves + 31) / 32;
   const uint32_t used = kFull ? 0xffffffffu : (1u << lanes) - 1u;
   bool has = false, exhausted = n == 0;
   uint32_t rid = 0, next = 0, end = 0;
@@ -429,28 +440,30 @@ __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, in
           }
         }
       } while (__popc(__ballot_sync(0xffffffffu, cur >= 0)) >= stay);
-    } else if (cur < 0 && cur != kDone) {
-      // the leaf's first triangle; the leaf reference moves on to the rest
-      const uint32_t v = ~(uint32_t)cur;
-      const uint32_t first = v >> 3;
-      {
-        ++ntris;
-        const float4* tp = a.scene.tris + 3 * (size_t)first;
-        const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
-        float t, u, vv;
-        if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
-                              kRayEpsilon, __int_as_float(0x7f800000), &t, &u, &vv)) {
-          const uint64_t key = packHitKey(t, a.domains[dom].gprim_base + __float_as_uint(ta.w));
-          if (key < best_key) {
-            best_key = key;
-            best_t = t;
-            best_u = u;
-            best_v = vv;
-            best_dom = dom;
+    } else {
+      do {
+        if (cur < 0 && cur != kDone) {
+          // the leaf's first triangle; the leaf reference moves on to the rest
+          const uint32_t v = ~(uint32_t)cur;
+          const uint32_t first = v >> 3;
+          ++ntris;
+          const float4* tp = a.scene.tris + 3 * (size_t)first;
+          const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+          float t, u, vv;
+          if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
+                                kRayEpsilon, __int_as_float(0x7f800000), &t, &u, &vv)) {
+            const uint64_t key = packHitKey(t, a.domains[dom].gprim_base + __float_as_uint(ta.w));
+            if (key < best_key) {
+              best_key = key;
+              best_t = t;
+              best_u = u;
+              best_v = vv;
+              best_dom = dom;
+            }
           }
+          cur = (v & 7u) ? (int)~(v + 7u) : pop();
         }
-        cur = (v & 7u) ? (int)~(v + 7u) : pop();
-      }
+      } while (__popc(__ballot_sync(0xffffffffu, cur < 0 && cur != kDone)) >= leaves);
     }
   }
   addCounts(&a.ctr->visits_radiance, visits, lane);
@@ -466,7 +479,7 @@ __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, i
   uint32_t visits = 0, nnodes = 0, ntris = 0;
   const int lanes = kFull ? 32 : spread;
   const int refill = kFull ? kRefill : (lanes * kRefill + 31) / 32, turn = kFull ? kSwitch : (lanes * kSwitch + 31) / 32;
-  const int stay = kFull ? kStay : (lanes * kStay + 31) / 32;
+  const int stay = kFull ? kStay : (lanes * kStay + 31) / 32, leaves = kFull ? kLeaves : (lanes * kLeaves + 31) / 32;
   const uint32_t used = kFull ? 0xffffffffu : (1u << lanes) - 1u;
   bool has = false, exhausted = n == 0;
   uint32_t rid = 0, next = 0, end = 0;
@@ -534,25 +547,27 @@ __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, i
           }
         }
       } while (__popc(__ballot_sync(0xffffffffu, cur >= 0)) >= stay);
-    } else if (cur < 0 && cur != kDone) {
-      const uint32_t v = ~(uint32_t)cur;
-      const uint32_t first = v >> 3;
-      {
-        ++ntris;
-        const float4* tp = a.scene.tris + 3 * (size_t)first;
-        const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
-        float t, u, vv;
-        if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
-                              kRayEpsilon, tfar, &t, &u, &vv)) {
-          nnodes += steps;
-          a.sh.occluded[rid] = 1;
-          has = false;
-          sp = 0;
-          cur = kDone;
-        } else {
-          cur = (v & 7u) ? (int)~(v + 7u) : (sp > 0 ? stack[--sp] : kDone);
+    } else {
+      do {
+        if (cur < 0 && cur != kDone) {
+          const uint32_t v = ~(uint32_t)cur;
+          const uint32_t first = v >> 3;
+          ++ntris;
+          const float4* tp = a.scene.tris + 3 * (size_t)first;
+          const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+          float t, u, vv;
+          if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
+                                kRayEpsilon, tfar, &t, &u, &vv)) {
+            nnodes += steps;
+            a.sh.occluded[rid] = 1;
+            has = false;
+            sp = 0;
+            cur = kDone;
+          } else {
+            cur = (v & 7u) ? (int)~(v + 7u) : (sp > 0 ? stack[--sp] : kDone);
+          }
         }
-      }
+      } while (__popc(__ballot_sync(0xffffffffu, cur < 0 && cur != kDone)) >= leaves);
     }
   }
   addCounts(&a.ctr->visits_shadow, visits, lane);
