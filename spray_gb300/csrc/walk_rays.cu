@@ -26,13 +26,16 @@
 #endif
 
 #ifndef SPRAY_WALK_STAY
-#define SPRAY_WALK_STAY 8
+#define SPRAY_WALK_STAY 7
 #endif
 #ifndef SPRAY_WALK_SWITCH
-#define SPRAY_WALK_SWITCH 4
+#define SPRAY_WALK_SWITCH 2
+#endif
+#ifndef SPRAY_WALK_SHADOW_SWITCH
+#define SPRAY_WALK_SHADOW_SWITCH 4
 #endif
 #ifndef SPRAY_WALK_LEAVES
-#define SPRAY_WALK_LEAVES 4
+#define SPRAY_WALK_LEAVES 5
 #endif
 
 namespace spray {
@@ -43,18 +46,15 @@ constexpr int kWalkThreads = 256;
 // Idle lanes a warp gathers before it fetches new rays for them (closest hits
 // of that frame at 12, 16, 20 and 24: 4.13, 4.05, 4.00 and 4.17 ms).
 constexpr int kRefill = SPRAY_WALK_REFILL;
-// Lanes at the end of a domain that the warp gathers before it moves them on (24
-// views at 5, 8 and 12 before the runs of triangles below: 115.0, 115.9 and 119.7
-// ms; at 3 and 4 with them 112.3 and 112.2).
-constexpr int kSwitch = SPRAY_WALK_SWITCH;
-// Lanes at inner nodes with which a warp takes another node without weighing
-// the other steps (8, 12 and 16: 115.1, 115.9 and 116.6 ms; with the runs of
-// triangles 8 and 10: 112.2 and 112.7).
-constexpr int kStay = SPRAY_WALK_STAY;
-// And lanes at triangles with which it takes another triangle: leaves hold up to
-// eight, and weighing the steps is dear beside one test (one a round: 113.8 ms; 16,
-// 8, 5, 4, 3, 1: 114.4, 113.3, 112.3, 112.2, 112.3, 113.1 ms).
-constexpr int kLeaves = SPRAY_WALK_LEAVES;
+// Lanes at the end of a domain that the warp gathers before it moves them on
+// (closest hits at 2, 3, 4 and 6: 6.62, 6.64, 6.72 and 6.75 ms a frame).
+constexpr int kSwitch = SPRAY_WALK_SWITCH, kShadowSwitch = SPRAY_WALK_SHADOW_SWITCH;
+// Lanes at inner nodes with which a warp takes another node, lanes at triangles
+// with which it takes another triangle (24 views, before the two followed each
+// other in a round: 8, 12 and 16 at nodes 115.1, 115.9 and 116.6 ms; 1, 4, 5, 8, 16
+// and no run at triangles 113.1, 112.2, 112.3, 113.3, 114.4 and 113.8 ms).
+constexpr int kStay = SPRAY_WALK_STAY, kLeaves = SPRAY_WALK_LEAVES;
+
 __device__ __forceinline__ uint32_t lanesBelowMask() {
   uint32_t m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -316,9 +316,10 @@ __device__ __forceinline__ uint32_t fetchWork(unsigned int* work, uint32_t idle,
 }  // namespace
 
 // Closest hits.  The lanes of a warp walk independently: each is at an inner
-// node, at a triangle, at the end of a domain, or idle, and every round of the
-// warp runs the step most lanes are at.  Idle lanes fetch new rays once
-// kRefill of them have gathered.
+// node, at a triangle, at the end of a domain, or idle, and a round of the warp
+// goes through the four: new rays for the idle lanes once kRefill have gathered,
+// domain ends once kSwitch have, then nodes and triangles, each as long as kStay,
+// kLeaves lanes are at one.
 //
 // Rays walk 12 nodes and 4 triangles each, unevenly: lanes that take whole
 // leaves and node runs together leave two thirds of a warp idle (7 to 13 of 32
@@ -326,8 +327,9 @@ __device__ __forceinline__ uint32_t fetchWork(unsigned int* work, uint32_t idle,
 // rounds 15 to 19 lanes are active; then L1's requests bound the walks (75 % of
 // its data pipe with 128-byte nodes in four requests, 4.02 ms; in seven, 4.35),
 // so nodes take 64 bytes in two, which leaves instruction issue (70 %) and
-// latency: 3.68 ms.  Runs of triangles as well as of nodes take another 3 % off the
-// frame (7.05 -> 6.83 ms).
+// latency: 3.68 ms.  Runs of triangles as well as of nodes took another 3 % off the
+// frame (7.05 -> 6.83 ms), rounds that go through the steps in turn instead of
+// running the one most lanes are at 3 % more (6.62 ms).
 template <bool kFull>
 __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, int spread) {
   const int lane = threadIdx.x & 31;
@@ -353,10 +355,8 @@ __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, in
     return kDone;
   };
   while (true) {
-    const uint32_t inner = __ballot_sync(0xffffffffu, cur >= 0);
-    const uint32_t leaf = __ballot_sync(0xffffffffu, cur < 0 && cur != kDone);
     const uint32_t idle = __ballot_sync(0xffffffffu, !has) & used;
-    const int ni = __popc(inner), nl = __popc(leaf), nd = __popc(idle), ne = lanes - ni - nl - nd;
+    const int nd = __popc(idle);
     if (nd == lanes || (nd >= refill && !exhausted)) {
       if (!has && best_key != kNoHit) {
         // the finished ray's hit: TriMeshBuffer::updateIntersection
@@ -393,7 +393,9 @@ __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, in
           has = true;
         }
       }
-    } else if (ne >= turn || (ni == 0 && nl == 0)) {
+    }
+    const uint32_t ends = __ballot_sync(0xffffffffu, has && cur == kDone);
+    if (__popc(ends) >= turn || !__any_sync(0xffffffffu, cur != kDone)) {
       if (has && cur == kDone) {
         // the next domain of the list; the rest start beyond the hit once one does
         has = next < end;
@@ -411,7 +413,8 @@ __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, in
         }
         if (!has) nnodes += steps;
       }
-    } else if (ni >= nl) {
+    }
+    if (__any_sync(0xffffffffu, cur >= 0)) {
       do {
         if (cur >= 0) {
           ++steps;
@@ -440,7 +443,8 @@ __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, in
           }
         }
       } while (__popc(__ballot_sync(0xffffffffu, cur >= 0)) >= stay);
-    } else {
+    }
+    if (__any_sync(0xffffffffu, cur < 0 && cur != kDone)) {
       do {
         if (cur < 0 && cur != kDone) {
           // the leaf's first triangle; the leaf reference moves on to the rest
@@ -472,13 +476,16 @@ __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, in
   addCounts(&a.ctr->tris_radiance, ntris, lane);
 }
 
-// Occlusion, in the same rounds.
+// Occlusion, in such rounds, but one that fetches rays or moves lanes on does no more
+// (24 views: 109.4 ms; as for closest hits 110.1): a new ray starts in its first
+// domain at once.
 template <bool kFull>
 __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, int spread) {
   const int lane = threadIdx.x & 31;
   uint32_t visits = 0, nnodes = 0, ntris = 0;
   const int lanes = kFull ? 32 : spread;
-  const int refill = kFull ? kRefill : (lanes * kRefill + 31) / 32, turn = kFull ? kSwitch : (lanes * kSwitch + 31) / 32;
+  const int refill = kFull ? kRefill : (lanes * kRefill + 31) / 32;
+  const int turn = kFull ? kShadowSwitch : (lanes * kShadowSwitch + 31) / 32;
   const int stay = kFull ? kStay : (lanes * kStay + 31) / 32, leaves = kFull ? kLeaves : (lanes * kLeaves + 31) / 32;
   const uint32_t used = kFull ? 0xffffffffu : (1u << lanes) - 1u;
   bool has = false, exhausted = n == 0;
@@ -489,10 +496,8 @@ __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, i
   int sp = 0, cur = kDone;
   uint32_t steps = 0;
   while (true) {
-    const uint32_t inner = __ballot_sync(0xffffffffu, cur >= 0);
-    const uint32_t leaf = __ballot_sync(0xffffffffu, cur < 0 && cur != kDone);
     const uint32_t idle = __ballot_sync(0xffffffffu, !has) & used;
-    const int ni = __popc(inner), nl = __popc(leaf), nd = __popc(idle), ne = lanes - ni - nl - nd;
+    const int nd = __popc(idle);
     if (nd == lanes && exhausted) break;
     if (nd >= refill && !exhausted) {
       const uint32_t i = fetchWork(a.work, idle, n, &exhausted);
@@ -512,7 +517,8 @@ __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, i
           cur = enterDomain(a, (int)a.arena[next++].x, r);
         }
       }
-    } else if (ne >= turn || (ni == 0 && nl == 0)) {
+    } else if (__popc(__ballot_sync(0xffffffffu, has && cur == kDone)) >= turn ||
+               !__any_sync(0xffffffffu, cur != kDone)) {
       if (has && cur == kDone) {
         has = next < end;
         if (has) {
@@ -523,51 +529,54 @@ __device__ __forceinline__ void walkOccluded(const RayWalkArgs& a, uint32_t n, i
           a.sh.occluded[rid] = 0;
         }
       }
-    } else if (ni >= nl) {
-      do {
-        if (cur >= 0) {
-          ++steps;
-          if (sp > kStack - 3) {
-            raise(a.ctr, kErrTraversalBound);
-            cur = kDone;
-            sp = 0;
-            next = end;
-          } else {
-            float tn[4];
-            bool hit[4];
-            const int4 ch = testNode<true>(a.nodes, cur, r, tfar, tn, hit);
-            int nx = kDone;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              if (!hit[c]) continue;
-              if (nx != kDone) stack[sp++] = nx;
-              nx = childAt(ch, c);
-            }
-            cur = nx != kDone ? nx : (sp > 0 ? stack[--sp] : kDone);
-          }
-        }
-      } while (__popc(__ballot_sync(0xffffffffu, cur >= 0)) >= stay);
     } else {
-      do {
-        if (cur < 0 && cur != kDone) {
-          const uint32_t v = ~(uint32_t)cur;
-          const uint32_t first = v >> 3;
-          ++ntris;
-          const float4* tp = a.scene.tris + 3 * (size_t)first;
-          const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
-          float t, u, vv;
-          if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
-                                kRayEpsilon, tfar, &t, &u, &vv)) {
-            nnodes += steps;
-            a.sh.occluded[rid] = 1;
-            has = false;
-            sp = 0;
-            cur = kDone;
-          } else {
-            cur = (v & 7u) ? (int)~(v + 7u) : (sp > 0 ? stack[--sp] : kDone);
+      if (__any_sync(0xffffffffu, cur >= 0)) {
+        do {
+          if (cur >= 0) {
+            ++steps;
+            if (sp > kStack - 3) {
+              raise(a.ctr, kErrTraversalBound);
+              cur = kDone;
+              sp = 0;
+              next = end;
+            } else {
+              float tn[4];
+              bool hit[4];
+              const int4 ch = testNode<true>(a.nodes, cur, r, tfar, tn, hit);
+              int nx = kDone;
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                if (!hit[c]) continue;
+                if (nx != kDone) stack[sp++] = nx;
+                nx = childAt(ch, c);
+              }
+              cur = nx != kDone ? nx : (sp > 0 ? stack[--sp] : kDone);
+            }
           }
-        }
-      } while (__popc(__ballot_sync(0xffffffffu, cur < 0 && cur != kDone)) >= leaves);
+        } while (__popc(__ballot_sync(0xffffffffu, cur >= 0)) >= stay);
+      }
+      if (__any_sync(0xffffffffu, cur < 0 && cur != kDone)) {
+        do {
+          if (cur < 0 && cur != kDone) {
+            const uint32_t v = ~(uint32_t)cur;
+            const uint32_t first = v >> 3;
+            ++ntris;
+            const float4* tp = a.scene.tris + 3 * (size_t)first;
+            const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+            float t, u, vv;
+            if (intersectTriangle(r.sh, r.org, v3(ta.x, ta.y, ta.z), v3(tb.x, tb.y, tb.z), v3(tc.x, tc.y, tc.z),
+                                  kRayEpsilon, tfar, &t, &u, &vv)) {
+              nnodes += steps;
+              a.sh.occluded[rid] = 1;
+              has = false;
+              sp = 0;
+              cur = kDone;
+            } else {
+              cur = (v & 7u) ? (int)~(v + 7u) : (sp > 0 ? stack[--sp] : kDone);
+            }
+          }
+        } while (__popc(__ballot_sync(0xffffffffu, cur < 0 && cur != kDone)) >= leaves);
+      }
     }
   }
   addCounts(&a.ctr->visits_shadow, visits, lane);
