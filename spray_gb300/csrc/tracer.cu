@@ -1851,15 +1851,23 @@ void Tracer::oocPass(bool with_r, bool with_s, int S, int rb, int rb_first, int 
   nextBatch(batch);
   cudaEvent_t loaded = poolEvent();
   if (!batch.empty()) issueLoads(batch, loaded);
-  // A batch's radiance entries go in one launch, its buckets one after the other
-  // in the segment table: nearer list positions are still taken first, and one
-  // launch has one tail (2048x2048, 8 spp, 216 domains: closest hits 19.2 -> 17.0 ms a
-  // frame against a launch per bucket).  With so many domains that the tables
-  // would crowd the traversal's shared memory, a launch per bucket.
-  const bool merge = rb_count > 1 && (size_t)(rb * D + 2 * (rb_count * D) + 2) * 4 <= kMergedTables;
-  const int nr_tables = merge ? 1 : rb_count;             // radiance tables, then the shadows'
-  const size_t per = (size_t)(merge ? rb_count : 1) * D;  // segments a radiance table may hold
   while (!batch.empty()) {
+    // A batch's radiance entries go in one launch, its buckets one after the other
+    // in the segment table: nearer list positions are still taken first, and one
+    // launch has one tail (2048x2048, 8 spp, 216 domains: closest hits 19.2 -> 17.0 ms a
+    // frame against a launch per bucket).  A launch per bucket when the tables would
+    // crowd the traversal's shared memory, and for less than two entries a lane: all
+    // buckets would be in flight at once and cull nothing (317x162, 8 spp, 64 domains
+    // in place: 1.15 ms a frame merged, 1.02 not; merged from 0, 2, 4, 8 entries a lane
+    // on the learned 1600x900 frame takes 7.71, 7.76, 8.34, 8.50 ms).
+    uint64_t entries = 0;
+    for (int q = rb_first; q < rb_end && with_r; ++q)
+      for (int d : batch)
+        if (hlive[d] > 0) entries += rk[q * D + d + 1] - rk[q * D + d];
+    const bool merge = rb_count > 1 && entries >= 2ull * 256 * traceBlocks() &&
+                       (size_t)(rb * D + 2 * (rb_count * D) + 2) * 4 <= kMergedTables;
+    const int nr_tables = merge ? 1 : rb_count;             // radiance tables, then the shadows'
+    const size_t per = (size_t)(merge ? rb_count : 1) * D;  // segments a radiance table may hold
     // domain table, then segment tables (begins, prefixes): radiance, shadows
     DomainDev* sd = reinterpret_cast<DomainDev*>(h_stage);
     std::memcpy(sd, hdoms.data(), D * sizeof(DomainDev));
