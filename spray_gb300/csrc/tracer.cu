@@ -1135,6 +1135,10 @@ void Tracer::planWaves() {
     frame_pixels += (int64_t)f.w * f.h;
     mix((uint64_t)f.ao_mode | ((uint64_t)f.bounces << 8) | ((uint64_t)f.ao_samples << 16));
   }
+  // what the launches of a captured frame hold beside the tiles (the shader settings
+  // themselves are read from the view table): shadow slots per alive ray, depths
+  mix((uint64_t)S);
+  mix((uint64_t)maxBounces());
   if (sig != plan_sig) {
     plan_sig = sig;
     ++buf_gen;  // the captured frame no longer matches

@@ -71,3 +71,21 @@ def test_a_failed_update_leaves_no_scene(lib_built):
     assert e.value.code == sg.ESTATE
     t.set_scene(sc)
     assert np.array_equal(bits(t.trace()[0]), bits(want))
+
+
+@pytest.mark.parametrize("order", ["ABA", "ABBA", "BAAB", "BAB", "AABBA"])
+@pytest.mark.parametrize("queues", [0, 4])
+def test_views_that_differ_in_their_shadow_slots_only(lib_built, order, queues):
+    # a captured frame holds the slots per hit: one of A's nine slots (light_shadow) may
+    # not be replayed for B's eight, nor the other way round
+    sc = scenes.wavelet_grid(2, 24, colors="albedo", light="point")
+    pos, look, up = scenes.orbit_camera(sc)
+    cfg = small_config(image_w=64, image_h=48, ao_mode=1, ao_samples=8, ao_max_distance=0.5, bucket_launches=queues)
+    want = {k: _fresh(dict(cfg, ao_light_shadow=int(k == "A")), sc, (pos, look, up)) for k in "AB"}
+    assert not np.array_equal(bits(want["A"]), bits(want["B"]))
+    t = sg.Tracer(cfg)
+    t.set_scene(sc)
+    for k in order:
+        view = dict(position=pos, lookat=look, up=up, image_w=64, image_h=48, pixel_samples=1, ao_mode=1, ao_samples=8,
+                    ao_max_distance=0.5, ao_light_shadow=int(k == "A"), bounces=1)
+        assert np.array_equal(bits(t.trace_views([view])[0][0]), bits(want[k])), k
