@@ -488,6 +488,12 @@ int Tracer::maxBounces() const {
   return b;
 }
 
+// In core the domains' vertices are numbered scene-wide in 31 bits
+// (DomainDev::vert_base); out of core each domain starts at 0.
+static void checkVertexNumbering(uint64_t vertices) {
+  if (vertices >= (1ull << 31)) throw std::invalid_argument("scene too large for 32-bit vertex numbering");
+}
+
 void Tracer::setScene(const spray_gpu_domain* doms, int nd, const spray_gpu_light* ls, int nl) {
   if (nd <= 0) throw std::invalid_argument("scene needs at least one domain");
   if (nd > 65535) throw std::invalid_argument("at most 65535 domains");
@@ -510,7 +516,15 @@ void Tracer::setScene(const spray_gpu_domain* doms, int nd, const spray_gpu_ligh
   }
   const bool dev_bvh = cfg.bvh_device != 0;
   // every domain resident for certain (with cache_bytes that depends on the trees' sizes)
-  if (dev_bvh && !situ() && cfg.cache_bytes <= 0 && (cfg.cache_size < 0 || cfg.cache_size >= nd)) {
+  const bool resident = !situ() && cfg.cache_bytes <= 0 && (cfg.cache_size < 0 || cfg.cache_size >= nd);
+  if (resident) {
+    uint64_t nv = 0;
+    for (int d = 0; d < nd; ++d) {
+      nv += (uint64_t)std::max<int64_t>(doms[d].num_vertices, 0);
+      checkVertexNumbering(nv);
+    }
+  }
+  if (dev_bvh && resident) {
     setResidentScene(doms, nd);
     finishScene(ls, nl);
     return;
@@ -638,6 +652,7 @@ void Tracer::installScene(std::vector<DomainPack>& packs, const spray_gpu_light*
   else if (cfg.cache_size > 0 && cfg.cache_size < nd) capacity = cfg.cache_size;
   ooc = capacity < nd;
   if (ooc && situ()) throw std::invalid_argument("domain-parallel tracing keeps each rank's domains in core");
+  if (!ooc) checkVertexNumbering(nvv);
   if (ooc) {
     setupOutOfCore(packs, capacity, max_nodes, max_tris, max_verts, slot_bytes);
     packs.clear();

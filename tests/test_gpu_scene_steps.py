@@ -89,3 +89,25 @@ def test_views_that_differ_in_their_shadow_slots_only(lib_built, order, queues):
         view = dict(position=pos, lookat=look, up=up, image_w=64, image_h=48, pixel_samples=1, ao_mode=1, ao_samples=8,
                     ao_max_distance=0.5, ao_light_shadow=int(k == "A"), bounces=1)
         assert np.array_equal(bits(t.trace_views([view])[0][0]), bits(want[k])), k
+
+
+@pytest.mark.parametrize("bvh_device", [0, 1])
+def test_more_vertices_than_the_numbering_holds_are_refused(lib_built, bvh_device):
+    # two domains that claim 2^30 vertices each: refused before any is read
+    class Claims(sg.Scene):
+        def domain_structs(self):
+            doms = super().domain_structs()
+            for d in doms:
+                d.num_vertices = 1 << 30
+            return doms
+
+    tri = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0]], np.float32)
+    doms = [sg.Domain(tri + [2 * k, 0, 0], [[0, 1, 2]]) for k in range(2)]
+    lights = [sg.Light(0, (0, 0, 9))]
+    t = sg.Tracer(small_config(image_w=32, image_h=32, bvh_device=bvh_device))
+    with pytest.raises(sg.SprayError) as e:
+        t.set_scene(Claims(doms, lights))
+    assert e.value.code == sg.EINVAL and "vertex numbering" in str(e.value)
+    t.set_scene(sg.Scene(doms, lights))
+    t.set_camera((0.5, 0.3, 4), (0.5, 0.3, 0), (0, 1, 0))
+    t.trace()
