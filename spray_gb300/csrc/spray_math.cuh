@@ -133,16 +133,18 @@ SPRAY_HD float powShininess(float x, float e) {
 // ---------------------------------------------------------------- float-float
 // GB300 runs FP64 at 1/64 of its FP32 rate, so the two places where the
 // reference multiplies in double precision and rounds to float compute the
-// product (and sum) as a pair of floats t + lo with an error below 2^-47 of t.
-// The double expression differs from the exact value by less than 2^-52 of t:
-// when t + lo moved by 2^-45 of t either way rounds to the same float, that is
-// what the double expression rounds to as well; otherwise (a value that close
-// to a rounding boundary, or near the ends of the exponent range) *ok is false
-// and the caller evaluates the double expression.
-SPRAY_HD float roundPair(float t, float lo, bool* ok) {
-  const float eps = fabsf(t) * 2.8421709430404007e-14f;  // 2^-45
+// product (and sum) as a pair of floats t + lo.  With `size` at least the sum of
+// the terms' magnitudes (|acc| + |product|, which a sum of opposite signs can
+// leave far above |t|), the pair's error and the roundings here are together below
+// 2^-44 of size and the double expression's own below 2^-51: when t + lo moved by
+// 2^-43 of size either way rounds to the same float, that is what the double
+// expression rounds to as well.  Otherwise (a value that close to a rounding
+// boundary, terms that cancel, or the ends of the exponent range) *ok is false and
+// the caller evaluates the double expression.
+SPRAY_HD float roundPair(float t, float lo, float size, bool* ok) {
+  const float eps = size * 1.1368683772161603e-13f;  // 2^-43
   const float a = t + (lo + eps), b = t + (lo - eps);
-  *ok = a == b && fabsf(t) > 1e-30f && fabsf(t) < 1e37f;
+  *ok = a == b && fabsf(t) > 1e-30f && size < 1e37f;
   return a;
 }
 
@@ -151,12 +153,12 @@ SPRAY_HD float addScaled(float acc, float w, double scale, float hi, float lo) {
   const float p = w * hi;
   const float e = fmaf(w, hi, -p);  // exact: w * hi = p + e
   const float t = acc + p;
+  // an exact product: one rounding
+  if (w == 0.0f || (lo == 0.0f && e == 0.0f && fabsf(p) > 1e-30f)) return t;
   const float q = t - acc;
   const float z = (acc - (t - q)) + (p - q);  // exact: acc + p = t + z
-  const float r = e + w * lo;
-  if (r == 0.0f && (fabsf(p) > 1e-30f || w == 0.0f)) return t;  // an exact product: one rounding
   bool ok;
-  const float v = roundPair(t, z + r, &ok);
+  const float v = roundPair(t, z + (e + w * lo), fabsf(acc) + fabsf(p), &ok);
   return ok ? v : (float)((double)acc + scale * (double)w);
 }
 
@@ -165,7 +167,7 @@ SPRAY_HD float timesQuarterPi(float x) {
   const float hi = (float)(kPi / 4.0), lo = (float)(kPi / 4.0 - (double)hi);
   const float p = x * hi;
   bool ok;
-  const float v = roundPair(p, fmaf(x, lo, fmaf(x, hi, -p)), &ok);
+  const float v = roundPair(p, fmaf(x, lo, fmaf(x, hi, -p)), fabsf(p), &ok);
   return ok ? v : (float)((double)x * (kPi / 4.0));
 }
 
