@@ -438,6 +438,9 @@ void buildDomainGroups(const float* boxes, int n, std::vector<BvhNode4>* out, in
     }
     DomCollapse::setSlot((*out)[g / 4], g & 3, glo, ghi, g);
   }
+  // no box turns a ray of no finite origin away, the unused ones' neither: they
+  // name a domain for the exact test to turn down
+  for (int i = n; i < 4 * n2; ++i) (*out)[n1 + i / 4].child[i & 3] = order[n - 1].second;
 }
 
 }  // namespace spray

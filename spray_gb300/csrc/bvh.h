@@ -53,7 +53,7 @@ void buildDomainBvh4(const float* boxes, int n, std::vector<BvhNode4>* out);
 // group-of-16 boxes each, then L2 nodes (index *l1_count + k) four domain boxes
 // each with child = the domain; the group of 16 behind slot c of L1 node q is
 // L2 nodes 4 * (4 * q + c) .. + 3.  Domains are in Morton order of their
-// centres, unused slots are empty boxes.
+// centres, unused slots are empty boxes (of some domain).
 void buildDomainGroups(const float* boxes, int n, std::vector<BvhNode4>* out, int* l1_count);
 
 struct BvhBuildResult {

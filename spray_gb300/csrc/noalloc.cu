@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(kStaticThreads) kStaticLists(StaticScratch* s,
   __syncthreads();
   // slot c of a node: plane p at float 4 * p + c, the domain at int 24 + c; one
   // thread per slot and axis.  An inverted box spans both of its planes, a NaN
-  // bound everything, so that nothing the exact test accepts is left out.
+  // bound everything, so that nothing the exact test accepts is left out; an unused
+  // slot names a domain that exists (a ray of no finite origin meets every slot).
   for (int q = threadIdx.x; q < 12 * (n1 + n2); q += blockDim.x) {
     const int k = q / 3, c = q - 3 * k;
     const bool group = k < 4 * n1;
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(kStaticThreads) kStaticLists(StaticScratch* s,
     float* node = reinterpret_cast<float*>(table + (k >> 2) * kNodeStride);
     node[8 * c + (k & 3)] = lo;
     node[8 * c + 4 + (k & 3)] = hi;
-    if (c == 0) reinterpret_cast<int*>(node)[24 + (k & 3)] = d0;
+    if (c == 0) reinterpret_cast<int*>(node)[24 + (k & 3)] = min(d0, D - 1);
   }
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) s->count = n;
