@@ -25,14 +25,16 @@ constexpr int kStack = 64;
 // [1e-30, 1e18], so that an empty slot (lo = +inf, hi = -inf) is never entered
 // and an axis the ray is parallel to gives finite distances of the right sign
 // (fma(p, inf, -inf) would be a NaN); its planes count as touched within 1e-6
-// of the origin (1e12 / 1e18), as (p - org) * inf = NaN for p = org would.
+// of the origin (1e12 / 1e18), as (p - org) * inf = NaN for p = org would.  A NaN
+// component of the direction passes the comparisons of the exact slab test, so here
+// its axis spans [-1e12, 1e12].
 struct BoxRay {
   V3 inv, cnear, cfar;
   int sx, sy, sz;  // 1 when the direction component is negative
 };
 
 __device__ __forceinline__ float boxPad(float oi, float inv) {
-  return fabsf(oi) * 2.384185791015625e-7f + (fabsf(inv) > 1e18f ? 1e12f : 0.0f);
+  return fabsf(oi) * 2.384185791015625e-7f + (fabsf(inv) <= 1e18f ? 0.0f : 1e12f);
 }
 
 __device__ __forceinline__ void boxAxis(float org, float inv, float& binv, float& cnear, float& cfar) {
