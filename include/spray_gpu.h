@@ -462,7 +462,10 @@ int spray_gpu_schedule_static(const float* domain_bounds, int32_t num_domains, c
  * until its work has finished.  `params` holds spray_mlp_param_count() floats
  * (W1 b1 W2 b2 W3 b3 W4 b4, weights [out][in], W1 64x64 with input columns
  * 54..63 zero, W4 16x64 with rows 8..15 zero); `boxes` 6 floats per domain;
- * `norm` = centre xyz and scale, features are (p - centre) * scale. */
+ * `norm` = centre xyz and scale, features are (p - centre) * scale.
+ * A calling thread keeps its workspace between calls, per device it used: a pinned
+ * word and, once it trained, about 8 MB of device memory.  They are given back when
+ * the thread ends; after cudaDeviceReset the next call allocates them anew. */
 typedef struct spray_mlp_sample {
   float org[3];
   float dir[3];

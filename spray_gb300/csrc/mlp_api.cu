@@ -1,4 +1,6 @@
 // C ABI of the learned proposal's kernels on caller-owned device buffers.
+#include <cuda.h>
+
 #include <algorithm>
 #include <map>
 #include <stdexcept>
@@ -26,13 +28,34 @@ static_assert(sizeof(spray_mlp_sample) == sizeof(ml::Sample), "sample layout");
 // workspace per thread and device is enough.
 constexpr int kCountSteps = 1024;
 
+// The driver's number of the allocation that holds `p`, 0 for none.  Numbers are
+// never given twice in a process, so a changed one tells that the allocation went
+// away (cudaDeviceReset), also when its address is in use again.  30 ns.
+unsigned long long allocationId(const void* p) {
+  using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+  static const Query query = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found) != cudaSuccess)
+      f = nullptr;
+    return reinterpret_cast<Query>(f);
+  }();
+  unsigned long long id = 0;
+  if (!query || query(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return 0;
+  return id;
+}
+
 struct Workspace {
   int device = -1, nsms = 0;
   int* err = nullptr;      // pinned, mapped
   int* err_dev = nullptr;  // the same word as the device addresses it
+  unsigned long long err_id = 0;
   float* partial = nullptr;
   float* grad = nullptr;
   uint32_t* counts = nullptr;
+  // Whether the buffers are still there: a reset of the device takes them all.
+  // (Its context is current.)
+  bool alive() const { return err && allocationId(err) == err_id; }
   void release() {
     if (err) cudaFreeHost(err);
     if (partial) cudaFree(partial);
@@ -46,7 +69,7 @@ struct Workspaces {
   std::map<int, Workspace> of;
   ~Workspaces() {
     for (auto& w : of)
-      if (cudaSetDevice(w.first) == cudaSuccess) w.second.release();
+      if (w.second.err && cudaSetDevice(w.first) == cudaSuccess && w.second.alive()) w.second.release();
   }
 };
 thread_local Workspaces t_workspaces;
@@ -57,10 +80,12 @@ int setup(Workspace** out, int32_t device, bool training) {
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) return fail(SPRAY_GPU_ECUDA, cudaGetErrorString(e));
   Workspace& w = t_workspaces.of[device];
+  if (w.err && !w.alive()) w = Workspace{};
   if (!w.err) {
     e = cudaDeviceGetAttribute(&w.nsms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaHostAlloc(&w.err, sizeof(int), cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(&w.err_dev, w.err, 0);
+    if (e == cudaSuccess && (w.err_id = allocationId(w.err)) == 0) e = cudaErrorNotSupported;
     w.device = device;
   }
   if (e == cudaSuccess && training && !w.counts) {
