@@ -9,8 +9,8 @@
 // instruction, BF16 inputs, FP32 accumulator in tensor memory) and commits to
 // an mbarrier; the four warps read their 32 accumulator lanes back with
 // tcgen05.ld.  Every mbarrier wait is bounded (one second); a wait that gives
-// up sets Net::error; the kernel then runs to its end without waiting again and
-// frees its tensor memory.
+// up sets Net::error; the kernel then runs to its end without waiting for another
+// product, waits once more, as long, for those in flight and frees its tensor memory.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -552,9 +552,11 @@ struct ArenaRows {
 // 89); issue bounds it, 63 %.
 constexpr int kFwdGroups = 5, kFwdThreads = kFwdGroups * kTile;
 // Shared memory: W1 W2 W3 (8 KB each), W4 (2 KB), box records, biases, mbarriers,
-// the tensor-memory address; per group the staged samples.
+// (each group's, and one more that a wait which gave up needs), the tensor-memory
+// address; per group the staged samples.
 constexpr int kFwdW = 0, kFwdBox = 3 * 8192 + 2048, kFwdBias = kFwdBox + kBoxBytes;
-constexpr int kFwdBar = kFwdBias + (3 * kHid + kOutPad) * 4, kFwdSlot = kFwdBar + 8 * kFwdGroups;
+constexpr int kFwdBar = kFwdBias + (3 * kHid + kOutPad) * 4, kFwdDrain = kFwdBar + 8 * kFwdGroups;
+constexpr int kFwdSlot = kFwdDrain + 8 * kFwdGroups;
 constexpr int kFwdStage = (kFwdSlot + 4 + 15) / 16 * 16, kFwdSmem = 116 * 1024;
 static_assert(kFwdStage + kFwdGroups * kStageBytes <= kFwdSmem, "forward shared memory");
 // (more than half of an SM's, so that one CTA has it and its tensor memory alone)
@@ -576,7 +578,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
   uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kFwdSlot);
   uint8_t* stage = sm + kFwdStage + kStageBytes * g;
   BoxCache cache(sm + kFwdBox);
-  const uint32_t mbar = smemAddr(sm + kFwdBar + 8 * g), stage_to = smemAddr(stage);
+  const uint32_t mbar = smemAddr(sm + kFwdBar + 8 * g), drain = smemAddr(sm + kFwdDrain + 8 * g);
+  const uint32_t stage_to = smemAddr(stage);
   const int64_t n = rows.rows();
   // tiles go to the CTAs first, then to their groups
   int64_t tile = blockIdx.x + (int64_t)gridDim.x * g;
@@ -586,7 +589,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
   cache.init(net, threadIdx.x, kFwdThreads);
   weights.store(sm + kFwdW, bias);
   if (threadIdx.x < 32) tmemAlloc(smemAddr(tslot), 512);
-  if (t == 0) mbarInit(mbar, 1);
+  if (t == 0) {
+    mbarInit(mbar, 1);
+    mbarInit(drain, 1);
+  }
   fenceProxyAsync();
   fenceBeforeSync();
   __syncthreads();
@@ -668,7 +674,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kForward(Net net, Rows rows) {
   }
   if (!ok) atomicExch(net.error, 1);
   fenceBeforeSync();
-  __syncthreads();
+  if (__syncthreads_or(!ok)) {
+    // products may still be in flight: their memory is kept until they end, or for
+    // another second
+    if (warp == 0) {
+      commit(drain, t == 0);
+      mbarWait(drain, 0);
+    }
+    __syncthreads();
+  }
   fenceAfterSync();
   if (threadIdx.x < 32) tmemDealloc(*tslot, 512);
 }
@@ -686,10 +700,11 @@ constexpr int kGradThreads = 4 * kTile;           // row threads
 constexpr int kGThreads = kGradThreads + kTile + 4 * 32 + 32;  // feature threads, bias warps, issuing warp
 // Shared memory: W1..W3 (8 KB each), W4 (2 KB); X of this tile and the last, H1, H2,
 // H3, dZ1..dZ3 (128 x 64, 16 KB each), dZ4 (128 x 16), exponentials (128 x 8), box
-// records, (candidates, label) of both X, biases, mbarrier, tensor-memory address.
+// records, (candidates, label) of both X, biases, mbarrier, tensor-memory address, a
+// second mbarrier that a wait which gave up needs.
 constexpr int kGW = 0, kGAct = 3 * 8192 + 2048, kGDz = kGAct + 5 * 16384, kGDz4 = kGDz + 3 * 16384;
 constexpr int kGExp = kGDz4 + 4096, kGBox = kGExp + 4096, kGRow = kGBox + kBoxBytes, kGBias = kGRow + 2 * kTile * 8;
-constexpr int kGBar = kGBias + (3 * kHid + kOutPad) * 4, kGSmem = kGBar + 16;
+constexpr int kGBar = kGBias + (3 * kHid + kOutPad) * 4, kGSmem = kGBar + 32;
 static_assert(kGSmem <= 227 * 1024, "training shared memory");  // one CTA per SM: 512 columns
 // Tensor-memory columns: D0 (64), logits (16), dW1..dW4 (64 each).
 constexpr uint32_t kGCols = 512, kColLogit = 64, kColDw = 128;
@@ -717,7 +732,7 @@ __global__ void __launch_bounds__(kGThreads, 1) kGrad(Net net, const Sample* bat
   uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kGBar + 8);
   int2* row_data = reinterpret_cast<int2*>(sm + kGRow);
   BoxCache cache(sm + kGBox);
-  const uint32_t mbar = smemAddr(sm + kGBar);
+  const uint32_t mbar = smemAddr(sm + kGBar), drain = mbar + 16;
   const int64_t ntiles = (n + kTile - 1) / kTile;
   const bool any = blockIdx.x < ntiles;
   if (labelled_rows) {
@@ -761,7 +776,10 @@ __global__ void __launch_bounds__(kGThreads, 1) kGrad(Net net, const Sample* bat
   // columns 8..15 of dZ4 stay zero
   if (quarter == 0) *reinterpret_cast<uint4*>(sm + kGDz4 + opOff(t, 8, 2)) = make_uint4(0u, 0u, 0u, 0u);
   if (warp == 0) tmemAlloc(smemAddr(tslot), kGCols);
-  if (threadIdx.x == 0) mbarInit(mbar, 1);
+  if (threadIdx.x == 0) {
+    mbarInit(mbar, 1);
+    mbarInit(drain, 1);
+  }
   fenceProxyAsync();
   fenceBeforeSync();
   __syncthreads();
@@ -856,11 +874,14 @@ __global__ void __launch_bounds__(kGThreads, 1) kGrad(Net net, const Sample* bat
     uint32_t phase = 0;
     uint8_t* x = sm + kGAct;
     auto h = [&](int l) { return l == 0 ? x : sm + kGAct + 16384 * (l + 1); };
-    // an operand is written: its product may be issued
+    // an operand is written: its product may be issued.  The rows meet the issuing
+    // warp here (their wait for the product would, too): an arrival alone could be
+    // repeated before the issuing warp has taken the last one, once a wait for a
+    // product gave up, and the barrier would be out of step for good.
     auto ready = [&]() {
       fenceProxyAsync();
       fenceBeforeSync();
-      barArrive(kBarOp, kBarCount);
+      barSync(kBarOp, kBarCount);
     };
     auto product = [&]() {
       ok = ok && mbarWait(mbar, phase);
@@ -918,8 +939,8 @@ __global__ void __launch_bounds__(kGThreads, 1) kGrad(Net net, const Sample* bat
           mine[k] = label >= 0 && c < ncand ? p : 0.0f;
         }
         *reinterpret_cast<uint32_t*>(sm + kGDz4 + opOff(t, 2 * quarter, 2)) = packBf16(mine[0], mine[1]);
-        ready();
         barArrive(kBarDz + 3, kBarCount);
+        ready();
         if (quarter == 0 && label >= 0) {
           loss += logf(s) - (zl - m);
           labelled += 1.0f;
@@ -944,8 +965,8 @@ __global__ void __launch_bounds__(kGThreads, 1) kGrad(Net net, const Sample* bat
           *reinterpret_cast<uint4*>(sm + kGDz + 16384 * (l - 1) + opOff(t, c0 + 8 * c, 8)) =
               make_uint4(p.x & a[c].x, p.y & a[c].y, p.z & a[c].z, p.w & a[c].w);
         }
-        ready();
         barArrive(kBarDz + l - 1, kBarCount);
+        ready();
       }
       x = x == sm + kGAct ? sm + kGAct + 16384 : sm + kGAct;
     }
@@ -985,7 +1006,13 @@ __global__ void __launch_bounds__(kGThreads, 1) kGrad(Net net, const Sample* bat
   // loss and labelled rows: block sums in a fixed order
   float* red = reinterpret_cast<float*>(sm + kGExp);
   fenceBeforeSync();
-  __syncthreads();
+  if (__syncthreads_or(!ok)) {  // as in kForward
+    if (!rows && !feature_warp && !bias_warp) {
+      commit(drain, lane == 0);
+      mbarWait(drain, 0);
+    }
+    __syncthreads();
+  }
   fenceAfterSync();
   if (quarter == 0) {
     red[t] = loss;
