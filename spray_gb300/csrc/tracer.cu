@@ -1176,9 +1176,16 @@ void Tracer::ensureBuffers(int64_t nsamples) {
       throw std::runtime_error("too few scheduling chunks for 16-bit histogram counters");
   }
   if (nsamples <= cap_samples && S <= cap_slots && queues == !d_walk_work && cap_entries >= needed_entries &&
-      (!side || d_side_ref || side_refused) && frame_pixels <= image_cap && (int64_t)tiles.size() <= tiles_cap && fviews.size() <= views_cap &&
-      walkLaunches() <= walk_work_cap)
+      frame_pixels <= image_cap && (int64_t)tiles.size() <= tiles_cap && fviews.size() <= views_cap &&
+      walkLaunches() <= walk_work_cap) {
+    // the side lists alone may be missing: given back before a scene was loaded, or
+    // not needed by the frames before
+    if (side && !d_side_ref && !side_refused) {
+      ensureSide();
+      ++buf_gen;
+    }
     return;
+  }
   freeBuffers();
   ++buf_gen;
   int64_t N = std::max<int64_t>(nsamples, 1024);
@@ -1258,21 +1265,26 @@ void Tracer::ensureBuffers(int64_t nsamples) {
   devAlloc(&d_order, D);
   devAlloc(&d_tiles, tiles.size() + 1);
   tiles_cap = (int64_t)tiles.size();
-  if (side) {
-    // last, and from at most a quarter of the memory left: a frame can do without
-    size_t left = 0, total = 0;
-    CK(cudaMemGetInfo(&left, &total));
-    side_bytes = E * sizeof(uint2) + (size_t)NS * sizeof(uint2);
-    side_refused = side_bytes > left / 4 || cudaMalloc((void**)&d_side_arena, E * sizeof(uint2)) != cudaSuccess ||
-                   cudaMalloc((void**)&d_side_ref, NS * sizeof(uint2)) != cudaSuccess;
-    if (side_refused) {
-      cudaGetLastError();
-      freeSide();
-    }
-  }
   cap_samples = N;
   cap_slots = S;
   cap_entries = E;
+  if (side) ensureSide();
+}
+
+// The second lists of a frame whose occlusion runs beside the next closest hits, as
+// large as the first: last, and from at most a quarter of the memory left, for a
+// frame can do without.
+void Tracer::ensureSide() {
+  const size_t arena = cap_entries * sizeof(uint2), refs = (size_t)cap_samples * cap_slots * sizeof(uint2);
+  size_t left = 0, total = 0;
+  CK(cudaMemGetInfo(&left, &total));
+  side_bytes = arena + refs;
+  side_refused = side_bytes > left / 4 || cudaMalloc((void**)&d_side_arena, arena) != cudaSuccess ||
+                 cudaMalloc((void**)&d_side_ref, refs) != cudaSuccess;
+  if (side_refused) {
+    cudaGetLastError();
+    freeSide();
+  }
 }
 
 void Tracer::schedule(bool shadow, int order_by_depth, uint32_t* count, uint32_t* list, int S,

@@ -440,6 +440,7 @@ class Tracer {
   uint2* d_side_ref = nullptr;
   size_t side_bytes = 0;
   bool side_refused = false;  // there was no memory for them
+  void ensureSide();
   void freeSide();
   size_t walk_work_cap = 0, walk_launch = 0;
   size_t walkLaunches() const { return walksRays() ? waves.size() * (size_t)maxBounces() * 2 : 0; }
