@@ -717,7 +717,7 @@ void Tracer::setResidentScene(const spray_gpu_domain* doms, int nd) {
   devAlloc(&d_normals, 3 * nv);
   devAlloc(&d_tris, 3 * nt);
   DeviceBuffer<float> verts(3 * nv);
-  // groups of domains of at most kUploadBytes (at least one domain)
+  // groups of domains of at most kUploadBytes, or one larger domain
   auto bytesOf = [&](int d) { return (size_t)doms[d].num_vertices * 28 + (size_t)doms[d].num_faces * 12; };
   for (int g0 = 0, g1 = 0; g0 < nd; g0 = g1) {
     size_t bytes = 0, gv = 0, gf = 0;
@@ -726,6 +726,21 @@ void Tracer::setResidentScene(const spray_gpu_domain* doms, int nd) {
       gv += (size_t)doms[g1].num_vertices;
       gf += (size_t)doms[g1].num_faces;
       ++g1;
+    }
+    if (bytes > kUploadBytes) {
+      // one large domain: from the caller's arrays, so that the pinned buffer stays small
+      const spray_gpu_domain& s = doms[g0];
+      checkMesh(s, g0);
+      std::vector<float> normals(3 * gv);
+      computeVertexNormals(s.vertices, s.num_vertices, s.faces, s.num_faces, normals.data());
+      const size_t v0 = (size_t)hdoms[g0].vert_base, f0 = (size_t)hdoms[g0].face_base;
+      CK(cudaMemcpyAsync(verts.p + 3 * v0, s.vertices, 12 * gv, cudaMemcpyHostToDevice, stream));
+      CK(cudaMemcpyAsync(d_faces + 3 * f0, s.faces, 12 * gf, cudaMemcpyHostToDevice, stream));
+      if (s.colors) CK(cudaMemcpyAsync(d_colors + v0, s.colors, 4 * gv, cudaMemcpyHostToDevice, stream));
+      else CK(cudaMemsetAsync(d_colors + v0, 0, 4 * gv, stream));
+      CK(cudaMemcpyAsync(d_normals + 3 * v0, normals.data(), 12 * gv, cudaMemcpyHostToDevice, stream));
+      CK(cudaStreamSynchronize(stream));
+      continue;
     }
     if (g0 > 0) CK(cudaStreamSynchronize(stream));  // the previous group's copies
     if (bytes > h_upload_cap) {
