@@ -56,13 +56,14 @@ NODE_BYTES, TRI_BYTES, ENTRY_BYTES, RAY_BYTES, HIT_BYTES = 128, 48, 8, 32, 24
 WALK_NODE_BYTES = 64  # half-precision nodes of the in-core whole-ray walks
 
 
-def node_bytes(cfg: dict, num_domains: int) -> int:
-    """Bytes of a node as the frame's traversal reads it: whole-ray walks in core,
-    the queue kernels otherwise (out of core, learned order, round loop, captures)."""
-    size = cfg.get("cache_size", -1)
-    in_core = not cfg.get("cache_bytes") and (size <= 0 or size >= num_domains)
+def node_bytes(cfg: dict, st: dict) -> int:
+    """Bytes of a node as the frame's traversal reads it: whole-ray walks in core (the
+    frame reports no cache slots; whether cache_bytes holds a scene depends on its
+    trees), the queue kernels otherwise (out of core, learned order, round loop,
+    captures)."""
     queues = cfg.get("debug_capture") or cfg.get("schedule_policy", 0) in (3, 5) or not cfg.get("cull", 1)
-    return WALK_NODE_BYTES if in_core and not queues and cfg.get("bucket_launches", 0) != 4 else NODE_BYTES
+    walks = st["cache_slots"] == 0 and not queues and cfg.get("bucket_launches", 0) != 4
+    return WALK_NODE_BYTES if walks else NODE_BYTES
 
 
 def describe(name: str, spec: dict, cfg: dict) -> str:
@@ -282,7 +283,7 @@ def accuracy_report(scene, cfg, cam, mode_a_img, oracle_obj, device: int) -> dic
     rep = A.frame_report(img, mode_a_img, mode_b, hits, shadows)
     rep["frame"] = [c["image_w"], c["image_h"]]
     rep["captured_frame_equals_plain_frame"] = bool(np.array_equal(plain.view(np.uint32), img.view(np.uint32)))
-    nb = node_bytes(cfg, len(scene.domains))
+    nb = node_bytes(cfg, st)
     gpu_bytes = (st["visits_radiance"] * (RAY_BYTES + ENTRY_BYTES + HIT_BYTES)
                  + st["nodes_radiance"] * nb + st["tris_radiance"] * TRI_BYTES)
     orc_bytes = (ost["bvh4_visits"] * (RAY_BYTES + ENTRY_BYTES + HIT_BYTES)
@@ -616,7 +617,7 @@ def main():
 
     s0 = stats[-1]
     peak, peak_kind = hbm_peak()
-    nb = node_bytes(cfg, len(scene.domains))
+    nb = node_bytes(cfg, s0)
     trace_bytes = (s0["visits_radiance"] * (RAY_BYTES + ENTRY_BYTES + HIT_BYTES)
                    + s0["nodes_radiance"] * nb + s0["tris_radiance"] * TRI_BYTES)
     occl_bytes = (s0["visits_shadow"] * (RAY_BYTES + ENTRY_BYTES)

@@ -84,3 +84,15 @@ def test_reference_arm_runs_without_the_cuda_library(tmp_path):
     assert d["impl"] == "reference" and d["value"] > 0 and d["cpu_baseline"]["kind"] == "port"
     mapped = next(l for l in r.stdout.splitlines() if l.startswith("MAPPED"))
     assert "libspray_gpu.so" not in mapped and "liboracle.so" in mapped
+
+
+@pytest.mark.parametrize("cfg,slots,want", [
+    ({}, 0, 64),
+    ({"cache_bytes": 1 << 34}, 0, 64),    # a cache that holds the whole scene: in core
+    ({"cache_bytes": 1 << 20}, 3, 128),
+    ({"cache_size": 8, "schedule_policy": 2}, 8, 128),
+    ({"schedule_policy": 3}, 0, 128), ({"schedule_policy": 5}, 0, 128), ({"cull": 0}, 0, 128),
+    ({"debug_capture": 1}, 0, 128), ({"bucket_launches": 4}, 0, 128),
+])
+def test_node_bytes_follow_what_the_frame_reports(bench, cfg, slots, want):
+    assert bench.node_bytes(cfg, {"cache_slots": slots}) == want
