@@ -644,7 +644,7 @@ __global__ void kWalkNodes(const BvhNode4* __restrict__ nodes, uint32_t num_node
     const float centre = wd.centre[x], scale = 1.0f / wd.half[x];
     for (int q = 0; q < 4; ++q) {
       c[q] = __ushort_as_half(0);
-      e[q] = __ushort_as_half(0xfc00);  // -inf: an unused slot is never entered
+      e[q] = __ushort_as_half(0xfc00);  // -inf: an unused slot is not entered
       if (nd.child[q] == kEmptyChild) continue;
       const float a = (l[q] - centre) * scale, b = (h[q] - centre) * scale;
       const __half m = __float2half_rn(0.5f * a + 0.5f * b);
@@ -665,10 +665,11 @@ __global__ void kWalkNodes(const BvhNode4* __restrict__ nodes, uint32_t num_node
     // triangles: the walks rely on it and check nothing
     const bool ok = c == kEmptyChild || (c >= 0 ? (uint32_t)c > k - (uint32_t)wd.root && c < domains[lo].num_nodes
                                                 : (leaf >> 3) + (leaf & 7u) < (uint32_t)domains[lo].num_tris);
-    if (!ok) {
-      *bad = 1;
-      w.child[q] = kEmptyChild;
-    } else if (c == kEmptyChild) w.child[q] = kEmptyChild;
+    if (!ok) *bad = 1;
+    // an unused slot holds the domain's first triangle: a ray whose distances in the
+    // domain overflow along every axis (extents near the largest float) enters all
+    // four slots, and one more test of a triangle changes nothing
+    if (!ok || c == kEmptyChild) w.child[q] = (int)~(tri_base << 3);
     else if (c >= 0) w.child[q] = c + wd.root;
     else w.child[q] = (int)~(leaf + (tri_base << 3));
   }
