@@ -65,3 +65,65 @@ def test_several_upload_groups(lib_built):
     # 40 MB, 126 MB and small domains: groups of their own and a large one between them
     _images(_scene(_sheet(900, (0, 0, 0)), _sheet(900, (1, 0, 0)), _sheet(1550, (2, 0, 0)), _sheet(50, (3, 0, 0)),
                    _sheet(30, (0, 1, 0))))
+
+
+def test_several_build_batches(lib_built):
+    # 17 million triangles: two batches, their nodes joined; out of core every domain
+    # keeps its own
+    sc = _scene(_sheet(2062, (0, 0, 0)), _sheet(2062, (1, 0, 0)), _sheet(30, (0, 1, 0)))
+    cfg = small_config(image_w=96, image_h=72, ao_mode=0, ao_samples=2, pixel_samples=2, bounces=2)
+    out = []
+    for cache in (-1, 1):
+        t = sg.Tracer(dict(cfg, cache_size=cache))
+        t.set_scene(sc)
+        t.set_camera(*scenes.orbit_camera(sc))
+        out.append(t.trace()[0])
+        t.close()
+    assert out[0][..., :3].max() > 0
+    assert np.array_equal(bits(out[0]), bits(out[1]))
+
+
+def _check_tree(nodes, tris, faces):
+    """Every triangle in one leaf, inside its box and all boxes above it."""
+    assert np.array_equal(np.sort(tris["v"][:, 0, 3].view(np.uint32)), np.arange(faces))
+    v = tris["v"][:, :, :3]
+    lo, hi = v.min(1), v.max(1)
+    seen = np.zeros(faces, int)
+
+    def walk(k):
+        n = nodes[k]
+        low, high = np.full(3, np.inf), np.full(3, -np.inf)
+        for c in range(4):
+            child = int(n["child"][c])
+            if child == -2 ** 31:
+                continue
+            blo, bhi = n["box"][0::2, c], n["box"][1::2, c]
+            if child >= 0:
+                l, h = walk(child)
+            else:
+                first, count = (~child) >> 3, ((~child) & 7) + 1
+                seen[first:first + count] += 1
+                l, h = lo[first:first + count].min(0), hi[first:first + count].max(0)
+            assert np.all(blo <= l) and np.all(h <= bhi)
+            low, high = np.minimum(low, blo), np.maximum(high, bhi)
+        return low, high
+
+    walk(0)
+    assert np.all(seen == 1)
+
+
+@pytest.mark.parametrize("octaves,tail", [(3, 126), (20, 160), (36, 150), (42, 150)])
+def test_more_split_levels_than_a_group(lib_built, octaves, tail):
+    # a point per octave down to `tail` at one place: every split of a task above 128
+    # triangles takes the largest off, 2, 20, 36 and 42 levels (the first group launches
+    # 4, then 8 at a time up to 32, then another group)
+    s = 2.0 ** -np.minimum(np.arange(octaves + tail), octaves)
+    v = np.zeros((octaves + tail, 3, 3), np.float32)
+    v[:, :, 0] = s[:, None]
+    lopsided = sg.Domain(v.reshape(-1, 3), np.arange(3 * len(v)).reshape(-1, 3))
+    sc = _scene(lopsided, _sheet(20, (0.0, -1.0, -0.5)))
+    _images(sc)
+    t = sg.Tracer(small_config(image_w=32, image_h=32))
+    t.set_scene(sc)
+    for d, dom in enumerate(sc.domains):
+        _check_tree(t.debug(sg.DBG_NODES, d), t.debug(sg.DBG_TRIS, d), len(dom.faces))
