@@ -433,9 +433,10 @@ void launchTraceClosest(cudaStream_t s, const TraceArgs& a, int nblocks);
 void launchResolve(cudaStream_t s, const TraceArgs& a, float4* hit_ns, int nblocks, bool interpolate);
 void launchTraceOccluded(cudaStream_t s, const TraceArgs& a, int nblocks);
 // Sets *bad when a node references a child outside its domain's nodes (or before
-// itself) or triangles.
+// itself) or triangles, *loose when the relative boxes would have the walks visit too
+// many nodes.  Both are cleared by the caller.
 void launchWalkNodes(cudaStream_t s, const BvhNode4* nodes, uint32_t num_nodes, const DomainDev* domains, int D,
-                     WalkDomain* wdomains, WalkNode* out, int* bad);
+                     WalkDomain* wdomains, WalkNode* out, int* bad, int* loose);
 void launchListDomains(cudaStream_t s, const RayWalkArgs& a, int nblocks);
 void launchWalkClosest(cudaStream_t s, const RayWalkArgs& a, int nblocks);
 void launchWalkOccluded(cudaStream_t s, const RayWalkArgs& a, int nblocks);

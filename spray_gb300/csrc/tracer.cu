@@ -352,6 +352,7 @@ Tracer::~Tracer() {
 
 void Tracer::freeScene() {
   has_scene = false;  // until the next one is complete
+  loose_boxes = false;
   ++buf_gen;          // a captured frame holds this scene's addresses
   freeProposal();
   if (side_bytes > kSideKept) freeSide();  // room for the next scene
@@ -842,19 +843,24 @@ void Tracer::finishScene(const spray_gpu_light* ls, int nl) {
       q[10 + c] = ls[l].edge2[c];
     }
   }
-  int b = 0;
+  int flags[2] = {0, 0};  // a bad hierarchy, loose boxes
   if (walksRays()) {
     devAlloc(&d_wnodes, nn);
     devAlloc(&d_wdomains, nd);
-    int* bad = reinterpret_cast<int*>(d_ctr);  // a word that every frame clears
-    CK(cudaMemsetAsync(bad, 0, sizeof(int), stream));
-    launchWalkNodes(stream, d_nodes, (uint32_t)nn, d_domains, nd, d_wdomains, d_wnodes, bad);
-    CK(cudaMemcpyAsync(&b, bad, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    int* f = reinterpret_cast<int*>(d_ctr);  // words that every frame clears
+    CK(cudaMemsetAsync(f, 0, sizeof(flags), stream));
+    launchWalkNodes(stream, d_nodes, (uint32_t)nn, d_domains, nd, d_wdomains, d_wnodes, f, f + 1);
+    CK(cudaMemcpyAsync(flags, f, sizeof(flags), cudaMemcpyDeviceToHost, stream));
   }
   devAlloc(&d_lights, lf.size());
   CK(cudaMemcpyAsync(d_lights, lf.data(), lf.size() * 4, cudaMemcpyHostToDevice, stream));
   CK(cudaStreamSynchronize(stream));
-  bad_hierarchy = b != 0;
+  bad_hierarchy = flags[0] != 0;
+  loose_boxes = flags[1] != 0;
+  if (loose_boxes) {
+    devFree(d_wnodes);
+    devFree(d_wdomains);
+  }
   if (situ()) devAlloc(&d_segs, 2 * (size_t)D + 2);  // one segment table over the owned domains
   // the queues' sizes depend on the domain count; the walks' buffers stay (a
   // simulation's next time step), their slots are checked when a frame starts

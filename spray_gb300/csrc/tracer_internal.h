@@ -210,11 +210,12 @@ class Tracer {
   bool rounded() const { return cfg.schedule_policy == 5; }
   // In core, frames that need no per-domain queues walk whole rays
   // (walk_rays.cu): the queues stay for the captured stage buffers, the pairs
-  // the proposal learns from, domain-parallel ranks, uncut visits (cull 0) and
-  // the per-bucket launches with their own visit counts.
+  // the proposal learns from, domain-parallel ranks, uncut visits (cull 0), the
+  // per-bucket launches with their own visit counts, and scenes whose boxes the
+  // walks' nodes hold too loosely (kWalkNodes).
   bool walksRays() const {
     return !ooc && !situ() && !learned() && !rounded() && cfg.cull && !cfg.debug_capture &&
-           cfg.bucket_launches != kDepthBuckets && total_tris < kMaxWalkTris;
+           cfg.bucket_launches != kDepthBuckets && total_tris < kMaxWalkTris && !loose_boxes;
   }
   RayWalkArgs walkArgs(bool shadow, bool primary, int S, bool side);
   void setupProposal();
@@ -304,6 +305,7 @@ class Tracer {
   DomainDev* d_domains = nullptr;
   BvhNode4* d_nodes = nullptr;
   bool bad_hierarchy = false;    // a node's child lies outside its domain
+  bool loose_boxes = false;      // the scene's nodes are too fine for the walks'
   WalkDomain* d_wdomains = nullptr;
   WalkNode* d_wnodes = nullptr;  // d_nodes as the whole-ray walks read them
   float4* d_tris = nullptr;
