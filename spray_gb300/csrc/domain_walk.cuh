@@ -128,7 +128,7 @@ __device__ __forceinline__ uint32_t boxMask(const float4* p, const BoxRay& r, fl
 // within (1e-3, t1], 64 at a time: every group of 16 is tested, the four nodes
 // of a group some lane may enter are tested by all of the warp's lanes that
 // may, at the same addresses, and then each lane goes through its own bits.
-// Against the descent of a hierarchy (domain_walk.cuh) that is more tests and
+// Against the descent of a hierarchy (descendDomains) that is more tests and
 // far fewer instructions, for the lanes of a warp stay together.
 template <class F>
 __device__ __forceinline__ void groupDomains(const float4* table, int n1, int n2, const BoxRay& r, float t1,

@@ -2,7 +2,8 @@
 //
 // One frame is traced as a sequence of wavefronts ("waves").  A wave holds
 // whole blocking tiles (src/render/tile.cc:317-391), so every sample keeps the
-// tile-local id SpRay seeds its random streams with.  Per bounce a wave runs:
+// tile-local id SpRay seeds its random streams with.  Per bounce a wave runs
+// through per-domain queues (out of core, and in core where Tracer::walksRays says):
 //   schedule  : slab test of every live ray against every domain AABB, sorted
 //               (t, id) domain list, stable partition of the (ray, domain)
 //               entries into per-domain queues        (ooc_isector.h:116-174)
@@ -13,6 +14,9 @@
 //                                                     (ooc_shader_ao.h, ooc_shader_pt.h)
 //   schedule + occlusion of the shadow rays, then retire into the image
 //                                                     (ooc_tcontext.inl:123-135)
+// In core most frames have no queues: a list pass writes every ray's sorted domains,
+// then each ray walks its own (walk_rays.cu), closest hits with their colours and
+// normals, shading, occlusion, retire.
 // Counts live in device memory so a bounce needs no host round trip.
 #pragma once
 
@@ -447,13 +451,6 @@ void launchShade(cudaStream_t s, const ShadeArgs& a, int nblocks);
 void launchCompact(cudaStream_t s, const uint8_t* flag, const uint32_t* n_dev, uint32_t n_mul,
                    uint64_t n_host, uint32_t* list, uint32_t* count, int32_t* index_of,
                    uint32_t* block_tmp, int nblocks);
-// Adds the unoccluded shadow rays of every pixel of a wave (npix pixels over
-// ntiles tiles) to the frame image, samples of a pixel in order.
-// Stable compaction of a list: keeps src[i] (i < *n_dev) where flag[src[i]] is
-// set, in order, into list and count; index_of[src[i]] = new position or -1.
-// list must not alias src.
-void launchCompactList(cudaStream_t s, const uint32_t* src, const uint32_t* n_dev, const uint8_t* flag,
-                       uint32_t* list, uint32_t* count, int32_t* index_of, uint32_t* block_tmp, int nblocks);
 // The write pass of a compaction.
 struct CompactArgs {
   const uint8_t* flag;
@@ -464,10 +461,10 @@ struct CompactArgs {
   uint32_t* list;
   uint32_t* count;         // set: block_tmp holds kept counts, *count is written
   int32_t* index_of;       // optional
-  const uint32_t* src;     // element k is src[k] (null: k)
+  const uint32_t* src;     // element k is src[k] (null: k); list must not alias it
   unsigned long long* dropped;  // optional, with count: += elements not kept
 };
-// The write pass of launchCompact / launchCompactList when block_tmp already
+// The write pass of launchCompact when block_tmp already
 // holds each block's kept count (kShade's block counts): each block adds the
 // counts before its own, the last writes *count.  One launch, also for two.
 void launchCompactCounted(cudaStream_t s, const CompactArgs& a, int nblocks);

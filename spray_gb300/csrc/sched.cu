@@ -706,14 +706,13 @@ void launchSchedScatter(cudaStream_t s, const SchedArgs& a, int D, int nwarps) {
 
 // ---------------------------------------------------------------- compaction
 __global__ void kCompactCount(const uint8_t* __restrict__ flag, const uint32_t* n_dev,
-                              uint32_t n_mul, uint64_t n_host, uint32_t* block_tmp,
-                              const uint32_t* __restrict__ src) {
+                              uint32_t n_mul, uint64_t n_host, uint32_t* block_tmp) {
   __shared__ uint32_t ws[32];
   const uint64_t n = n_dev ? (uint64_t)(*n_dev) * n_mul : n_host;
   const uint64_t per = compactPer(n_dev ? *n_dev : n_host, n_dev ? n_mul : 1u, gridDim.x);
   const uint64_t b0 = min(n, per * blockIdx.x), b1 = min(n, b0 + per);
   uint32_t c = 0;
-  for (uint64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) c += flag[src ? src[i] : i] != 0;
+  for (uint64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) c += flag[i] != 0;
   for (int o = 16; o; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
   __syncthreads();
@@ -833,7 +832,7 @@ __global__ void __launch_bounds__(kCompactThreads) kCompactPair(CompactArgs a, C
 void launchCompact(cudaStream_t s, const uint8_t* flag, const uint32_t* n_dev, uint32_t n_mul,
                    uint64_t n_host, uint32_t* list, uint32_t* count, int32_t* index_of,
                    uint32_t* block_tmp, int nblocks) {
-  kCompactCount<<<nblocks, 256, 0, s>>>(flag, n_dev, n_mul, n_host, block_tmp, nullptr);
+  kCompactCount<<<nblocks, 256, 0, s>>>(flag, n_dev, n_mul, n_host, block_tmp);
   kCompactScan<<<1, 1024, 0, s>>>(block_tmp, nblocks, count);
   kCompactWrite<<<nblocks, kCompactThreads, 0, s>>>(
       CompactArgs{flag, n_dev, n_mul, n_host, block_tmp, list, nullptr, index_of, nullptr, nullptr});
@@ -845,14 +844,6 @@ void launchCompactCounted(cudaStream_t s, const CompactArgs& a, int nblocks) {
 
 void launchCompactPair(cudaStream_t s, const CompactArgs& a, const CompactArgs& b, int nblocks) {
   kCompactPair<<<dim3(nblocks, 2), kCompactThreads, 0, s>>>(a, b);
-}
-
-void launchCompactList(cudaStream_t s, const uint32_t* src, const uint32_t* n_dev, const uint8_t* flag,
-                       uint32_t* list, uint32_t* count, int32_t* index_of, uint32_t* block_tmp, int nblocks) {
-  kCompactCount<<<nblocks, 256, 0, s>>>(flag, n_dev, 1, 0, block_tmp, src);
-  kCompactScan<<<1, 1024, 0, s>>>(block_tmp, nblocks, count);
-  kCompactWrite<<<nblocks, kCompactThreads, 0, s>>>(
-      CompactArgs{flag, n_dev, 1, 0, block_tmp, list, nullptr, index_of, src, nullptr});
 }
 
 // ---------------------------------------------------------------- scores

@@ -18,9 +18,6 @@
 #ifndef SPRAY_TRACE_MIN_BLOCKS
 #define SPRAY_TRACE_MIN_BLOCKS 4
 #endif
-#ifndef SPRAY_TRACE_REFILL
-#define SPRAY_TRACE_REFILL 20
-#endif
 
 namespace spray {
 
@@ -69,8 +66,10 @@ __device__ __forceinline__ uint32_t lanesBelow() {
   return m;
 }
 
-// Idle lanes a warp gathers before it takes new entries for them.
-constexpr int kTraceRefill = SPRAY_TRACE_REFILL;
+// Idle lanes a warp gathers before it takes new entries for them (2048x2048, 8 spp,
+// 216 domains out of core, batched, at 12, 16, 20 and 24: 34.7, 34.5, 34.3 and 34.2 ms
+// a frame; 1600x900, 4 spp, learned order: 7.84, 7.76, 7.74 and 7.75).
+constexpr int kTraceRefill = 20;
 
 // Work indices for the idle lanes of a warp, one atomic; E or more once the
 // queue has run out, and *exhausted is set.
@@ -327,15 +326,15 @@ void launchResolve(cudaStream_t s, const TraceArgs& a, float4* hit_ns, int nbloc
   else kResolve<false><<<nblocks, 256, 0, s>>>(a, hit_ns);
 }
 
-// Occlusion, in rounds as in the whole-ray walks (walk_rays.cu): the lanes of a
-// warp walk independently, each at an inner node, at a triangle, or idle, and
-// every round runs the step most lanes are at; once kTraceRefill lanes are idle
-// the warp takes the next queue entries for them and drops those whose ray is
-// already occluded.  Against warps that queued 32 live entries and walked them
+// Occlusion, in rounds: the lanes of a warp walk independently, each at an inner
+// node, at a triangle, or idle, and every round runs the step most lanes are at
+// (the whole-ray walks, walk_rays.cu, go through the steps in turn); once kTraceRefill
+// lanes are idle the warp takes the next queue entries for them and drops those whose
+// ray is already occluded.  Against warps that queued 32 live entries and walked them
 // together, out of core (2048x2048, 8 spp, 4 bounces, 216 domains, batched):
-// 4.95 -> 4.60 ms a frame (12 and 16 idle lanes: 5.01 and 4.75).  The closest-hit
-// kernel above keeps its 32 entries together: the entries of one domain's queue
-// are coherent and rounds took 20.2 instead of 19.3 ms there.
+// 4.95 -> 4.60 ms a frame.  The closest-hit kernel above keeps its 32 entries together:
+// the entries of one domain's queue are coherent and rounds took 20.2 instead of
+// 19.3 ms there.
 template <bool kOoc>
 __global__ void __launch_bounds__(256, SPRAY_TRACE_MIN_BLOCKS) kTraceOccluded(TraceArgs a) {
   extern __shared__ uint32_t skeys[];

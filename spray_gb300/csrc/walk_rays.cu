@@ -21,39 +21,24 @@
 #include "spray_math.cuh"
 #include "traverse.cuh"
 
-#ifndef SPRAY_WALK_REFILL
-#define SPRAY_WALK_REFILL 20
-#endif
-
-#ifndef SPRAY_WALK_STAY
-#define SPRAY_WALK_STAY 7
-#endif
-#ifndef SPRAY_WALK_SWITCH
-#define SPRAY_WALK_SWITCH 2
-#endif
-#ifndef SPRAY_WALK_SHADOW_SWITCH
-#define SPRAY_WALK_SHADOW_SWITCH 4
-#endif
-#ifndef SPRAY_WALK_LEAVES
-#define SPRAY_WALK_LEAVES 5
-#endif
-
 namespace spray {
 
 namespace {
 
 constexpr int kWalkThreads = 256;
-// Idle lanes a warp gathers before it fetches new rays for them (closest hits
-// of that frame at 12, 16, 20 and 24: 4.13, 4.05, 4.00 and 4.17 ms).
-constexpr int kRefill = SPRAY_WALK_REFILL;
-// Lanes at the end of a domain that the warp gathers before it moves them on
-// (closest hits at 2, 3, 4 and 6: 6.62, 6.64, 6.72 and 6.75 ms a frame).
-constexpr int kSwitch = SPRAY_WALK_SWITCH, kShadowSwitch = SPRAY_WALK_SHADOW_SWITCH;
-// Lanes at inner nodes with which a warp takes another node, lanes at triangles
-// with which it takes another triangle (24 views, before the two followed each
-// other in a round: 8, 12 and 16 at nodes 115.1, 115.9 and 116.6 ms; 1, 4, 5, 8, 16
-// and no run at triangles 113.1, 112.2, 112.3, 113.3, 114.4 and 113.8 ms).
-constexpr int kStay = SPRAY_WALK_STAY, kLeaves = SPRAY_WALK_LEAVES;
+// The rounds' thresholds, in lanes of 32.  Each was varied by itself; the figures are
+// frames of 24 views of up to 2048x2048, 16 spp, ambient occlusion and path tracing.
+// Idle lanes a warp gathers before it fetches new rays for them (12, 16, 20 and 24:
+// 113.0, 110.4, 109.1 and 110.2 ms).
+constexpr int kRefill = 20;
+// Lanes at the end of a domain that the warp gathers before it moves them on: closest
+// hits (1, 2 and 4: 109.7, 109.1 and 109.8 ms) and occlusion (2, 4, 6 and 8: 108.9,
+// 109.1, 109.6 and 110.5 ms).
+constexpr int kSwitch = 2, kShadowSwitch = 4;
+// Lanes at inner nodes with which a warp takes another node (3, 5, 7, 9 and 12: 111.4,
+// 109.5, 109.1, 109.6 and 111.1 ms), lanes at triangles with which it takes another
+// triangle (1, 3, 5, 8 and 12: 111.5, 109.4, 109.1, 109.9 and 111.2 ms).
+constexpr int kStay = 7, kLeaves = 5;
 
 __device__ __forceinline__ uint32_t lanesBelowMask() {
   uint32_t m;
