@@ -1211,7 +1211,9 @@ void Tracer::ensureBuffers(int64_t nsamples) {
   ++buf_gen;
   int64_t N = std::max<int64_t>(nsamples, 1024);
   int64_t NS = N * S;
-  if (needed_entries == 0) needed_entries = (uint64_t)std::max<int64_t>(4 * N, 2 * NS);
+  // at least what a frame of this size starts with: an earlier frame may have been tiny,
+  // and a frame is traced again only a few times
+  needed_entries = std::max(needed_entries, (uint64_t)std::max<int64_t>(4 * N, 2 * NS));
   uint64_t E = needed_entries;
   for (int k = 0; k < 2; ++k) {
     devAlloc(&rays[k].org, N);

@@ -135,3 +135,19 @@ def test_a_large_frames_next_step_keeps_its_buffers(lib_built):
     later = [step(t, sc) for _ in range(5)]
     assert all(np.array_equal(bits(img), bits(want)) for _, img in later)
     assert min(ms for ms, _ in later) < 2.0 * first, (first, [ms for ms, _ in later])
+
+
+@pytest.mark.parametrize("queues", [0, 4])
+def test_a_large_frame_after_a_tiny_one(lib_built, queues):
+    # the entry arena's size follows the frame, not the first frame ever traced
+    sc = scenes.wavelet_grid(4, 24, colors="albedo", light="quad")
+    pos, look, up = scenes.orbit_camera(sc)
+    cfg = small_config(image_w=16, image_h=16, ao_mode=0, ao_samples=1, pixel_samples=1, bounces=2, bucket_launches=queues)
+    t = sg.Tracer(cfg)
+    t.set_scene(sc)
+    t.set_camera(pos, look, up)
+    t.trace()
+    view = dict(position=pos, lookat=look, up=up, image_w=512, image_h=512, pixel_samples=4)
+    got = t.trace_views([view])[0][0]
+    want = _fresh(dict(cfg, image_w=512, image_h=512, pixel_samples=4), sc, (pos, look, up))
+    assert np.array_equal(bits(got), bits(want))
