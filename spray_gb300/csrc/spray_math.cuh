@@ -344,6 +344,12 @@ SPRAY_HD float hitKeyT(uint64_t key) {
 }
 constexpr uint64_t kNoHit = ~0ull;
 
+// Whether a domain entered at tdom may be left out for a hit at t.  A surface on the
+// domain's boundary has its own t, rounded in the triangle test (some units in the last
+// place), tdom is rounded in the slab test (1.5): without the slack a ray that met such
+// a surface of a neighbour first, or one that coincides, could miss this domain's.
+SPRAY_HD bool beyondHit(float tdom, float t) { return tdom > t * 1.000004f; }
+
 // Interpolated vertex colour with truncation to integer channels and the
 // unnormalised shading normal (src/render/trimesh_buffer.cc:328-360).
 SPRAY_HD uint32_t interpolateColor(uint32_t c0, uint32_t c1, uint32_t c2, float u, float v) {

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256, SPRAY_TRACE_MIN_BLOCKS) kTraceClosest(Tra
         if (kPack && a.cull) {
           const uint2 ent = a.entries[ce];
           const uint64_t cur = *((volatile uint64_t*)&a.ray_key[ent.x & kRayIdMask]);
-          if (cur != kNoHit && __uint_as_float(ent.y) > hitKeyT(cur)) {
+          if (cur != kNoHit && beyondHit(__uint_as_float(ent.y), hitKeyT(cur))) {
             a.rec_key[ce] = kNoHit;
             ++culled;
             live = false;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256, SPRAY_TRACE_MIN_BLOCKS) kTraceClosest(Tra
       if (cur != kNoHit) {
         best_key = cur;
         best_t = hitKeyT(cur);
-        if (tdom > best_t) {
+        if (beyondHit(tdom, best_t)) {
           a.rec_key[e] = kNoHit;
           ++culled;
           continue;
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(256) kCountLive(LiveArgs a) {
         bool live = true;
         if (a.cull) {
           const uint64_t cur = a.ray_key[ent.x & kRayIdMask];
-          live = !(cur != kNoHit && __uint_as_float(ent.y) > hitKeyT(cur));
+          live = !(cur != kNoHit && beyondHit(__uint_as_float(ent.y), hitKeyT(cur)));
         }
         if (live) ++c;
         else a.rec_key[e] = kNoHit;

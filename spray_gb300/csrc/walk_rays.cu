@@ -386,7 +386,7 @@ __device__ __forceinline__ void walkClosest(const RayWalkArgs& a, uint32_t n, in
         has = next < end;
         if (has) {
           const uint2 e = a.arena[next];
-          if (__uint_as_float(e.y) > best_t) {
+          if (beyondHit(__uint_as_float(e.y), best_t)) {
             culled += end - next;
             has = false;
           } else {
